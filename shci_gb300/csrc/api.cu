@@ -119,6 +119,7 @@ void load_csr(shci_ctx* c, size_t n, const uint64_t* row_ptr, const uint32_t* co
     SHCI_CUDA(cudaMemcpyAsync(H.val64.p, vals, nnz * 8, cudaMemcpyHostToDevice, s));
   }
   SHCI_CUDA(cudaMemcpyAsync(H.diag.p, diag, n * 8, cudaMemcpyHostToDevice, s));
+  build_items(c);
   H.valid = true;
   H.build_id++;
 }
@@ -171,6 +172,8 @@ shci_status shci_create(shci_ctx** out, int device, size_t hbm_budget_bytes) {
     H.row_ptr.mt = H.col.mt = H.row_cnt.mt = &c->mem;
     H.val64.mt = H.diag.mt = &c->mem;
     H.val32.mt = H.res32.mt = &c->mem;
+    H.items.it.mt = &c->mem;
+    H.items.off.mt = &c->mem;
     H.scal.mt = H.xs.mt = H.yfix.mt = H.rowabs.mt = &c->mem;
     c->dav.scal.mt = c->dav.partial.mt = &c->mem;
   });

@@ -54,6 +54,17 @@ struct JoinIndex {
 // Segments an incremental update may leave before the next update rebuilds the whole matrix.
 constexpr size_t kMaxSegments = 12;
 
+// Work items of a store segment's row kernels (H*v, the energy correction, the RDM): every row in
+// pieces of at most kItemLen elements, in row order, so that a row of 100,000 elements is shared
+// by many warps instead of being one warp's serial walk.  ok = false: no list (it did not fit);
+// the kernels then take whole rows.
+struct RowItems {
+  DevBuf<uint4> it;       // {row, length, start (low), start (high)}
+  DevBuf<uint32_t> off;   // [n + 1] first item of each row; off[n] = number of items
+  size_t cap = 0;         // bound on the number of items
+  bool ok = false;
+};
+
 // A store segment kept from an earlier build: rows [0, n) of the strict upper part, row i at
 // [row_ptr[i], row_ptr[i] + row_cnt[i]).
 struct HSeg {
@@ -63,6 +74,7 @@ struct HSeg {
   DevBuf<uint32_t> row_cnt, col;
   DevBuf<double> val64;
   DevBuf<float> val32, res32;
+  RowItems items;
 };
 
 // Read-only view of one segment (older segments first, then the current build's).
@@ -76,6 +88,7 @@ struct SegView {
   const double* val64;
   const float* val32;
   const float* res32;
+  const RowItems* items;
 };
 
 // Upper-triangle Hamiltonian (strict upper part in CSR; FP64 diagonal kept apart).  An
@@ -99,6 +112,7 @@ struct DevHamiltonian {
   DevBuf<float> res32;        // [nnz]   mixed storage: FP32 residual (value - (double)val32)
   DevBuf<double> diag;        // [n]
   DevBuf<uint32_t> row_cnt;   // [n+1] elements of each row
+  RowItems items;             // work items of the current segment
   bool valid = false;
   // the stored matrix is that of the first n dets of the current list (dets were only
   // appended since the build): an update can be incremental
@@ -120,9 +134,9 @@ inline std::vector<SegView> segments(const DevHamiltonian& H) {
   std::vector<SegView> v;
   for (const auto& s : H.older)
     v.push_back(SegView{s->n, s->nnz, s->col.n, s->packed, s->row_ptr.p, s->row_cnt.p,
-                        s->col.p, s->val64.p, s->val32.p, s->res32.p});
+                        s->col.p, s->val64.p, s->val32.p, s->res32.p, &s->items});
   v.push_back(SegView{H.n, H.nnz_current, H.col.n, H.packed, H.row_ptr.p, H.row_cnt.p, H.col.p,
-                      H.val64.p, H.val32.p, H.res32.p});
+                      H.val64.p, H.val32.p, H.res32.p, &H.items});
   return v;
 }
 
@@ -151,7 +165,7 @@ struct Davidson {
   DevBuf<double> sv[5 * kMaxStates], sHv[5 * kMaxStates], sw[kMaxStates], sHw[kMaxStates];
   DevBuf<double> scal;     // device scalars
   DevBuf<double> partial;  // dot partial sums
-  DevBuf<double> rt;       // residual-store row sums of the FP64 energy correction
+  DevBuf<double> rt;       // shares of the work items in the FP64 energy correction
   // w and Hw hold the last Ritz vector and its image under the Hamiltonian of build ritz_h
   bool ritz = false;
   uint64_t ritz_h = 0;

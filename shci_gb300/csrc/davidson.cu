@@ -43,7 +43,7 @@ struct Ptrs6 {
   const double* p[6];
 };
 
-// partial[m * kDotBlocks + b] = block b's share of <x, ys[m]>
+// partial[m * kDotBlocks + b] = block b's share of <x, ys[m]> (ys[m] null: of sum x)
 __global__ void __launch_bounds__(kDotThreads)
     k_mdot_partial(const double* __restrict__ x, Ptrs6 ys, int m, size_t n,
                    double* __restrict__ partial) {
@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kDotThreads)
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const double xi = x[i];
-    for (int k = 0; k < m; k++) acc[k] += xi * ys.p[k][i];
+    for (int k = 0; k < m; k++) acc[k] += ys.p[k] ? xi * ys.p[k][i] : xi;
   }
   for (int k = 0; k < m; k++) {
     const double t = block_sum(acc[k]);
@@ -496,7 +496,7 @@ DavidsonStatesOut davidson_states(shci_ctx* c, double tol) {
 // Rayleigh quotient of d_coef with value + residual.  When d_coef is still the Ritz vector w
 // of the last Davidson call on this (mixed) Hamiltonian, w^T H w = w^T Hw + w^T R w with Hw =
 // H32 w kept by Davidson (FP32 values, FP64 diagonal), so only the residual store R is read
-// (2 sum_i w_i (R w)_i over its upper triangle: one gather per element, no atomics);
+// (2 w^T R w over its upper triangle: one gather per element, no atomics);
 // otherwise H w is formed from value + residual.
 double rayleigh_fp64(shci_ctx* c) {
   const size_t n = c->H.n;
@@ -514,9 +514,8 @@ double rayleigh_fp64(shci_ctx* c) {
     SHCI_CUDA(cudaStreamSynchronize(s));
     if (differs == 0.0) {
       D.rt.mt = &c->mem;
-      D.rt.resize(n, 1.1);
-      residual_rows(c, D.w.p, D.rt.p);
-      const double num = dots.dot_host(D.w.p, D.Hw.p, n) + 2.0 * dots.dot_host(D.w.p, D.rt.p, n);
+      const size_t len = residual_rows(c, D.w.p, D.rt);
+      const double num = dots.dot_host(D.w.p, D.Hw.p, n) + 2.0 * dots.dot_host(D.rt.p, nullptr, len);
       const double den = dots.dot_host(D.w.p, D.w.p, n);
       c->launches += 1;
       return num / den;

@@ -511,6 +511,8 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
     auto seg = std::make_unique<HSeg>();
     seg->row_ptr.mt = seg->col.mt = &c->mem;
     seg->row_cnt.mt = &c->mem;
+    seg->items.it.mt = &c->mem;
+    seg->items.off.mt = &c->mem;
     seg->val64.mt = seg->val32.mt = seg->res32.mt = &c->mem;
     seg->n = H.n;
     seg->nnz = H.nnz_current;
@@ -521,10 +523,15 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
     seg->val64.swap(H.val64);
     seg->val32.swap(H.val32);
     seg->res32.swap(H.res32);
+    seg->items.it.swap(H.items.it);
+    seg->items.off.swap(H.items.off);
+    seg->items.cap = H.items.cap;
+    seg->items.ok = H.items.ok;
     H.older.push_back(std::move(seg));
   } else {
     H.older.clear();
   }
+  H.items.ok = false;
   H.n_prev = n_prev;
   H.n = n;
   H.precision = precision;
@@ -650,6 +657,7 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
   SHCI_CUDA(cudaStreamSynchronize(s));
   if (H.join) join_release(c);
   if (row_sort_enabled()) sort_rows(c);
+  build_items(c);
   c->prof.flush();
   H.valid = true;
   H.prefix_ok = true;

@@ -57,10 +57,14 @@ uint64_t join_row_caps(shci_ctx* c, uint64_t* row_start, uint32_t n_prev);
 bool row_sort_enabled();
 void sort_rows(shci_ctx* c);
 
+// spmv.cu: the work items of the current segment (rows in pieces; see RowItems)
+void build_items(shci_ctx* c);
+
 // spmv.cu: y = H x (FP64 vectors on the device); residual adds the FP32 residual store.
 void spmv(shci_ctx* c, const double* x, double* y, bool residual);
-// t_i = sum_j R_ij w_j over the stored (upper) elements of the residual store R (mixed H).
-void residual_rows(shci_ctx* c, const double* w, double* t);
+// out[k] = w_i sum_j R_ij w_j over work item k of row i of the residual store R (mixed H, upper
+// elements; unused entries 0).  Returns the length of out.
+size_t residual_rows(shci_ctx* c, const double* w, DevBuf<double>& out);
 // Mixed H*v needs a bound on the row abs sums: a mixed build sums |H_ij| into H.rowabs
 // (off-diagonal) during its count or single fill pass, and this turns the sums into the bound.
 void finish_mixed_bound(shci_ctx* c);

@@ -341,6 +341,13 @@ void exclusive_scan_u64_async(const uint64_t* in, uint64_t* out, size_t n, cudaS
   scan_rec<uint64_t>(in, out, n, s, sc.part64.p, total_dev);
 }
 
+void exclusive_scan_u32_async(const uint32_t* in, uint32_t* out, size_t n, cudaStream_t s,
+                              SortScratch& sc, uint32_t* total_dev) {
+  if (n == 0) return;
+  sc.part32.reserve(scan_part_size(n) + 1, 1.25);
+  scan_rec<uint32_t>(in, out, n, s, sc.part32.p, total_dev);
+}
+
 uint32_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, cudaStream_t s,
                             SortScratch& sc) {
   if (n == 0) return 0;

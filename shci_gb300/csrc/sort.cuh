@@ -33,6 +33,8 @@ uint32_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, cudaStr
 // Same without returning the total (no synchronisation); total written to *total_dev if set.
 void exclusive_scan_u64_async(const uint64_t* in, uint64_t* out, size_t n, cudaStream_t s,
                               SortScratch& sc, uint64_t* total_dev);
+void exclusive_scan_u32_async(const uint32_t* in, uint32_t* out, size_t n, cudaStream_t s,
+                              SortScratch& sc, uint32_t* total_dev);
 
 // Stable sort of the first n (keys, vals) by key bits [begin_bit, end_bit).  When the
 // result ends up in the scratch ping-pong buffers, their storage is swapped into `keys` /

@@ -1,8 +1,8 @@
 // Symmetric sparse H*v over the upper-triangle store (K4).
 //
 // Replaces SparseMatrix::mul (src/solver/sparse_matrix.cc:28-56): y = H x with H stored as
-// its strict upper triangle plus an FP64 diagonal.  One warp per row i streams the row's
-// (col, val) pairs once: the row part y_i += H_ij x_j is reduced in registers and the
+// its strict upper triangle plus an FP64 diagonal.  A warp takes a piece of a row i at a time
+// (items.cuh) and streams its (col, val) pairs once: the row part y_i += H_ij x_j is reduced in registers and the
 // transpose part y_j += H_ij x_i goes out as atomics (y is L2 resident).
 //
 // FP64 storage: FP64 products and FP64 atomics (the exact path).
@@ -27,25 +27,50 @@
 #include <cstring>
 
 #include "ctx.h"
+#include "items.cuh"
 #include "kernels.h"
 
 namespace shci {
 
 namespace {
 
-// FP64 store: FP64 products, FP64 atomics.
+__global__ void k_item_counts(const uint32_t* __restrict__ row_cnt, uint32_t n, uint32_t* cnt) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    cnt[i] = (row_cnt[i] + kItemLen - 1) / kItemLen;
+}
+
+__global__ void k_item_fill(const uint64_t* __restrict__ row_ptr,
+                            const uint32_t* __restrict__ row_cnt,
+                            const uint32_t* __restrict__ off, uint32_t n, uint4* it) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t len = row_cnt[i];
+    uint32_t k = off[i];
+    for (uint32_t b = 0; b < len; b += kItemLen) {
+      const uint64_t st = row_ptr[i] + b;
+      it[k++] = make_uint4(i, min(len - b, kItemLen), static_cast<uint32_t>(st),
+                           static_cast<uint32_t>(st >> 32));
+    }
+  }
+}
+
+// y = diag * x
+__global__ void k_diag_mul(const double* __restrict__ diag, const double* __restrict__ x,
+                           double* __restrict__ y, uint32_t n) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    y[i] = diag[i] * x[i];
+}
+
+// FP64 store: FP64 products, FP64 atomics (y holds diag * x).
 __global__ void __launch_bounds__(256)
-    k_spmv(const uint64_t* __restrict__ row_ptr, const uint32_t* __restrict__ row_len,
-           const uint32_t* __restrict__ col, const double* __restrict__ v64,
-           const double* __restrict__ diag, const double* __restrict__ x, double* __restrict__ y,
-           uint32_t n) {
+    k_spmv(const __grid_constant__ ItemTab T, const double* __restrict__ x,
+           double* __restrict__ y) {
   const unsigned lane = threadIdx.x & 31;
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-    const uint64_t rs = row_ptr[i], re = rs + row_len[i];
+  for_items(T, [&](const ItemSeg& S, uint64_t, uint32_t i, uint64_t rs, uint32_t len) {
     const double xi = x[i];
     double acc = 0.0;
-    for (uint64_t k = rs + lane; k < re; k += 32) {
+    const uint32_t* __restrict__ col = S.col + rs;
+    const double* __restrict__ v64 = S.v64 + rs;
+    for (uint32_t k = lane; k < len; k += 32) {
       const uint32_t j = col[k];
       const double v = v64[k];
       acc += v * x[j];
@@ -53,8 +78,8 @@ __global__ void __launch_bounds__(256)
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
-    if (lane == 0) atomicAdd(&y[i], diag ? acc + diag[i] * xi : acc);
-  }
+    if (lane == 0) atomicAdd(&y[i], acc);
+  });
 }
 
 // ---------------------------------------------------------------- mixed: fixed point
@@ -98,15 +123,17 @@ __device__ __forceinline__ int fix_scale(double B) {
   return 61 - e;
 }
 
-// x -> float pairs; max |x| (as ordered bits of a non-negative double) into *xmax_bits.
+// x -> float pairs; max |x| (as ordered bits of a non-negative double) into *xmax_bits; the
+// fixed-point accumulators (when given) cleared.
 __global__ void k_split_x(const double* __restrict__ x, uint32_t n, float2* xs,
-                          unsigned long long* xmax_bits) {
+                          unsigned long long* xmax_bits, unsigned long long* yfix) {
   unsigned long long mx = 0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double v = x[i];
     const float h = static_cast<float>(v);
     const float l = static_cast<float>(v - static_cast<double>(h));
     xs[i] = make_float2(h, l);
+    if (yfix) yfix[i] = 0ull;
     const unsigned long long a = static_cast<unsigned long long>(__double_as_longlong(fabs(v)));
     mx = a > mx ? a : mx;
   }
@@ -155,20 +182,18 @@ __global__ void k_max_bound(const float* __restrict__ a, const double* __restric
 // Mixed H*v: float-pair products, fixed-point accumulation (off-diagonal part only).
 template <bool RES>
 __global__ void __launch_bounds__(256)
-    k_spmv_fix(const uint64_t* __restrict__ row_ptr, const uint32_t* __restrict__ row_len,
-               const uint32_t* __restrict__ col,
-               const float* __restrict__ v32, const float* __restrict__ r32,
-               const float2* __restrict__ xs, const double* __restrict__ scal,
-               unsigned long long* __restrict__ yfix, uint32_t n) {
+    k_spmv_fix(const __grid_constant__ ItemTab T, const float2* __restrict__ xs,
+               const double* __restrict__ scal, unsigned long long* __restrict__ yfix) {
   const int s = fix_scale(scal[0] * __longlong_as_double(static_cast<long long>(
                                         reinterpret_cast<const unsigned long long*>(scal)[1])));
   const unsigned lane = threadIdx.x & 31;
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-    const uint64_t rs = row_ptr[i], re = rs + row_len[i];
+  for_items(T, [&](const ItemSeg& S, uint64_t, uint32_t i, uint64_t rs, uint32_t len) {
     const float2 xi = xs[i];
     float ah = 0.0f, al = 0.0f;
-    for (uint64_t k = rs + lane; k < re; k += 32) {
+    const uint32_t* __restrict__ col = S.col + rs;
+    const float* __restrict__ v32 = S.v32 + rs;
+    const float* __restrict__ r32 = RES ? S.r32 + rs : nullptr;
+    for (uint32_t k = lane; k < len; k += 32) {
       const uint32_t j = col[k];
       const float v = v32[k];
       const float r = RES ? r32[k] : 0.0f;
@@ -191,7 +216,7 @@ __global__ void __launch_bounds__(256)
     }
     if (lane == 0)
       atomicAdd(&yfix[i], static_cast<unsigned long long>(f2fix(ah, s) + f2fix(al, s)));
-  }
+  });
 }
 
 // y = yfix * 2^-s + diag * x
@@ -250,21 +275,20 @@ void mixed_bound(shci_ctx* c, unsigned grid) {
   finish_mixed_bound(c);
 }
 
-// t_i += sum over row i's stored elements of residual_ij * w_j (no atomics: the FP64 energy
-// correction needs only w^T R w = 2 sum_i w_i t_i of the residual store R).  w comes split
-// into float pairs and the products and sums are float pairs, as in the mixed H*v (about
-// 2^-44 relative): the FP64 form spent two FP64 operations per element (conversion and FMA),
-// more than the gathers cost on GB300.
+// out[item] = w_i * sum over the item's elements of residual_ij * w_j (no atomics: the FP64
+// energy correction needs only w^T R w = 2 sum_i w_i sum_j R_ij w_j of the residual store R).  w
+// comes split into float pairs and the products and sums are float pairs, as in the mixed H*v
+// (about 2^-44 relative): the FP64 form spent two FP64 operations per element (conversion and
+// FMA), more than the gathers cost on GB300.
 __global__ void __launch_bounds__(256)
-    k_res_rows(const uint64_t* __restrict__ row_ptr, const uint32_t* __restrict__ row_len,
-               const uint32_t* __restrict__ col, const float* __restrict__ r32,
-               const float2* __restrict__ ws, double* __restrict__ t, uint32_t n) {
+    k_res_rows(const __grid_constant__ ItemTab T, const float2* __restrict__ ws,
+               const double* __restrict__ w, double* __restrict__ out) {
   const unsigned lane = threadIdx.x & 31;
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  for (uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-    const uint64_t rs = row_ptr[i], re = rs + row_len[i];
+  for_items(T, [&](const ItemSeg& S, uint64_t at, uint32_t i, uint64_t rs, uint32_t len) {
     float ah = 0.0f, al = 0.0f;
-    for (uint64_t k = rs + lane; k < re; k += 32) {
+    const uint32_t* __restrict__ col = S.col + rs;
+    const float* __restrict__ r32 = S.r32 + rs;
+    for (uint32_t k = lane; k < len; k += 32) {
       const float2 wj = ws[col[k]];
       float p, e, s2, se;
       prod2<false>(r32[k], 0.0f, wj.x, wj.y, &p, &e);
@@ -280,35 +304,66 @@ __global__ void __launch_bounds__(256)
       ah = s2;
       al = al + bl + se;
     }
-    if (lane == 0) t[i] += static_cast<double>(ah) + static_cast<double>(al);
-  }
+    if (lane == 0) out[at] = w[i] * (static_cast<double>(ah) + static_cast<double>(al));
+  });
+}
+
+// Grid of the item kernels: eight CTAs of eight warps per SM, fewer when the matrix is small.
+unsigned item_grid(shci_ctx* c, size_t items) {
+  int sms = 0;
+  SHCI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  return grid_for(items * 32, 256, (unsigned)sms * 8u);
 }
 
 }  // namespace
 
-void residual_rows(shci_ctx* c, const double* w, double* t) {
+void build_items(shci_ctx* c) {
+  auto& H = c->H;
+  auto& R = H.items;
+  cudaStream_t s = c->stream;
+  const uint32_t n = static_cast<uint32_t>(H.n);
+  R.ok = false;
+  if (n == 0) return;
+  R.cap = H.nnz_current / kItemLen + n;  // sum of ceil(len / kItemLen) over n rows
+  if (R.cap >= 0xffffffffull) return;
+  try {
+    R.off.resize((size_t)n + 1, 1.1);
+    R.it.resize(R.cap, 1.1);
+    k_item_counts<<<grid_for(n, 256), 256, 0, s>>>(H.row_cnt.p, n, R.off.p);
+    SHCI_LAUNCH_CHECK();
+    exclusive_scan_u32_async(R.off.p, R.off.p, n, s, c->sort, R.off.p + n);
+  } catch (const OomError&) {  // no room: the kernels take whole rows
+    R.off.release();
+    R.it.release();
+    return;
+  }
+  k_item_fill<<<grid_for(n, 256), 256, 0, s>>>(H.row_ptr.p, H.row_cnt.p, R.off.p, n, R.it.p);
+  SHCI_LAUNCH_CHECK();
+  R.ok = true;
+  c->launches += 4;
+}
+
+size_t residual_rows(shci_ctx* c, const double* w, DevBuf<double>& out) {
   auto& H = c->H;
   if (!H.valid || H.precision == SHCI_PREC_FP64) throw ArgError("no mixed Hamiltonian built");
   const uint32_t n = static_cast<uint32_t>(H.n);
-  int sms = 0;
-  SHCI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  const unsigned grid = grid_for((size_t)n * 32, 256, (unsigned)sms * 8u);
   cudaStream_t s = c->stream;
+  size_t len = 0;
+  const ItemTab T = item_tab(H, &len);
+  out.resize(len, 1.1);
   ProfScope ps(c->prof, s, "spmv_res_rows");
   H.xs.resize(2 * (size_t)n, 1.1);
   float2* ws = reinterpret_cast<float2*>(H.xs.p);
   SHCI_CUDA(cudaMemsetAsync(H.scal.p + 1, 0, 8, s));
   k_split_x<<<grid_for(n, 256), 256, 0, s>>>(w, n, ws,
-                                             reinterpret_cast<unsigned long long*>(H.scal.p + 1));
+                                             reinterpret_cast<unsigned long long*>(H.scal.p + 1),
+                                             nullptr);
   SHCI_LAUNCH_CHECK();
-  SHCI_CUDA(cudaMemsetAsync(t, 0, (size_t)n * 8, s));
-  for (const SegView& g : segments(H)) {
-    k_res_rows<<<grid, 256, 0, s>>>(g.row_ptr, g.row_cnt, g.col, g.res32, ws, t,
-                                    static_cast<uint32_t>(g.n));
-    SHCI_LAUNCH_CHECK();
-    c->launches += 1;
-  }
-  c->launches += 1;
+  SHCI_CUDA(cudaMemsetAsync(out.p, 0, len * 8, s));
+  k_res_rows<<<item_grid(c, len), 256, 0, s>>>(T, ws, w, out.p);
+  SHCI_LAUNCH_CHECK();
+  c->launches += 2;
+  return len;
 }
 
 void spmv(shci_ctx* c, const double* x, double* y, bool residual) {
@@ -316,48 +371,33 @@ void spmv(shci_ctx* c, const double* x, double* y, bool residual) {
   if (!H.valid) throw ArgError("no Hamiltonian built");
   cudaStream_t s = c->stream;
   const uint32_t n = static_cast<uint32_t>(H.n);
-  int sms = 0;
-  SHCI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  const unsigned grid = grid_for((size_t)n * 32, 256, (unsigned)sms * 8u);
+  size_t len = 0;
+  const ItemTab T = item_tab(H, &len);
+  const unsigned grid = item_grid(c, len);
   if (H.precision == SHCI_PREC_FP64) {
     ProfScope ps(c->prof, s, "spmv");
-    SHCI_CUDA(cudaMemsetAsync(y, 0, H.n * sizeof(double), s));
-    const auto segs = segments(H);
-    for (size_t k = 0; k < segs.size(); k++) {
-      const SegView& g = segs[k];
-      // the diagonal goes in with the current segment, which covers every row
-      k_spmv<<<grid, 256, 0, s>>>(g.row_ptr, g.row_cnt, g.col, g.val64,
-                                  k + 1 == segs.size() ? H.diag.p : nullptr, x, y,
-                                  static_cast<uint32_t>(g.n));
-      SHCI_LAUNCH_CHECK();
-      c->launches += 1;
-    }
+    k_diag_mul<<<grid_for(n, 256), 256, 0, s>>>(H.diag.p, x, y, n);
+    SHCI_LAUNCH_CHECK();
+    k_spmv<<<grid, 256, 0, s>>>(T, x, y);
+    SHCI_LAUNCH_CHECK();
+    c->launches += 2;
     return;
   }
   if (!H.bound_valid) mixed_bound(c, grid);
   H.xs.resize(2 * (size_t)n, 1.1);
   H.yfix.resize(n, 1.1);
   ProfScope ps(c->prof, s, "spmv");
-  SHCI_CUDA(cudaMemsetAsync(H.yfix.p, 0, (size_t)n * 8, s));
   SHCI_CUDA(cudaMemsetAsync(H.scal.p + 1, 0, 8, s));
   float2* xs = reinterpret_cast<float2*>(H.xs.p);
   k_split_x<<<grid_for(n, 256), 256, 0, s>>>(
-      x, n, xs, reinterpret_cast<unsigned long long*>(H.scal.p + 1));
+      x, n, xs, reinterpret_cast<unsigned long long*>(H.scal.p + 1), H.yfix.p);
   SHCI_LAUNCH_CHECK();
-  for (const SegView& g : segments(H)) {
-    const uint32_t gn = static_cast<uint32_t>(g.n);
-    if (residual)
-      k_spmv_fix<true><<<grid, 256, 0, s>>>(g.row_ptr, g.row_cnt, g.col, g.val32, g.res32, xs,
-                                             H.scal.p, H.yfix.p, gn);
-    else
-      k_spmv_fix<false><<<grid, 256, 0, s>>>(g.row_ptr, g.row_cnt, g.col, g.val32, nullptr, xs,
-                                              H.scal.p, H.yfix.p, gn);
-    SHCI_LAUNCH_CHECK();
-    c->launches += 1;
-  }
+  if (residual) k_spmv_fix<true><<<grid, 256, 0, s>>>(T, xs, H.scal.p, H.yfix.p);
+  else k_spmv_fix<false><<<grid, 256, 0, s>>>(T, xs, H.scal.p, H.yfix.p);
+  SHCI_LAUNCH_CHECK();
   k_fix_out<<<grid_for(n, 256), 256, 0, s>>>(H.yfix.p, H.diag.p, x, H.scal.p, y, n);
   SHCI_LAUNCH_CHECK();
-  c->launches += 2;
+  c->launches += 3;
 }
 
 }  // namespace shci

@@ -237,6 +237,7 @@ size_t build_time_sym(shci_ctx* c, int precision) {
   H.candidates = K;
   H.cand_parts[0] = K;
   H.cand_parts[1] = H.cand_parts[2] = 0;
+  build_items(c);
   H.valid = true;
   H.prefix_ok = false;  // every update rebuilds (the unpacked list is not append-only)
   H.build_id++;
