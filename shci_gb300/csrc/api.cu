@@ -155,7 +155,7 @@ shci_status shci_create(shci_ctx** out, int device, size_t hbm_budget_bytes) {
     for (auto* b : {&c->h1, &c->g2, &c->dtab, &c->xtab, &c->jtab, &c->ktab, &c->d_coef, &c->f0,
                     &c->f1})
       b->mt = &c->mem;
-    for (auto* b : {&c->d_up, &c->d_dn, &c->set_up, &c->set_dn, &c->k0, &c->k1, &c->k2})
+    for (auto* b : {&c->d_up, &c->d_dn, &c->k0, &c->k1, &c->k2})
       b->mt = &c->mem;
     for (auto* b : {&c->u0, &c->u1, &c->u2}) b->mt = &c->mem;
     c->err_word.mt = &c->mem;

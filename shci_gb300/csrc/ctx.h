@@ -207,9 +207,8 @@ struct shci_ctx {
   shci::DevBuf<double> d_xcoef[shci::kMaxStates - 1];
   std::vector<double> state_energy;
 
-  // sorted membership keys of the current det list (for selection / PT2)
-  shci::DevBuf<uint64_t> set_up, set_dn;
-  shci::DevBuf<unsigned long long> set_hash;  // hash set of the det list (in_set)
+  // membership set of the current det list (selection, PT2, S^2, 1-RDM)
+  shci::DevBuf<unsigned long long> set_hash;  // hash set of the det list (set_index)
   uint64_t set_hash_mask = 0;
 
   std::vector<double> eps_tried;

@@ -28,10 +28,7 @@ struct SelParams {
   const double* s_S;
   const uint32_t* s_r;
   const uint32_t* pair_tab;  // pair k -> p_id | q_id << 16
-  const uint64_t* set_up;    // sorted variational set
-  const uint64_t* set_dn;
-  uint32_t set_n;
-  const unsigned long long* set_hash;  // hash set of the variational dets (see in_set)
+  const unsigned long long* set_hash;  // hash set of the variational dets (see set_index)
   uint64_t set_hash_mask;
   double eps_var;
   double max_hci, max_singles;
@@ -139,33 +136,27 @@ __host__ __device__ __forceinline__ uint64_t set_slot_hash(uint64_t u, uint64_t 
   return h;
 }
 
-// Is (u, d) a variational det?  With the hash set (slots hold fingerprint << 32 | det id + 1,
-// linear probing, at most half full) one or two probes and a comparison against the det
-// list; otherwise a binary search of the sorted set.
-__device__ __forceinline__ bool in_set(const SelParams& P, uint64_t u, uint64_t d) {
-  if (P.set_hash) {
-    const uint64_t h = set_slot_hash(u, d);
-    const uint32_t fp = static_cast<uint32_t>(h >> 32);
-    uint64_t p = h & P.set_hash_mask;
-    for (uint64_t probe = 0; probe <= P.set_hash_mask; probe++) {
-      const unsigned long long v = P.set_hash[p];
-      if (v == 0ull) return false;
-      if (static_cast<uint32_t>(v >> 32) == fp) {
-        const uint32_t id = static_cast<uint32_t>(v) - 1u;
-        if (P.up[id] == u && P.dn[id] == d) return true;
-      }
-      p = (p + 1) & P.set_hash_mask;
+// Id of det (u, d) in the hash set of the variational dets, or -1 (slots hold fingerprint << 32 |
+// det id + 1, linear probing, at most half full): one or two probes, then a comparison against
+// the det list.
+__device__ __forceinline__ long long set_index(const SelParams& P, uint64_t u, uint64_t d) {
+  const uint64_t h = set_slot_hash(u, d);
+  const uint32_t fp = static_cast<uint32_t>(h >> 32);
+  uint64_t p = h & P.set_hash_mask;
+  for (uint64_t probe = 0; probe <= P.set_hash_mask; probe++) {
+    const unsigned long long v = P.set_hash[p];
+    if (v == 0ull) return -1;
+    if (static_cast<uint32_t>(v >> 32) == fp) {
+      const uint32_t id = static_cast<uint32_t>(v) - 1u;
+      if (P.up[id] == u && P.dn[id] == d) return id;
     }
-    return false;
+    p = (p + 1) & P.set_hash_mask;
   }
-  uint32_t lo = 0, hi = P.set_n;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    const uint64_t su = P.set_up[mid], sd = P.set_dn[mid];
-    if (su < u || (su == u && sd < d)) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo < P.set_n && P.set_up[lo] == u && P.set_dn[lo] == d;
+  return -1;
+}
+
+__device__ __forceinline__ bool in_set(const SelParams& P, uint64_t u, uint64_t d) {
+  return set_index(P, u, d) >= 0;
 }
 
 __device__ __forceinline__ double src_eps_min(const SelParams& P, uint32_t i) {

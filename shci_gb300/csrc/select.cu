@@ -13,8 +13,8 @@
 //   k_sel_count: a warp per source det -> candidate count (also updates eps_tried_prev),
 //   scan        : output segment per det,
 //   k_sel_emit  : a warp per source det flattens its (slot, entry) ranges over lanes, builds
-//                 each candidate det, tests membership by binary search in the sorted
-//                 variational set and (singles) the |H_ai| >= eps_min rule,
+//                 each candidate det, tests membership in the hash set of the
+//                 variational dets and (singles) the |H_ai| >= eps_min rule,
 //   compaction + two-stage radix sort + unique -> this pass's new dets in ascending Det order.
 // New dets of a pass join the variational set before the next pass, as in the reference.
 // With second rejection (off by default) the emission also drops window entries whose
@@ -357,44 +357,62 @@ void compact_valid(shci_ctx* c, const uint64_t* a, const uint64_t* b, const doub
   *n_out = at + nv;
 }
 
-// Sorted copy of the whole det list, the membership set used by selection and PT2.
-// Inserts det ids into the variational hash set (slot = fingerprint << 32 | id + 1, linear
-// probing; the table is at most half full, so every insertion finds an empty slot).
+// Inserts det ids [begin, end) into the variational hash set (slot = fingerprint << 32 | id + 1,
+// linear probing; the table is at most half full, so every insertion finds an empty slot).  Equal
+// dets probe the same slots and slots are never emptied, so of two equal dets the one inserted
+// later meets the other on its way: *dup is set.
 __global__ void k_hash_insert(const uint64_t* __restrict__ up, const uint64_t* __restrict__ dn,
-                              size_t n, unsigned long long* table, uint64_t mask) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+                              size_t begin, size_t end, unsigned long long* table, uint64_t mask,
+                              unsigned* dup) {
+  for (size_t i = begin + blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < end;
        i += (size_t)gridDim.x * blockDim.x) {
-    const uint64_t h = set_slot_hash(up[i], dn[i]);
+    const uint64_t u = up[i], d = dn[i];
+    const uint64_t h = set_slot_hash(u, d);
     const unsigned long long v = ((h >> 32) << 32) | (static_cast<unsigned long long>(i) + 1ull);
     uint64_t p = h & mask;
     for (uint64_t probe = 0; probe <= mask; probe++) {
-      if (atomicCAS(&table[p], 0ull, v) == 0ull) break;
+      const unsigned long long old = atomicCAS(&table[p], 0ull, v);
+      if (old == 0ull) break;
+      if ((old >> 32) == (v >> 32)) {
+        const uint32_t id = static_cast<uint32_t>(old) - 1u;
+        if (up[id] == u && dn[id] == d) {
+          atomicOr(dup, 1u);
+          break;
+        }
+      }
       p = (p + 1) & mask;
     }
   }
 }
 
-void rebuild_det_set(shci_ctx* c) {
+// The membership set used by selection, PT2, S^2 and the 1-RDM: a hash set of the det list, a power
+// of two >= 2n slots.  n_have > 0: the set holds the first n_have dets already (n_have < n): the
+// others are inserted, unless the table has become too small for them.  (The set used to come
+// with a sorted copy of the list that only the duplicate check read: two radix sorts per call,
+// six calls per selection.)
+void rebuild_det_set(shci_ctx* c, size_t n_have) {
   const size_t n = c->up.size();
   cudaStream_t s = c->stream;
-  c->set_up.mt = c->set_dn.mt = &c->mem;
-  c->set_up.resize(n, 1.25);
-  c->set_dn.resize(n, 1.25);
-  SHCI_CUDA(cudaMemcpyAsync(c->set_up.p, c->d_up.p, n * 8, cudaMemcpyDeviceToDevice, s));
-  SHCI_CUDA(cudaMemcpyAsync(c->set_dn.p, c->d_dn.p, n * 8, cudaMemcpyDeviceToDevice, s));
-  const size_t nu = sort_unique_pairs(c, c->set_up, c->set_dn, n);
-  if (nu != n) throw ArgError("the det list contains duplicates");
-  // hash set over the det list: a power of two >= 2n slots
-  size_t slots = 1024;
-  while (slots < 2 * n) slots <<= 1;
-  c->set_hash.mt = &c->mem;
-  c->set_hash.resize(slots, 1.0);
-  c->set_hash_mask = slots - 1;
-  SHCI_CUDA(cudaMemsetAsync(c->set_hash.p, 0, slots * 8, s));
-  k_hash_insert<<<grid_for(n, 256), 256, 0, s>>>(c->d_up.p, c->d_dn.p, n, c->set_hash.p,
-                                                 c->set_hash_mask);
+  c->err_word.resize(8);
+  unsigned* dup = c->err_word.p;
+  SHCI_CUDA(cudaMemsetAsync(dup, 0, sizeof(unsigned), s));
+  if (n_have == 0 || c->set_hash_mask + 1 < 2 * n) {
+    size_t slots = 1024;
+    while (slots < 2 * n) slots <<= 1;
+    c->set_hash.mt = &c->mem;
+    c->set_hash.resize(slots, 1.0);
+    c->set_hash_mask = slots - 1;
+    SHCI_CUDA(cudaMemsetAsync(c->set_hash.p, 0, slots * 8, s));
+    n_have = 0;
+  }
+  k_hash_insert<<<grid_for(n - n_have, 256), 256, 0, s>>>(c->d_up.p, c->d_dn.p, n_have, n,
+                                                          c->set_hash.p, c->set_hash_mask, dup);
   SHCI_LAUNCH_CHECK();
+  unsigned bad = 0;
+  SHCI_CUDA(cudaMemcpyAsync(&bad, dup, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+  SHCI_CUDA(cudaStreamSynchronize(s));
   c->launches += 1;
+  if (bad) throw ArgError("the det list contains duplicates");
 }
 
 size_t select_dets(shci_ctx* c, double eps_var, bool var_sd) {
@@ -485,9 +503,6 @@ size_t select_dets(shci_ctx* c, double eps_var, bool var_sd) {
     P.up = c->d_up.p;
     P.dn = c->d_dn.p;
     P.coef = c->n_states > 1 ? d_selc.p : c->d_coef.p;
-    P.set_up = c->set_up.p;
-    P.set_dn = c->set_dn.p;
-    P.set_n = static_cast<uint32_t>(c->set_up.n);
     P.set_hash = c->set_hash.p;
     P.set_hash_mask = c->set_hash_mask;
     const uint32_t n_src = n_dets > pass ? static_cast<uint32_t>((n_dets - pass + 4) / 5) : 0;
@@ -574,7 +589,7 @@ size_t select_dets(shci_ctx* c, double eps_var, bool var_sd) {
       SHCI_CUDA(cudaStreamSynchronize(s));
       n_new_total += pass_n;
       // the new dets join the membership set before the next pass
-      rebuild_det_set(c);
+      rebuild_det_set(c, old);
     }
   }
   // eps_tried_prev back to the host mirror (only the sources of this step changed)

@@ -22,23 +22,6 @@ namespace shci {
 
 namespace {
 
-// Id of det (u, d) in the hash set of the det list, or -1.
-__device__ __forceinline__ long long set_index(const SelParams& P, uint64_t u, uint64_t d) {
-  const uint64_t h = set_slot_hash(u, d);
-  const uint32_t fp = static_cast<uint32_t>(h >> 32);
-  uint64_t p = h & P.set_hash_mask;
-  for (uint64_t probe = 0; probe <= P.set_hash_mask; probe++) {
-    const unsigned long long v = P.set_hash[p];
-    if (v == 0ull) return -1;
-    if (static_cast<uint32_t>(v >> 32) == fp) {
-      const uint32_t id = static_cast<uint32_t>(v) - 1u;
-      if (P.up[id] == u && P.dn[id] == d) return id;
-    }
-    p = (p + 1) & P.set_hash_mask;
-  }
-  return -1;
-}
-
 __global__ void k_s2(SelParams P, const double* __restrict__ coef, uint32_t n, double nu,
                      double nd, double* __restrict__ out) {
   const unsigned lane = threadIdx.x & 31;
