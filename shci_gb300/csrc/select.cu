@@ -387,10 +387,11 @@ __global__ void k_hash_insert(const uint64_t* __restrict__ up, const uint64_t* _
 
 // The membership set used by selection, PT2, S^2 and the 1-RDM: a hash set of the det list, a power
 // of two >= 2n slots.  n_have > 0: the set holds the first n_have dets already (n_have < n): the
-// others are inserted, unless the table has become too small for them.  (The set used to come
+// others are inserted, unless the table has become too small for them.  allow_dup: the set holds
+// one of each group of equal dets instead of refusing the list.  (The set used to come
 // with a sorted copy of the list that only the duplicate check read: two radix sorts per call,
 // six calls per selection.)
-void rebuild_det_set(shci_ctx* c, size_t n_have) {
+void rebuild_det_set(shci_ctx* c, size_t n_have, bool allow_dup) {
   const size_t n = c->up.size();
   cudaStream_t s = c->stream;
   c->err_word.resize(8);
@@ -412,7 +413,7 @@ void rebuild_det_set(shci_ctx* c, size_t n_have) {
   SHCI_CUDA(cudaMemcpyAsync(&bad, dup, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
   c->launches += 1;
-  if (bad) throw ArgError("the det list contains duplicates");
+  if (bad && !allow_dup) throw ArgError("the det list contains duplicates");
 }
 
 size_t select_dets(shci_ctx* c, double eps_var, bool var_sd) {
