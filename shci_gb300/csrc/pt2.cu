@@ -66,13 +66,8 @@ struct StoSources {
   const double* weight;
   const uint32_t* batch;
   const uint8_t* is_dtm;
-  const uint32_t* remap;    // optional: launch source k' is source remap[k'] (re-runs)
   const uint32_t* ent_off;  // optional: entries of each source
 };
-
-__device__ __forceinline__ uint32_t src_index(const StoSources& S, uint32_t k) {
-  return S.remap ? S.remap[k] : k;
-}
 
 __device__ __forceinline__ uint32_t ent_begin(const StoSources& S, uint32_t k) {
   return S.ent_off ? S.ent_off[k] : k;
@@ -97,62 +92,32 @@ __device__ __forceinline__ uint64_t batch_of(const PtParams& Q, uint64_t h) {
   return r;
 }
 
-// Candidate a of source i belongs to the batch being computed (the first test of the
-// handler, solver.h:703-705: rehash(DetHasher(a)) % n_batches).  One batch: every candidate.
-__device__ __forceinline__ bool in_batch(const PtParams& Q, uint64_t batch, uint64_t cu,
-                                         uint64_t cd) {
-  return Q.n_batches <= 1 || batch_of(Q, rehash(det_hash(cu, cd))) == batch;
-}
-
 void set_batches(PtParams& Q, uint64_t n_batches) {
   Q.n_batches = n_batches;
   Q.batch_magic = n_batches ? ~0ull / n_batches : 0;
 }
 
-__device__ __forceinline__ uint64_t src_batch(const PtParams& Q, const StoSources& S, uint32_t k,
-                                              int mode) {
-  return mode == kSto ? S.batch[k] : Q.batch;
-}
-
-// Output slots of each source: its candidates in the current batch.
+// Window entries of each source: an upper bound of its candidates.
 template <int MODE>
 __global__ void __launch_bounds__(kPtWarps * 32, 4)
     k_pt_count(SelParams P, PtParams Q, StoSources S, uint32_t n_src, uint64_t* cnt_out) {
   const unsigned lane = threadIdx.x & 31;
   const uint32_t wpg = gridDim.x * kPtWarps;
   for (uint32_t k = blockIdx.x * kPtWarps + (threadIdx.x >> 5); k < n_src; k += wpg) {
-    const uint32_t kk = src_index(S, k);
-    const uint32_t i = src_det(S, kk, MODE);
+    const uint32_t i = src_det(S, k, MODE);
     const double ac = fabs(P.coef[i]);
     const double eps_min = Q.eps / ac;
     const double eps_max = 1.0e100 / ac;
     const uint64_t up = P.up[i], dn = P.dn[i];
     uint64_t tot = 0;
-    if (Q.n_batches <= 1) {
-      // every candidate counts: the slot ranges suffice
-      const int n_slots = P.n_elecs + P.n_pairs;
-      for (int s0 = 0; s0 < n_slots; s0 += 32) {
-        uint32_t lo = 0, c = 0;
-        if (s0 + (int)lane < n_slots) slot_range(P, up, dn, s0 + lane, eps_min, eps_max, &lo, &c);
-        uint64_t cc = c;
+    const int n_slots = P.n_elecs + P.n_pairs;
+    for (int s0 = 0; s0 < n_slots; s0 += 32) {
+      uint32_t lo = 0, c = 0;
+      if (s0 + (int)lane < n_slots) slot_range(P, up, dn, s0 + lane, eps_min, eps_max, &lo, &c);
+      uint64_t cc = c;
 #pragma unroll
-        for (int o = 16; o; o >>= 1) cc += __shfl_xor_sync(kFull, cc, o);
-        tot += cc;
-      }
-    } else if (MODE == kSto) {
-      // every entry of the source whose batch the candidate falls in
-      const uint32_t e0 = ent_begin(S, kk), e1 = ent_end(S, kk);
-      pt_walk(P, up, dn, eps_min, eps_max, [&](bool, bool ok, uint64_t cu, uint64_t cd) {
-        const uint64_t b = ok ? batch_of(Q, rehash(det_hash(cu, cd))) : ~0ull;
-        uint32_t m = 0;
-        for (uint32_t e = e0; e < e1; e++) m += b == S.batch[e] ? 1u : 0u;
-        tot += __reduce_add_sync(kFull, m);
-      });
-    } else {
-      const uint64_t batch = src_batch(Q, S, kk, MODE);
-      pt_walk(P, up, dn, eps_min, eps_max, [&](bool, bool ok, uint64_t cu, uint64_t cd) {
-        tot += __popc(__ballot_sync(kFull, ok && in_batch(Q, batch, cu, cd)));
-      });
+      for (int o = 16; o; o >>= 1) cc += __shfl_xor_sync(kFull, cc, o);
+      tot += cc;
     }
     if (lane == 0) cnt_out[k] = tot;
   }
@@ -207,63 +172,142 @@ __device__ __forceinline__ double h_one_fix(const SingleFix& F, uint64_t ui, uin
   return flip_sign(static_cast<double>(e) * F.inv_scale, move_parity(si, oi, oj));
 }
 
-constexpr uint32_t kPtQ = 64;  // per-warp queue of batch members (< 32 waiting + 32 pushed)
-struct PtQueue {
-  uint64_t u[kPtQ];
-  uint64_t d[kPtQ];
-  uint64_t pos[kPtQ];  // output slot of the member
-  uint32_t src[kPtQ];  // its source (launch-relative index k - k_begin)
-  uint8_t ent[kPtQ];   // stochastic stage: its entry within the source
+// A piece of a source's window: entries [begin, begin + len) of its slots' ranges in walk order.
+// Its members go to out[off[p], off[p] + cnt[p]), densely; cnt may come out larger than the
+// region, whose excess is then not written (the caller emits that piece again).
+struct PtPieces {
+  const uint32_t* src;
+  const uint32_t* begin;
+  const uint32_t* len;
+  const uint64_t* off;  // [n + 1]
+  uint32_t* cnt;
+  uint32_t n;
+  uint64_t base;  // off of the output arrays' first entry
 };
 
-// Emits the batch members of each source into its region [off[k], off[k + 1]) (one batch:
-// every index entry of the window, as counted by slot ranges).  A warp walks its sources one
-// after the other; members wait in a per-warp queue that carries them across sources (with
-// their source and output slot) and are finished 32 at a time (variational-set test,
-// H_ai c_i, the value columns), so the set search and the FP64 element run with full warps
-// even when most sources have only a few members.  Slots of members rejected there, of
-// entries that make no valid candidate, and the unused tail of a region are written invalid.
-// Members keep their walk order within their source's region.  A region may be sized by an
-// estimate (several batches): when the members do not fit, the queue is drained, the whole
-// region is written invalid and overflow[k] is set, and the caller emits that source again
-// with an exact count.
+// Entries a warp walks at most before the next piece: the heaviest determinant's window holds
+// 100,000 entries, 3,000 rounds of one warp.
+constexpr uint32_t kPieceLen = 4096;
+constexpr uint32_t kPtQ = 64;    // queue lengths (< 32 waiting + 32 pushed)
+constexpr uint32_t kPtSlots = 256;  // slots listed at a time
+
+struct PtWarp {
+  // slots of the current source with a non-empty range: first entry, entries, code
+  uint32_t s_lo[kPtSlots], s_cnt[kPtSlots], s_code[kPtSlots];
+  // stage 1 queue: entries whose targets are free
+  uint32_t a_rs[kPtQ], a_code[kPtQ], a_piece[kPtQ];
+  // stage 2 queue (several batches): members
+  uint64_t b_u[kPtQ], b_d[kPtQ];
+  uint32_t b_piece[kPtQ];
+  uint8_t b_ent[kPtQ];
+  uint8_t occ[128];  // electron -> spatial orbital, alpha electrons first
+};
+
+// Slot code: the strings that the targets r and s of an entry must be free in, and the orbitals
+// that the electrons leave.  A queue entry's r | s << 16 holds the targets of the stored pair; a
+// beta-beta pair is stored as its alpha image and an alpha-beta pair p > q as (q, p) (chem_system.cc:
+// 347-361), so the strings follow from the slot alone.
+enum : uint32_t { kADn = 1u << 16, kBDn = 1u << 17, kOne = 1u << 18 };
+
+// Entry range and code of slot `slot`; as slot_range (heatbath.cuh), the orbitals from `occ`.
+__device__ __forceinline__ uint32_t pt_slot(const SelParams& P, const uint8_t* occ, int slot,
+                                            double eps_min, double eps_max, uint32_t* lo,
+                                            uint32_t* cnt) {
+  *lo = 0;
+  *cnt = 0;
+  const int n = P.n_orbs;
+  if (slot < P.n_elecs) {
+    if (eps_min > P.max_singles) return 0;
+    const uint32_t p = occ[slot];
+    const uint32_t a = P.s_off[p], b = P.s_off[p + 1];
+    *lo = a;
+    *cnt = first_below(P.s_S, a, b, eps_min) - a;
+    return p | kOne | (slot < P.n_up ? 0u : kADn);
+  }
+  if (P.no_doubles || eps_min > P.max_hci) return 0;
+  const uint32_t pr = P.pair_tab[slot - P.n_elecs];
+  const int e1 = pr & 0xffff, e2 = pr >> 16;
+  const uint32_t p = occ[e1], q = occ[e2];
+  const bool dn1 = e1 >= P.n_up, dn2 = e2 >= P.n_up;
+  uint32_t code;
+  size_t pq;
+  if (dn1 == dn2) {
+    pq = c2(p, q);
+    code = p | (q << 8) | (dn1 ? kADn | kBDn : 0u);
+  } else if (p > q) {  // stored as (q, p + n): r goes to beta, s to alpha
+    pq = c2(q, p + n);
+    code = p | (q << 8) | kADn;
+  } else {
+    pq = c2(p, q + n);
+    code = p | (q << 8) | kBDn;
+  }
+  const uint32_t a = static_cast<uint32_t>(P.d_off[pq]), b = static_cast<uint32_t>(P.d_off[pq + 1]);
+  const uint32_t s = first_below(P.d_H, a, b, eps_max);
+  *lo = s;
+  *cnt = first_below(P.d_H, s, b, eps_min) - s;
+  return code;
+}
+
+__device__ __forceinline__ uint32_t bit_of(uint64_t x, uint32_t k) {
+  const uint32_t w = k & 32u ? static_cast<uint32_t>(x >> 32) : static_cast<uint32_t>(x);
+  return w >> (k & 31u) & 1u;
+}
+
+// Emits the members of each piece into its region: the window entries whose targets are free, that
+// fall in the current hash batch, are not variational and have |H_ai c_i| >= eps (the handler's
+// order, solver.h:703-713).  A warp takes a piece at a time.
+//
+// Most window entries go to occupied orbitals (four of five at n = 40, 10 alpha + 10 beta: the
+// large |H| couple neighbouring orbitals), and one candidate in n_batches is in the batch, so the
+// work is done in three stages, each on full warps: stage 1 tests the targets of 32 entries
+// against the source's strings and queues what passes; stage 2 builds 32 of those determinants and,
+// with several batches, hashes them and queues the members; the last stage evaluates 32 members.
+// Queues carry over from piece to piece.  Members keep their walk order within a piece.
+// At n = 40, 40,000 dets: 19.4 -> 4.6 ms deterministic (297M window entries), 11.3 -> 6.5 ms a
+// pseudo-stochastic batch of 16 (its hash is the work left: 56 % of issue), 21.4 -> 13.4 ms for six
+// stochastic iterations; n = 26, 30,000 dets: 5.3 -> 1.4 ms, of which the heaviest determinant's
+// window on one warp had been half.  (Before: build and hash at the walk, an output slot for
+// every window entry, a warp per source.)
 template <int MODE>
 __global__ void __launch_bounds__(kPtWarps * 32, 4)
-    k_pt_emit(SelParams P, PtParams Q, StoSources S, SingleFix F, uint32_t k_begin,
-              uint32_t k_end, const uint64_t* off, uint64_t* out_up, uint64_t* out_dn,
-              OutCols out, uint8_t* overflow) {
-  __shared__ PtQueue qs[kPtWarps];
-  PtQueue& q = qs[threadIdx.x >> 5];
+    k_pt_emit(SelParams P, PtParams Q, StoSources S, SingleFix F, PtPieces pc,
+              uint64_t* __restrict__ out_up, uint64_t* __restrict__ out_dn, OutCols out) {
+  extern __shared__ __align__(16) unsigned char pt_smem[];
+  PtWarp& W = reinterpret_cast<PtWarp*>(pt_smem)[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const uint32_t wpg = gridDim.x * kPtWarps;
-  uint32_t qh = 0, qn = 0;  // warp-uniform ring state, kept across sources
-  auto drain = [&](uint32_t m) {
-    __syncwarp();
-    if (lane < m) {
-      const uint32_t sl = (qh + lane) & (kPtQ - 1);
-      const uint64_t cu = q.u[sl], cd = q.d[sl], pos = q.pos[sl];
-      const uint32_t kk = src_index(S, k_begin + q.src[sl]);
+  const int n = P.n_orbs;
+  const uint32_t n_mask_off = static_cast<uint32_t>(n);
+  uint32_t ah = 0, an = 0, bh = 0, bn = 0;           // warp-uniform ring states
+  uint32_t run_piece = 0xffffffffu, run_cnt = 0;      // kept members of the last piece seen
+
+  // Last stage: evaluates the lanes' members (piece 0xffffffff: no member) and writes the kept
+  // ones.  A piece's members arrive in order, over one or several calls (one entry's, in the
+  // stochastic stage).
+  auto finish = [&](uint32_t piece, uint64_t cu, uint64_t cd, uint32_t ent) {
+    const bool act = piece != 0xffffffffu;
+    bool ok = false;
+    double hc = 0.0, count = 1.0, weight = 1.0;
+    bool dtm_src = true;
+    uint64_t iter_tag = 0;
+    if (act) {
+      const uint32_t kk = pc.src[piece];
       const uint32_t i = src_det(S, kk, MODE);
-      const uint64_t up = P.up[i], dn = P.dn[i];
-      const double coef = P.coef[i];
-      double count = 1.0, weight = 1.0;
-      bool dtm_src = true;
-      uint64_t iter_tag = 0;
       if (MODE == kSto) {
-        const uint32_t e = ent_begin(S, kk) + q.ent[sl];
+        const uint32_t e = ent_begin(S, kk) + ent;
         dtm_src = S.is_dtm[e] != 0;
         count = dtm_src ? 1.0 : S.count[e];
         weight = dtm_src ? 1.0 : S.weight[e];
         iter_tag = static_cast<uint64_t>(S.iter[e]) << Q.iter_shift;
       }
-      // handler order of solver.h:703-713: batch (done), variational set, |H_ai c_i|
-      bool ok = cu != kInvalid && !in_set(P, cu, cd);
-      double hc = 0.0;
+      ok = !in_set(P, cu, cd);
       // the pilot's handler tests |H_ai c_i| for single excitations only (solver.h:958-962)
-      const bool test = MODE != kSto || !Q.pilot || popc64(up ^ cu) + popc64(dn ^ cd) == 2;
-      if (ok && test) {
-        if (popc64(up ^ cu) + popc64(dn ^ cd) == 2) {  // single excitation
+      const uint64_t up = P.up[i], dn = P.dn[i];
+      const bool one = popc64(up ^ cu) + popc64(dn ^ cd) == 2;
+      if (ok && (MODE != kSto || !Q.pilot || one)) {
+        const double coef = P.coef[i];
+        if (one) {
           hc = h_one_fix(F, up, dn, cu, cd) * coef;
           const double a = fabs(hc), m = F.margin * fabs(coef);
           bool near = fabs(a - Q.eps) <= m;
@@ -275,88 +319,299 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
         }
         if (fabs(hc) < Q.eps) ok = false;
       }
-      out_up[pos] = ok ? (cu | iter_tag) : kInvalid;
-      out_dn[pos] = ok ? cd : kInvalid;
-      if (MODE == kDtm) {
-        out.v[0][pos] = hc;
-      } else if (MODE == kPsto) {
-        out.v[0][pos] = hc;
-        out.v[1][pos] = fabs(hc) >= Q.eps_dtm ? hc : 0.0;
-      } else {
-        // solver.h:1093-1103
-        const double x = count * hc / weight;
-        const bool above = fabs(hc) > Q.eps_psto;
-        double v2 = 0.0, v3 = 0.0, v4 = 0.0;
-        if (!dtm_src) {
-          v2 = count * hc / weight * sqrt(Q.factor);
-          if (above) v3 = v2;
-          else v4 = x * x * (1. - weight / count + Q.factor);
+    }
+    const unsigned keep = __ballot_sync(kFull, ok);
+    const unsigned mates = __match_any_sync(kFull, piece);
+    uint32_t before, after;
+    if (MODE == kSto) {
+      // members of several pieces alternate (an entry of each in turn): the count so far is read
+      const int lead = __ffs(mates) - 1;
+      before = 0;
+      if (act && static_cast<int>(lane) == lead)
+        before = atomicAdd(&pc.cnt[piece], static_cast<uint32_t>(__popc(keep & mates)));
+      before = __shfl_sync(kFull, before, lead);
+      after = 0;
+    } else {
+      before = piece == run_piece ? run_cnt : 0u;
+      after = before + __popc(keep & mates);
+    }
+    if (ok) {
+      uint64_t pos = pc.off[piece] + before + __popc(keep & mates & lt);
+      if (pos < pc.off[piece + 1]) {
+        pos -= pc.base;
+        out_up[pos] = cu | iter_tag;
+        out_dn[pos] = cd;
+        if (MODE == kDtm) {
+          out.v[0][pos] = hc;
+        } else if (MODE == kPsto) {
+          out.v[0][pos] = hc;
+          out.v[1][pos] = fabs(hc) >= Q.eps_dtm ? hc : 0.0;
+        } else {
+          // solver.h:1093-1103
+          const double x = count * hc / weight;
+          const bool above = fabs(hc) > Q.eps_psto;
+          double v2 = 0.0, v3 = 0.0, v4 = 0.0;
+          if (!dtm_src) {
+            v2 = count * hc / weight * sqrt(Q.factor);
+            if (above) v3 = v2;
+            else v4 = x * x * (1. - weight / count + Q.factor);
+          }
+          out.v[0][pos] = x;
+          out.v[1][pos] = above ? x : 0.0;
+          out.v[2][pos] = v2;
+          out.v[3][pos] = v3;
+          out.v[4][pos] = v4;
         }
-        out.v[0][pos] = x;
-        out.v[1][pos] = above ? x : 0.0;
-        out.v[2][pos] = v2;
-        out.v[3][pos] = v3;
-        out.v[4][pos] = v4;
       }
     }
-    __syncwarp();
-    qh += m;
-    qn -= m;
+    if (MODE != kSto) {
+      if (act && lane == 31u - __clz(mates)) pc.cnt[piece] = after;  // the running count
+      const int last = 31 - __clz(__ballot_sync(kFull, act));
+      run_piece = __shfl_sync(kFull, piece, last);
+      run_cnt = __shfl_sync(kFull, after, last);
+    }
   };
-  for (uint32_t k = k_begin + blockIdx.x * kPtWarps + (threadIdx.x >> 5); k < k_end; k += wpg) {
-    const uint32_t kl = k - k_begin;
-    const uint32_t kk = src_index(S, k);
+
+  auto drain_b = [&](uint32_t m) {
+    __syncwarp();
+    const uint32_t sl = (bh + lane) & (kPtQ - 1);
+    const bool act = lane < m;
+    const uint32_t piece = act ? W.b_piece[sl] : 0xffffffffu;
+    const uint64_t cu = act ? W.b_u[sl] : 0, cd = act ? W.b_d[sl] : 0;
+    const uint32_t ent = act ? W.b_ent[sl] : 0;
+    __syncwarp();
+    bh += m;
+    bn -= m;
+    finish(piece, cu, cd, ent);
+  };
+
+  // Stage 2: the m oldest entries of stage 1's queue.
+  auto drain_a = [&](uint32_t m) {
+    __syncwarp();
+    const uint32_t sl = (ah + lane) & (kPtQ - 1);
+    const bool act = lane < m;
+    const uint32_t piece = act ? W.a_piece[sl] : 0xffffffffu;
+    const uint32_t code = act ? W.a_code[sl] : 0u, rs = act ? W.a_rs[sl] : 0u;
+    __syncwarp();
+    ah += m;
+    an -= m;
+    uint64_t cu = 0, cd = 0;
+    uint32_t kk = 0;
+    if (act) {
+      kk = pc.src[piece];
+      const uint32_t i = src_det(S, kk, MODE);
+      cu = P.up[i];
+      cd = P.dn[i];
+      const uint64_t out1 = 1ull << (code & 0xffu), out2 = 1ull << (code >> 8 & 0xffu);
+      const uint64_t in1 = 1ull << (rs & 0xffffu), in2 = 1ull << (rs >> 16);
+      // (targets are in the strings A and B; the electrons that leave: of the first electron's
+      // string and the second's, which for a swapped pair are B and A)
+      const bool a_dn = code & kADn, b_dn = code & kBDn;
+      if (code & kOne) {
+        if (a_dn) cd ^= out1 | in1;
+        else cu ^= out1 | in1;
+      } else if (a_dn == b_dn) {
+        const uint64_t x = out1 | out2 | in1 | in2;
+        if (a_dn) cd ^= x;
+        else cu ^= x;
+      } else {
+        cu ^= out1 | (a_dn ? in2 : in1);
+        cd ^= out2 | (a_dn ? in1 : in2);
+      }
+    }
+    if (Q.n_batches <= 1) {
+      if (MODE != kSto) {
+        finish(piece, cu, cd, 0);
+        return;
+      }
+    }
+    const uint64_t b = act && Q.n_batches > 1 ? batch_of(Q, rehash(det_hash(cu, cd))) : 0ull;
+    uint32_t e0 = 0, ne = act ? 1u : 0u;
+    if (MODE == kSto && act) {
+      e0 = ent_begin(S, kk);
+      ne = ent_end(S, kk) - e0;
+    }
+    const uint32_t most = MODE == kSto ? __reduce_max_sync(kFull, ne) : 1u;
+    for (uint32_t e = 0; e < most; e++) {
+      const bool mine =
+          e < ne && (Q.n_batches <= 1 || b == (MODE == kSto ? S.batch[e0 + e] : Q.batch));
+      const unsigned bal = __ballot_sync(kFull, mine);
+      if (!bal) continue;
+      if (mine) {
+        const uint32_t t = (bh + bn + __popc(bal & lt)) & (kPtQ - 1);
+        W.b_u[t] = cu;
+        W.b_d[t] = cd;
+        W.b_piece[t] = piece;
+        W.b_ent[t] = static_cast<uint8_t>(e);
+      }
+      bn += __popc(bal);
+      if (bn >= 32u) drain_b(32u);
+    }
+  };
+
+  for (uint32_t piece = blockIdx.x * kPtWarps + (threadIdx.x >> 5); piece < pc.n; piece += wpg) {
+    const uint32_t kk = pc.src[piece];
+    uint32_t skip = pc.begin[piece], left = pc.len[piece];
     const uint32_t i = src_det(S, kk, MODE);
     const double ac = fabs(P.coef[i]);
     const double eps_min = Q.eps / ac;
     const double eps_max = 1.0e100 / ac;
     const uint64_t up = P.up[i], dn = P.dn[i];
-    const uint64_t batch = MODE == kSto ? 0 : src_batch(Q, S, kk, MODE);
-    const uint32_t e0 = MODE == kSto ? ent_begin(S, kk) : 0u;
-    const uint32_t e1 = MODE == kSto ? ent_end(S, kk) : 1u;
-    const uint64_t start = off[kl], limit = off[kl + 1];
-    uint64_t cnt = 0;   // members of this source so far (warp-uniform)
-    bool over = false;  // warp-uniform
-    // queue the lanes with mine set (members of entry ent), each with its output slot
-    auto push = [&](bool mine, bool ok, uint64_t cu, uint64_t cd, uint32_t ent) {
-      const unsigned bal = __ballot_sync(kFull, mine);
-      if (!bal) return;
-      const uint32_t nb = __popc(bal);
-      if (start + cnt + nb > limit) over = true;
-      if (!over && mine) {
-        const uint32_t sl = (qh + qn + __popc(bal & lt)) & (kPtQ - 1);
-        q.u[sl] = ok ? cu : kInvalid;
-        q.d[sl] = ok ? cd : kInvalid;
-        q.pos[sl] = start + cnt + __popc(bal & lt);
-        q.src[sl] = kl;
-        q.ent[sl] = static_cast<uint8_t>(ent);
+    const uint64_t bu = up | P.inactive, bd = dn | P.inactive;  // (inactive targets: active space)
+    __syncwarp();
+    for (int o = lane; o < n; o += 32) {
+      if (up >> o & 1) W.occ[popc64(up & below(o))] = static_cast<uint8_t>(o);
+      if (dn >> o & 1) W.occ[P.n_up + popc64(dn & below(o))] = static_cast<uint8_t>(o);
+    }
+    __syncwarp();
+    const int n_slots = P.n_elecs + P.n_pairs;
+    for (int f0 = 0; f0 < n_slots && left; f0 += kPtSlots) {
+      // the non-empty slots of this stretch
+      uint32_t m = 0;
+      const int f1 = min(n_slots, f0 + (int)kPtSlots);
+      for (int s0 = f0; s0 < f1; s0 += 32) {
+        uint32_t lo = 0, c = 0, code = 0;
+        if (s0 + (int)lane < f1)
+          code = pt_slot(P, W.occ, s0 + lane, eps_min, eps_max, &lo, &c);
+        const unsigned bal = __ballot_sync(kFull, c != 0);
+        if (c) {
+          const uint32_t k = m + __popc(bal & lt);
+          W.s_lo[k] = lo;
+          W.s_cnt[k] = c;
+          W.s_code[k] = code;
+        }
+        m += __popc(bal);
       }
-      if (!over) qn += nb;
-      cnt += nb;
-      if (qn >= 32u) drain(32u);
-    };
-    pt_walk(P, up, dn, eps_min, eps_max, [&](bool slot, bool ok, uint64_t cu, uint64_t cd) {
-      if (MODE == kSto) {
-        // hash once, then one member per entry whose batch the candidate falls in
-        const uint64_t b =
-            (ok && Q.n_batches > 1) ? batch_of(Q, rehash(det_hash(cu, cd))) : 0ull;
-        for (uint32_t e = e0; e < e1; e++)
-          push(Q.n_batches <= 1 ? slot : (ok && b == S.batch[e]), ok, cu, cd, e - e0);
-        return;
+      __syncwarp();
+      for (uint32_t g = 0; g < m && left; g += 32) {
+        const uint32_t k = g + lane;
+        const uint32_t c = k < m ? W.s_cnt[k] : 0u;
+        uint32_t inc = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t t = __shfl_up_sync(kFull, inc, o);
+          if (lane >= (unsigned)o) inc += t;
+        }
+        const uint32_t total = __shfl_sync(kFull, inc, 31);
+        if (skip >= total) {
+          skip -= total;
+          continue;
+        }
+        const uint32_t end = min(total, skip + left);
+        left -= end - skip;
+        const uint32_t first = inc - c;  // of this lane's slot
+        for (uint32_t t0 = skip; t0 < end; t0 += 32) {
+          const uint32_t t = t0 + lane;
+          uint32_t ol = 0;  // owner: the number of slots that end at or before t
+#pragma unroll
+          for (uint32_t step = 16; step; step >>= 1) {
+            const uint32_t v = __shfl_sync(kFull, inc, ol + step - 1);
+            if (v <= t) ol += step;
+          }
+          const uint32_t o_first = __shfl_sync(kFull, first, ol);
+          bool pass = false;
+          uint32_t rs = 0, code = 0;
+          if (t < end) {
+            code = W.s_code[g + ol];
+            const uint32_t e = W.s_lo[g + ol] + (t - o_first);
+            const uint64_t A = code & kADn ? bd : bu;
+            if (code & kOne) {
+              rs = P.s_r[e];
+              pass = !bit_of(A, rs);
+            } else {
+              rs = P.d_rs[e];
+              const uint64_t B = code & kBDn ? bd : bu;
+              uint32_t x = rs >> 16;
+              if (x >= n_mask_off) x -= n_mask_off;
+              rs = (rs & 0xffffu) | (x << 16);
+              pass = !(bit_of(A, rs & 0xffffu) | bit_of(B, x));
+            }
+          }
+          const unsigned bal = __ballot_sync(kFull, pass);
+          if (!bal) continue;
+          if (pass) {
+            const uint32_t q = (ah + an + __popc(bal & lt)) & (kPtQ - 1);
+            W.a_rs[q] = rs;
+            W.a_code[q] = code;
+            W.a_piece[q] = piece;
+          }
+          an += __popc(bal);
+          if (an >= 32u) drain_a(32u);
+        }
+        skip = 0;
       }
-      push(Q.n_batches <= 1 ? slot : (ok && in_batch(Q, batch, cu, cd)), ok, cu, cd, 0u);
-    });
-    if (over) {
-      // members of this source may still wait in the queue: finish them, then void the region
-      while (qn) drain(qn < 32u ? qn : 32u);
-      for (uint64_t p = start + lane; p < limit; p += 32) out_up[p] = kInvalid;
-      if (lane == 0) overflow[kl] = 1;
-    } else {
-      // the region's unused tail (the members' slots are below start + cnt)
-      for (uint64_t p = start + cnt + lane; p < limit; p += 32) out_up[p] = kInvalid;
+      __syncwarp();
     }
   }
-  while (qn) drain(qn < 32u ? qn : 32u);
+  while (an) drain_a(an < 32u ? an : 32u);
+  while (bn) drain_b(bn < 32u ? bn : 32u);
+}
+
+// Pieces per source, and the pieces with their region sizes (into off[p], to be scanned): every
+// entry with one batch; with several, a piece's members are a binomial(len, 1 / n_batches) count
+// per entry of the source (a det walked once for several iterations), and len / n_batches * slack +
+// pad exceeds its mean by many standard deviations (pieces that overflow are emitted again).
+__global__ void k_piece_count(const uint64_t* __restrict__ entries, uint32_t n_src, uint32_t* np) {
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src; k += gridDim.x * blockDim.x)
+    np[k] = static_cast<uint32_t>((entries[k] + kPieceLen - 1) / kPieceLen);
+}
+__global__ void k_piece_fill(const uint64_t* __restrict__ entries, const uint32_t* __restrict__ first,
+                             uint32_t n_src, uint64_t n_batches, double slack, double pad,
+                             const uint32_t* __restrict__ ent_off, uint32_t* __restrict__ src,
+                             uint32_t* __restrict__ begin, uint32_t* __restrict__ len,
+                             uint64_t* __restrict__ off) {
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src;
+       k += gridDim.x * blockDim.x) {
+    const uint64_t m = entries[k];
+    const uint64_t mult = ent_off ? ent_off[k + 1] - ent_off[k] : 1u;
+    uint32_t p = first[k];
+    for (uint64_t b = 0; b < m; b += kPieceLen, p++) {
+      const uint64_t l = min(static_cast<unsigned long long>(kPieceLen),
+                             static_cast<unsigned long long>(m - b));
+      uint64_t r = l * mult;
+      if (n_batches > 1) {
+        const double est = ceil(static_cast<double>(r) / static_cast<double>(n_batches) * slack + pad);
+        if (est < static_cast<double>(r)) r = est > 0.0 ? static_cast<uint64_t>(est) : 0ull;
+      }
+      src[p] = k;
+      begin[p] = static_cast<uint32_t>(b);  // (a source's windows hold fewer than 2^32 entries)
+      len[p] = static_cast<uint32_t>(l);
+      off[p] = r;
+    }
+  }
+}
+
+// Members of each piece that were written: none of one whose region was too small (*over counts
+// those).
+__global__ void k_pt_kept(const uint32_t* __restrict__ cnt, const uint64_t* __restrict__ off,
+                          uint32_t n, uint64_t* __restrict__ kept, unsigned* over) {
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+    const bool fits = cnt[p] <= off[p + 1] - off[p];
+    kept[p] = fits ? cnt[p] : 0u;
+    if (!fits) atomicAdd(over, 1u);
+  }
+}
+
+// Copies each piece's members from its region to dst[p] (eight lanes a piece: most pieces hold
+// a few members when there are many batches).
+template <int NV>
+__global__ void __launch_bounds__(256)
+    k_pt_collect(const uint64_t* __restrict__ off, uint64_t base, const uint64_t* __restrict__ dst,
+                 const uint64_t* __restrict__ total, uint32_t n, const uint64_t* __restrict__ u,
+                 const uint64_t* __restrict__ d, OutCols v, uint64_t* __restrict__ ou,
+                 uint64_t* __restrict__ od, OutCols ov) {
+  const unsigned sub = threadIdx.x & 7;
+  const uint32_t step = gridDim.x * (blockDim.x >> 3);
+  for (uint32_t p = blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3); p < n; p += step) {
+    const uint64_t a = off[p] - base, b = dst[p];
+    const uint64_t m = (p + 1 < n ? dst[p + 1] : *total) - b;
+    for (uint64_t k = sub; k < m; k += 8) {
+      ou[b + k] = u[a + k];
+      od[b + k] = d[a + k];
+#pragma unroll
+      for (int c = 0; c < NV; c++) ov.v[c][b + k] = v.v[c][a + k];
+    }
+  }
 }
 
 // Diagonal H_aa of the PT dets in 64-bit fixed point.  The diagonal is a sum of about
@@ -661,109 +916,199 @@ constexpr int n_cols() {
   return MODE == kDtm ? 1 : MODE == kPsto ? 2 : 5;
 }
 
-// Emits the pairs of the sources [0, n_src) for one batch (or set of iterations), appending
-// the valid ones to (bu, bd, bv) after the first *bn; slots[k] = the size of source k's
-// region.  Sources whose region overflowed (regions sized by an estimate) are appended to
-// *over as launch indices.  The accumulation is sorted and reduced in place whenever it
-// grows past kCap, to keep it bounded.
+// Pieces of a set of sources (on the device); piece p's region is [off[p], off[p + 1]).
+struct PieceList {
+  DevBuf<uint32_t> src, begin, len;
+  DevBuf<uint64_t> off;
+  size_t n = 0;
+  uint64_t tot = 0;
+  explicit PieceList(shci_ctx* c) {
+    src.mt = begin.mt = len.mt = &c->mem;
+    off.mt = &c->mem;
+  }
+};
+// Pieces by host arrays (those to be emitted again), with exact sizes.
+struct PieceRerun {
+  std::vector<uint32_t> src, begin, len;
+  std::vector<uint64_t> off{0};
+};
+
+// Pieces of the sources with `entries` window entries each (device; ent_off as in StoSources).
+// SHCI_PT_SLOTS="slack,pad" replaces the region estimate's 1.3 and 64.
+void make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src, uint64_t n_batches,
+                 const uint32_t* ent_off, PieceList& L) {
+  double slack = 1.3, pad = 64.0;
+  if (const char* e = std::getenv("SHCI_PT_SLOTS")) std::sscanf(e, "%lf,%lf", &slack, &pad);
+  cudaStream_t s = c->stream;
+  L.n = 0;
+  L.tot = 0;
+  if (n_src == 0) return;
+  HostScope hs(c->prof, "pt2_host_offsets");
+  DevBuf<uint32_t> first;
+  first.mt = &c->mem;
+  first.resize(n_src);
+  k_piece_count<<<grid_for(n_src, 256), 256, 0, s>>>(entries.p, n_src, first.p);
+  SHCI_LAUNCH_CHECK();
+  L.n = exclusive_scan_u32(first.p, first.p, n_src, s, c->sort);
+  c->launches += 4;
+  if (L.n == 0) return;
+  L.src.resize(L.n);
+  L.begin.resize(L.n);
+  L.len.resize(L.n);
+  L.off.resize(L.n + 1);
+  k_piece_fill<<<grid_for(n_src, 256), 256, 0, s>>>(entries.p, first.p, n_src, n_batches, slack,
+                                                    pad, ent_off, L.src.p, L.begin.p, L.len.p,
+                                                    L.off.p);
+  SHCI_LAUNCH_CHECK();
+  exclusive_scan_u64_async(L.off.p, L.off.p, L.n, s, c->sort, L.off.p + L.n);
+  SHCI_CUDA(cudaMemcpyAsync(&L.tot, L.off.p + L.n, 8, cudaMemcpyDeviceToHost, s));
+  SHCI_CUDA(cudaStreamSynchronize(s));
+}
+
+// Emits the members of the pieces for one batch (or set of iterations), appending them to (bu, bd,
+// bv) after the first *bn.  Pieces whose region overflowed are appended to *over with their
+// exact sizes.  The accumulation is sorted and reduced in place whenever it grows past kCap, to
+// keep it bounded.
 template <int MODE>
 void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSources& S,
-                    uint32_t n_src, const std::vector<uint64_t>& slots, DevBuf<uint64_t>& bu,
-                    DevBuf<uint64_t>& bd, DevBuf<double>* bv, size_t* bn, int a_bits,
-                    std::vector<uint32_t>* over) {
+                    const PieceList& L, DevBuf<uint64_t>& bu, DevBuf<uint64_t>& bd,
+                    DevBuf<double>* bv, size_t* bn, int a_bits, PieceRerun* over) {
   constexpr int NV = n_cols<MODE>();
   cudaStream_t s = c->stream;
   const uint64_t kCap = 1ull << 27;
-  DevBuf<uint64_t> cu, cd;
+  DevBuf<uint64_t> cu, cd, d_dst;
+  DevBuf<uint32_t> d_cnt;
   DevBuf<double> cv[NV];
-  DevBuf<uint8_t> d_over;
-  cu.mt = cd.mt = &c->mem;
-  d_over.mt = &c->mem;
+  cu.mt = cd.mt = d_dst.mt = &c->mem;
+  d_cnt.mt = &c->mem;
   for (int v = 0; v < NV; v++) cv[v].mt = &c->mem;
-  uint32_t k0 = 0;
-  while (k0 < n_src) {
-    uint64_t tot = 0;
-    uint32_t k1 = k0;
-    while (k1 < n_src && (k1 == k0 || tot + slots[k1] <= kCap)) tot += slots[k1++];
-    if (tot > 0) {
-      HostScope hs_off(c->prof, "pt2_host_offsets");
-      std::vector<uint64_t> off(k1 - k0 + 1);
-      uint64_t acc = 0;
-      for (uint32_t k = k0; k < k1; k++) {
-        off[k - k0] = acc;
-        acc += slots[k];
+  const SingleFix F = single_fix(c);
+  const size_t smem = sizeof(PtWarp) * kPtWarps;
+  SHCI_CUDA(cudaFuncSetAttribute(k_pt_emit<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(smem)));
+  size_t k0 = 0;
+  uint64_t base = 0;  // off[k0]
+  auto off_at = [&](size_t k) {
+    uint64_t v = 0;
+    SHCI_CUDA(cudaMemcpyAsync(&v, L.off.p + k, 8, cudaMemcpyDeviceToHost, s));
+    SHCI_CUDA(cudaStreamSynchronize(s));
+    return v;
+  };
+  while (k0 < L.n) {
+    // the pieces whose regions fit kCap together: all of them, or up to the last whose end does
+    // (one at least)
+    size_t k1 = L.n;
+    uint64_t end = L.tot;
+    if (end - base > kCap) {
+      size_t lo = k0 + 1, hi = L.n;  // off[lo] is taken in any case; off[hi] - base > kCap
+      while (lo + 1 < hi) {
+        const size_t mid = lo + (hi - lo) / 2;
+        if (off_at(mid) - base <= kCap) lo = mid;
+        else hi = mid;
       }
-      off[k1 - k0] = acc;
-      DevBuf<uint64_t> d_off;
-      d_off.mt = &c->mem;
-      d_off.resize(off.size());
-      SHCI_CUDA(cudaMemcpyAsync(d_off.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice, s));
-      hs_off.stop();
-      d_over.resize(k1 - k0);
-      SHCI_CUDA(cudaMemsetAsync(d_over.p, 0, k1 - k0, s));
-      cu.resize(tot, 1.25);
-      cd.resize(tot, 1.25);
-      OutCols oc{};
-      const double* vptr[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-      for (int v = 0; v < NV; v++) {
-        cv[v].resize(tot, 1.25);
-        oc.v[v] = cv[v].p;
-        vptr[v] = cv[v].p;
-      }
-      {
-        ProfScope ps(c->prof, s, "pt2_emit");
-        k_pt_emit<MODE><<<st.grid, kPtWarps * 32, 0, s>>>(st.P, Q, S, single_fix(c), k0, k1,
-                                                          d_off.p, cu.p, cd.p, oc, d_over.p);
-        SHCI_LAUNCH_CHECK();
-      }
-      c->launches += 1;
-      {
-        ProfScope ps(c->prof, s, "pt2_compact");
-        compact_valid(c, cu.p, cd.p, vptr, NV, tot, bu, bd, bv, bn);
-      }
-      std::vector<uint8_t> h_over(k1 - k0);
-      SHCI_CUDA(cudaMemcpyAsync(h_over.data(), d_over.p, k1 - k0, cudaMemcpyDeviceToHost, s));
+      k1 = lo;
+      end = off_at(k1);
+    }
+    const uint64_t tot = end - base;
+    const uint32_t n = static_cast<uint32_t>(k1 - k0);
+    d_cnt.resize((size_t)n + 1);  // (the overflow count after the pieces')
+    d_dst.resize((size_t)n + 1);
+    SHCI_CUDA(cudaMemsetAsync(d_cnt.p, 0, ((size_t)n + 1) * 4, s));
+    cu.resize(std::max<uint64_t>(tot, 1), 1.25);
+    cd.resize(std::max<uint64_t>(tot, 1), 1.25);
+    OutCols oc{};
+    for (int v = 0; v < NV; v++) {
+      cv[v].resize(std::max<uint64_t>(tot, 1), 1.25);
+      oc.v[v] = cv[v].p;
+    }
+    const PtPieces pc{L.src.p + k0, L.begin.p + k0, L.len.p + k0, L.off.p + k0, d_cnt.p, n, base};
+    {
+      ProfScope ps(c->prof, s, "pt2_emit");
+      k_pt_emit<MODE><<<grid_for((size_t)n * 32, kPtWarps * 32, st.grid), kPtWarps * 32, smem, s>>>(
+          st.P, Q, S, F, pc, cu.p, cd.p, oc);
+      SHCI_LAUNCH_CHECK();
+    }
+    uint64_t got = 0;
+    unsigned n_over = 0;
+    {
+      ProfScope ps(c->prof, s, "pt2_compact");
+      k_pt_kept<<<grid_for(n, 256), 256, 0, s>>>(d_cnt.p, pc.off, n, d_dst.p, d_cnt.p + n);
+      SHCI_LAUNCH_CHECK();
+      exclusive_scan_u64_async(d_dst.p, d_dst.p, n, s, c->sort, d_dst.p + n);
+      SHCI_CUDA(cudaMemcpyAsync(&got, d_dst.p + n, 8, cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaMemcpyAsync(&n_over, d_cnt.p + n, 4, cudaMemcpyDeviceToHost, s));
       SHCI_CUDA(cudaStreamSynchronize(s));
-      for (uint32_t k = k0; k < k1; k++)
-        if (h_over[k - k0]) over->push_back(k);
-      if (*bn > kCap) {  // keep the accumulation buffer bounded
-        *bn = sort_unique_pairs(c, bu, bd, *bn, bv, NV, a_bits);
+      if (got) {
         bu.n = bd.n = *bn;
+        bu.grow_keep(*bn + got, s);
+        bd.grow_keep(*bn + got, s);
+        OutCols ov{};
+        for (int v = 0; v < NV; v++) {
+          bv[v].n = *bn;
+          bv[v].grow_keep(*bn + got, s);
+          ov.v[v] = bv[v].p + *bn;
+        }
+        k_pt_collect<NV><<<grid_for((size_t)n * 8, 256), 256, 0, s>>>(
+            pc.off, base, d_dst.p, d_dst.p + n, n, cu.p, cd.p, oc, bu.p + *bn, bd.p + *bn, ov);
+        SHCI_LAUNCH_CHECK();
+        *bn += got;
       }
     }
+    c->launches += 5;
+    if (n_over) {
+      std::vector<uint32_t> cnt(n), src(n), begin(n), len(n);
+      std::vector<uint64_t> off((size_t)n + 1);
+      SHCI_CUDA(cudaMemcpyAsync(cnt.data(), d_cnt.p, n * 4ull, cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaMemcpyAsync(src.data(), pc.src, n * 4ull, cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaMemcpyAsync(begin.data(), pc.begin, n * 4ull, cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaMemcpyAsync(len.data(), pc.len, n * 4ull, cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaMemcpyAsync(off.data(), pc.off, (n + 1ull) * 8, cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaStreamSynchronize(s));
+      for (uint32_t k = 0; k < n; k++)
+        if (cnt[k] > off[k + 1] - off[k]) {
+          over->src.push_back(src[k]);
+          over->begin.push_back(begin[k]);
+          over->len.push_back(len[k]);
+          over->off.push_back(over->off.back() + cnt[k]);
+        }
+    }
+    if (*bn > kCap) {  // keep the accumulation buffer bounded
+      *bn = sort_unique_pairs(c, bu, bd, *bn, bv, NV, a_bits);
+      bu.n = bd.n = *bn;
+    }
     k0 = k1;
+    base = end;
   }
 }
 
-template <int MODE>
-std::vector<uint64_t> pt_counts(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSources& S,
-                                uint32_t n_src);
-
-// Emits and reduces the pairs of the sources [0, n_src) for one batch / set of iterations;
-// returns the unique count, keys in (bu, bd) and value columns in bv[0..n_cols).  slots are
-// exact counts or estimates; sources whose estimated region overflowed are emitted again,
-// after the others, with exact counts.
+// Emits and reduces the members of the pieces for one batch / set of iterations; returns the
+// unique count, keys in (bu, bd) and value columns in bv[0..n_cols).  Pieces whose estimated
+// region overflowed are emitted again, after the others, with the sizes they turned out to have.
 template <int MODE>
 size_t pt_emit_reduce(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSources& S,
-                      uint32_t n_src, const std::vector<uint64_t>& slots, DevBuf<uint64_t>& bu,
-                      DevBuf<uint64_t>& bd, DevBuf<double>* bv, int a_bits) {
+                      const PieceList& L, DevBuf<uint64_t>& bu, DevBuf<uint64_t>& bd,
+                      DevBuf<double>* bv, int a_bits) {
   constexpr int NV = n_cols<MODE>();
   cudaStream_t s = c->stream;
   size_t bn = 0;
-  std::vector<uint32_t> over;
-  pt_emit_append<MODE>(c, st, Q, S, n_src, slots, bu, bd, bv, &bn, a_bits, &over);
-  if (!over.empty()) {
-    DevBuf<uint32_t> remap;
-    remap.mt = &c->mem;
-    remap.resize(over.size());
-    SHCI_CUDA(cudaMemcpyAsync(remap.p, over.data(), over.size() * 4, cudaMemcpyHostToDevice, s));
-    StoSources S2 = S;
-    S2.remap = remap.p;
-    const uint32_t n2 = static_cast<uint32_t>(over.size());
-    const std::vector<uint64_t> exact = pt_counts<MODE>(c, st, Q, S2, n2);
-    std::vector<uint32_t> over2;
-    pt_emit_append<MODE>(c, st, Q, S2, n2, exact, bu, bd, bv, &bn, a_bits, &over2);
-    if (!over2.empty()) throw std::logic_error("PT2 emission: exact regions overflowed");
+  PieceRerun over;
+  pt_emit_append<MODE>(c, st, Q, S, L, bu, bd, bv, &bn, a_bits, &over);
+  if (!over.src.empty()) {
+    PieceList again(c);
+    const size_t n = again.n = over.src.size();
+    again.tot = over.off.back();
+    again.src.resize(n);
+    again.begin.resize(n);
+    again.len.resize(n);
+    again.off.resize(n + 1);
+    SHCI_CUDA(cudaMemcpyAsync(again.src.p, over.src.data(), n * 4, cudaMemcpyHostToDevice, s));
+    SHCI_CUDA(cudaMemcpyAsync(again.begin.p, over.begin.data(), n * 4, cudaMemcpyHostToDevice, s));
+    SHCI_CUDA(cudaMemcpyAsync(again.len.p, over.len.data(), n * 4, cudaMemcpyHostToDevice, s));
+    SHCI_CUDA(cudaMemcpyAsync(again.off.p, over.off.data(), (n + 1) * 8, cudaMemcpyHostToDevice, s));
+    SHCI_CUDA(cudaStreamSynchronize(s));
+    PieceRerun over2;
+    pt_emit_append<MODE>(c, st, Q, S, again, bu, bd, bv, &bn, a_bits, &over2);
+    if (!over2.src.empty()) throw std::logic_error("PT2 emission: exact regions overflowed");
   }
   {
     ProfScope ps(c->prof, s, "pt2_reduce");
@@ -773,47 +1118,19 @@ size_t pt_emit_reduce(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSour
   return bn;
 }
 
-// Region sizes from bounds (each source's window entries, an exact count with one batch):
-// with several batches a source's members are a binomial(bound, 1 / n_batches) count, and
-// bound / n_batches * 1.3 + 64 exceeds its mean by many standard deviations (overflowing
-// sources are re-run exactly).  SHCI_PT_SLOTS="slack,pad" replaces 1.3 and 64.
-std::vector<uint64_t> region_slots(const std::vector<uint64_t>& bound, uint64_t n_batches,
-                                   const std::vector<uint32_t>* mult = nullptr) {
-  // mult[k]: entries of source k (a det walked once for several iterations)
-  double slack = 1.3, pad = 64.0;
-  if (const char* e = std::getenv("SHCI_PT_SLOTS")) std::sscanf(e, "%lf,%lf", &slack, &pad);
-  std::vector<uint64_t> r(bound.size());
-  for (size_t k = 0; k < bound.size(); k++) {
-    const uint64_t full = bound[k] * (mult ? (*mult)[k] : 1u);
-    if (n_batches <= 1) {
-      r[k] = full;
-      continue;
-    }
-    const double est = std::ceil(static_cast<double>(full) / n_batches * slack + pad);
-    r[k] = std::min<uint64_t>(full, static_cast<uint64_t>(std::max(0.0, est)));
-  }
-  return r;
-}
-
+// Window entries of each source (device).
 template <int MODE>
-std::vector<uint64_t> pt_counts(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSources& S,
-                                uint32_t n_src) {
+void pt_counts(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSources& S, uint32_t n_src,
+               DevBuf<uint64_t>& cnt) {
   cudaStream_t s = c->stream;
-  DevBuf<uint64_t> cnt;
   cnt.mt = &c->mem;
   cnt.resize(n_src ? n_src : 1);
-  std::vector<uint64_t> hc(n_src);
-  if (n_src) {
-    {
-      ProfScope ps(c->prof, s, "pt2_count");
-      k_pt_count<MODE><<<st.grid, kPtWarps * 32, 0, s>>>(st.P, Q, S, n_src, cnt.p);
-      SHCI_LAUNCH_CHECK();
-    }
-    SHCI_CUDA(cudaMemcpyAsync(hc.data(), cnt.p, n_src * 8, cudaMemcpyDeviceToHost, s));
-    SHCI_CUDA(cudaStreamSynchronize(s));
-    c->launches += 1;
-  }
-  return hc;
+  if (!n_src) return;
+  ProfScope ps(c->prof, s, "pt2_count");
+  k_pt_count<MODE><<<grid_for((size_t)n_src * 32, kPtWarps * 32, st.grid), kPtWarps * 32, 0, s>>>(
+      st.P, Q, S, n_src, cnt.p);
+  SHCI_LAUNCH_CHECK();
+  c->launches += 1;
 }
 
 // Sum and sum of squares of the contributions of one reduced batch (dtm / psto).
@@ -857,16 +1174,21 @@ Pt2Out pt_batched(shci_ctx* c, double e_var, PtParams Q, size_t n_batches, doubl
   pt_setup(c, st);
   const uint32_t n_var = static_cast<uint32_t>(c->up.size());
   StoSources S{};
-  // slots per source over all batches (sizes the automatic batch count)
-  set_batches(Q, 1);
+  // window entries per source (size the automatic batch count and the regions)
   Q.batch = 0;
-  std::vector<uint64_t> hc = pt_counts<MODE>(c, st, Q, S, n_var);
+  DevBuf<uint64_t> entries;
+  pt_counts<MODE>(c, st, Q, S, n_var, entries);
   if (n_batches == 0) {
     // Automatic batch count: every candidate pair costs ~48 device bytes while a batch is
     // processed (keys, value columns, compaction, sort ping-pong); keep a batch within 40% of
     // the free HBM.  (The dtm energy does not depend on the batch count.)
     uint64_t tot = 0;
-    for (uint64_t v : hc) tot += v;
+    {
+      DevBuf<uint64_t> sum;
+      sum.mt = &c->mem;
+      sum.resize(n_var);
+      tot = exclusive_scan_u64(entries.p, sum.p, n_var, c->stream, c->sort);
+    }
     size_t free_b = 0, total_b = 0;
     SHCI_CUDA(cudaMemGetInfo(&free_b, &total_b));
     free_b += c->mem.cached;  // cached blocks return to the driver on demand
@@ -875,8 +1197,9 @@ Pt2Out pt_batched(shci_ctx* c, double e_var, PtParams Q, size_t n_batches, doubl
     if (n_batches < 1) n_batches = 1;
   }
   set_batches(Q, n_batches);
-  // regions per source: exact with one batch, estimated from the window counts otherwise
-  const std::vector<uint64_t> slots = region_slots(hc, n_batches);
+  PieceList pieces(c);
+  make_pieces(c, entries, n_var, n_batches, nullptr, pieces);
+  entries.release();
   Pt2Out out;
   double esum = 0.0, esq = 0.0;
   size_t n_sum = 0;
@@ -886,7 +1209,7 @@ Pt2Out pt_batched(shci_ctx* c, double e_var, PtParams Q, size_t n_batches, doubl
   for (size_t batch = 0; batch < n_batches; batch++) {
     Q.batch = batch;
     bu.n = bd.n = 0;
-    const size_t bn = pt_emit_reduce<MODE>(c, st, Q, S, n_var, slots, bu, bd, bv, 0);
+    const size_t bn = pt_emit_reduce<MODE>(c, st, Q, S, pieces, bu, bd, bv, 0);
     double bs, bsq;
     pt_batch_sums<MODE>(c, bu, bd, bv, bn, e_var, &bs, &bsq);
     n_sum += bn;
@@ -1011,14 +1334,15 @@ size_t pilot_pt_dets(shci_ctx* c, PtSetup& st, const std::vector<size_t>& src, d
   Q.iter_shift = shift;
   Q.pilot = 1;
   set_batches(Q, 128);
-  PtParams Q1 = Q;
-  set_batches(Q1, 1);
-  const std::vector<uint64_t> hc = region_slots(pt_counts<kSto>(c, st, Q1, S, n_src), 128);
+  DevBuf<uint64_t> entries;
+  pt_counts<kSto>(c, st, Q, S, n_src, entries);
+  PieceList pieces(c);
+  make_pieces(c, entries, n_src, 128, nullptr, pieces);
   DevBuf<uint64_t> bu, bd;
   DevBuf<double> bv[5];
   bu.mt = bd.mt = &c->mem;
   for (auto& b : bv) b.mt = &c->mem;
-  return pt_emit_reduce<kSto>(c, st, Q, S, n_src, hc, bu, bd, bv, shift + 5);
+  return pt_emit_reduce<kSto>(c, st, Q, S, pieces, bu, bd, bv, shift + 5);
 }
 
 size_t psto_auto_batches(shci_ctx* c, double eps_pt_psto, double pt_mem_avail, double mem_usage,
@@ -1347,24 +1671,22 @@ Pt2Out pt2_sto(shci_ctx* c, double energy_var, double eps_pt_psto, double eps_pt
     SHCI_CUDA(cudaMemcpyAsync(d_count.p, h_count.data(), n_ent * 8, cudaMemcpyHostToDevice, s));
     SHCI_CUDA(cudaMemcpyAsync(d_weight.p, h_weight.data(), n_ent * 8, cudaMemcpyHostToDevice, s));
     SHCI_CUDA(cudaMemcpyAsync(d_dtm.p, h_dtm.data(), n_ent, cudaMemcpyHostToDevice, s));
-    StoSources S{d_det.p, d_iter.p, d_count.p, d_weight.p, d_batch.p, d_dtm.p, nullptr, d_off.p};
+    StoSources S{d_det.p, d_iter.p, d_count.p, d_weight.p, d_batch.p, d_dtm.p, d_off.p};
     PtParams Q{};
     Q.eps = eps_pt;
     Q.eps_psto = eps_pt_psto;
     set_batches(Q, n_batches);
     Q.factor = factor;
     Q.iter_shift = shift;
-    PtParams Q1 = Q;
-    set_batches(Q1, 1);
-    std::vector<uint32_t> mult(n_src);
-    for (uint32_t g = 0; g < n_src; g++) mult[g] = h_off[g + 1] - h_off[g];
-    const std::vector<uint64_t> hc =
-        region_slots(pt_counts<kSto>(c, st, Q1, S, n_src), n_batches, &mult);
+    DevBuf<uint64_t> entries;
+    pt_counts<kSto>(c, st, Q, S, n_src, entries);
+    PieceList pieces(c);
+    make_pieces(c, entries, n_src, n_batches, d_off.p, pieces);
     DevBuf<uint64_t> bu, bd;
     DevBuf<double> bv[5];
     bu.mt = bd.mt = &c->mem;
     for (auto& b : bv) b.mt = &c->mem;
-    const size_t bn = pt_emit_reduce<kSto>(c, st, Q, S, n_src, hc, bu, bd, bv, shift + 5);
+    const size_t bn = pt_emit_reduce<kSto>(c, st, Q, S, pieces, bu, bd, bv, shift + 5);
     // per-iteration sums of the contributions
     std::vector<double> it_sum(n_it, 0.0);
     if (bn) {
