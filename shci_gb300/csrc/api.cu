@@ -624,7 +624,7 @@ shci_status shci_get_hamiltonian(shci_ctx* c, uint64_t* row_ptr, uint32_t* cols,
         v.release();
         std::vector<uint64_t> rp(n + 1);
         std::vector<uint32_t> rc(n);
-        const size_t cap = H.col.cap;
+        const size_t cap = H.col.n;  // (as allocated: the values have as many)
         std::vector<uint32_t> hc(cap);
         std::vector<double> hv;
         std::vector<float> h32, r32;

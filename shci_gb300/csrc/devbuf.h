@@ -121,7 +121,11 @@ struct DevBuf {
     size_t c = static_cast<size_t>(k * slack);
     if (c < k) c = k;
     if (c == 0) c = 1;
-    const size_t bytes = c * sizeof(T);
+    // whole units of 256 bytes, which every element size divides, so that a block handed on to
+    // another type keeps its size
+    static_assert(256 % sizeof(T) == 0, "element sizes divide 256");
+    const size_t bytes = (c * sizeof(T) + 255) & ~static_cast<size_t>(255);
+    c = bytes / sizeof(T);
     if (mt) {
       size_t got = 0;
       if (void* b = mt->take(bytes, &got)) {

@@ -97,10 +97,9 @@ void jacobi_eig(int k, const double* lower, int ld, double* evals, double* evecs
 size_t select_dets(shci_ctx* c, double eps_var, bool var_sd);
 void rebuild_det_set(shci_ctx* c, size_t n_have = 0, bool allow_dup = false);
 size_t sort_unique_pairs(shci_ctx* c, DevBuf<uint64_t>& a, DevBuf<uint64_t>& b, size_t m,
-                         DevBuf<double>* vals = nullptr, int n_vals = 1, int a_bits = 0);
-void compact_valid(shci_ctx* c, const uint64_t* a, const uint64_t* b, const double* const* v,
-                   int n_vals, size_t m, DevBuf<uint64_t>& oa, DevBuf<uint64_t>& ob,
-                   DevBuf<double>* ov, size_t* n_out);
+                         int a_bits = 0);
+void compact_valid(shci_ctx* c, const uint64_t* a, const uint64_t* b, size_t m,
+                   DevBuf<uint64_t>& oa, DevBuf<uint64_t>& ob, size_t* n_out);
 
 // pt2.cu
 struct Pt2Out {

@@ -6,8 +6,7 @@
 // sample) and emits the connected dets a in the heat-bath window [eps / |c_i|, INF) that fall
 // in the current hash batch (rehash(DetHasher(a)) % n_batches), are not variational and have
 // |H_ai c_i| >= eps.  The reference accumulates (a -> sum) in a distributed hash map; here
-// the (a, values) pairs are compacted, radix-sorted by det and reduced by key in a fixed
-// order, and a second kernel forms each unique a's contribution with its diagonal H_aa.
+// the (a, values) pairs are grouped by det (group.cu) and reduced in a fixed order, and a second kernel forms each unique a's contribution with its diagonal H_aa.
 //   dtm : value  = H_ai c_i                          contribution S0^2 / (E - H_aa)
 //   psto: values = [hc, hc if |hc| >= eps_dtm]      contribution (S0^2 - S1^2) / (E - H_aa)
 //   sto : values = the five sums of solver.h:1093-1103, contribution of :1117-1124
@@ -32,6 +31,7 @@
 #include <unordered_map>
 
 #include "ctx.h"
+#include "group.cuh"
 #include "heatbath.cuh"
 #include "kernels.h"
 
@@ -123,9 +123,10 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
   }
 }
 
-struct OutCols {
-  double* v[5];
-};
+template <int MODE>
+constexpr int n_cols() {
+  return MODE == kDtm ? 1 : MODE == kPsto ? 2 : 5;
+}
 
 // Single-excitation elements in 64-bit fixed point.  H_ij of a single excitation p -> q is
 // +-(h_pq + sum_o (pq|oo) [2 (pq|oo) for a doubly occupied o] - sum_o (po|oq)), about 2 n_e
@@ -271,7 +272,7 @@ __device__ __forceinline__ uint32_t bit_of(uint64_t x, uint32_t k) {
 template <int MODE>
 __global__ void __launch_bounds__(kPtWarps * 32, 4)
     k_pt_emit(SelParams P, PtParams Q, StoSources S, SingleFix F, PtPieces pc,
-              uint64_t* __restrict__ out_up, uint64_t* __restrict__ out_dn, OutCols out) {
+              PtRec<n_cols<MODE>()>* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char pt_smem[];
   PtWarp& W = reinterpret_cast<PtWarp*>(pt_smem)[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31;
@@ -339,14 +340,12 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
       uint64_t pos = pc.off[piece] + before + __popc(keep & mates & lt);
       if (pos < pc.off[piece + 1]) {
         pos -= pc.base;
-        out_up[pos] = cu | iter_tag;
-        out_dn[pos] = cd;
-        if (MODE == kDtm) {
-          out.v[0][pos] = hc;
-        } else if (MODE == kPsto) {
-          out.v[0][pos] = hc;
-          out.v[1][pos] = fabs(hc) >= Q.eps_dtm ? hc : 0.0;
-        } else {
+        PtRec<n_cols<MODE>()> r{};
+        r.u = cu | iter_tag;
+        r.d = cd;
+        r.v[0] = hc;
+        if constexpr (MODE == kPsto) r.v[1] = fabs(hc) >= Q.eps_dtm ? hc : 0.0;
+        if constexpr (MODE == kSto) {
           // solver.h:1093-1103
           const double x = count * hc / weight;
           const bool above = fabs(hc) > Q.eps_psto;
@@ -356,12 +355,13 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
             if (above) v3 = v2;
             else v4 = x * x * (1. - weight / count + Q.factor);
           }
-          out.v[0][pos] = x;
-          out.v[1][pos] = above ? x : 0.0;
-          out.v[2][pos] = v2;
-          out.v[3][pos] = v3;
-          out.v[4][pos] = v4;
+          r.v[0] = x;
+          r.v[1] = above ? x : 0.0;
+          r.v[2] = v2;
+          r.v[3] = v3;
+          r.v[4] = v4;
         }
+        out[pos] = r;
       }
     }
     if (MODE != kSto) {
@@ -597,20 +597,17 @@ __global__ void k_pt_kept(const uint32_t* __restrict__ cnt, const uint64_t* __re
 template <int NV>
 __global__ void __launch_bounds__(256)
     k_pt_collect(const uint64_t* __restrict__ off, uint64_t base, const uint64_t* __restrict__ dst,
-                 const uint64_t* __restrict__ total, uint32_t n, const uint64_t* __restrict__ u,
-                 const uint64_t* __restrict__ d, OutCols v, uint64_t* __restrict__ ou,
-                 uint64_t* __restrict__ od, OutCols ov) {
+                 const uint64_t* __restrict__ total, uint32_t n, const PtRec<NV>* __restrict__ rec,
+                 PtRec<NV>* __restrict__ out) {
+  constexpr uint64_t W = sizeof(PtRec<NV>) / sizeof(uint4);
+  const uint4* __restrict__ in = reinterpret_cast<const uint4*>(rec);
+  uint4* __restrict__ o = reinterpret_cast<uint4*>(out);
   const unsigned sub = threadIdx.x & 7;
   const uint32_t step = gridDim.x * (blockDim.x >> 3);
   for (uint32_t p = blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3); p < n; p += step) {
-    const uint64_t a = off[p] - base, b = dst[p];
-    const uint64_t m = (p + 1 < n ? dst[p + 1] : *total) - b;
-    for (uint64_t k = sub; k < m; k += 8) {
-      ou[b + k] = u[a + k];
-      od[b + k] = d[a + k];
-#pragma unroll
-      for (int c = 0; c < NV; c++) ov.v[c][b + k] = v.v[c][a + k];
-    }
+    const uint64_t a = (off[p] - base) * W, b = dst[p] * W;
+    const uint64_t m = (p + 1 < n ? dst[p + 1] : *total) * W - b;
+    for (uint64_t k = sub; k < m; k += 8) o[b + k] = in[a + k];
   }
 }
 
@@ -653,21 +650,21 @@ __device__ __forceinline__ double h_diag_fix(const DiagFix& F, uint64_t up, uint
 
 // x[k] = contribution of unique PT det k (mapper of solver.h:727-732, 856-862, 1117-1124)
 template <int MODE>
-__global__ void k_pt_x(DiagFix D, const uint64_t* au, const uint64_t* ad, OutCols S,
-                       size_t m, double e_var, double n_batches, uint64_t orb_mask, double* x) {
+__global__ void k_pt_x(DiagFix D, const PtRec<n_cols<MODE>()>* __restrict__ rec, size_t m,
+                       double e_var, double n_batches, uint64_t orb_mask, double* x) {
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < m;
        k += (size_t)gridDim.x * blockDim.x) {
-    const double haa = h_diag_fix(D, au[k] & orb_mask, ad[k]);
+    const PtRec<n_cols<MODE>()> r = rec[k];
+    const double haa = h_diag_fix(D, r.u & orb_mask, r.d);
     double v;
-    if (MODE == kDtm) {
-      v = S.v[0][k] * S.v[0][k] / (e_var - haa);
-    } else if (MODE == kPsto) {
-      const double d = S.v[0][k] * S.v[0][k] - S.v[1][k] * S.v[1][k];
+    if constexpr (MODE == kDtm) {
+      v = r.v[0] * r.v[0] / (e_var - haa);
+    } else if constexpr (MODE == kPsto) {
+      const double d = r.v[0] * r.v[0] - r.v[1] * r.v[1];
       v = d / (e_var - haa);
     } else {
       const double f = n_batches / (e_var - haa);
-      v = (S.v[0][k] * S.v[0][k] - S.v[1][k] * S.v[1][k] + S.v[2][k] * S.v[2][k] -
-           S.v[3][k] * S.v[3][k] - S.v[4][k]) * f;
+      v = (r.v[0] * r.v[0] - r.v[1] * r.v[1] + r.v[2] * r.v[2] - r.v[3] * r.v[3] - r.v[4]) * f;
     }
     x[k] = v;
   }
@@ -773,15 +770,15 @@ void seg_reduce2(shci_ctx* c, const double* x, const uint64_t* starts, uint32_t 
 
 namespace {
 
-// starts[it] = first k with (au[k] >> shift) >= it, for it = 0..n_it (au sorted ascending)
-__global__ void k_iter_starts(const uint64_t* au, size_t m, int shift, uint32_t n_it,
+// starts[it] = first k with (rec[k].u >> shift) >= it, for it = 0..n_it (tags ascending)
+__global__ void k_iter_starts(const PtRec<5>* rec, size_t m, int shift, uint32_t n_it,
                               uint64_t* starts) {
   const uint32_t it = blockIdx.x * blockDim.x + threadIdx.x;
   if (it > n_it) return;
   size_t lo = 0, hi = m;
   while (lo < hi) {
     const size_t mid = (lo + hi) >> 1;
-    if ((au[mid] >> shift) < it) lo = mid + 1;
+    if ((rec[mid].u >> shift) < it) lo = mid + 1;
     else hi = mid;
   }
   starts[it] = lo;
@@ -911,11 +908,6 @@ void pt_setup(shci_ctx* c, PtSetup& st) {
   st.grid = static_cast<unsigned>(sms) * 8u;
 }
 
-template <int MODE>
-constexpr int n_cols() {
-  return MODE == kDtm ? 1 : MODE == kPsto ? 2 : 5;
-}
-
 // Pieces of a set of sources (on the device); piece p's region is [off[p], off[p + 1]).
 struct PieceList {
   DevBuf<uint32_t> src, begin, len;
@@ -965,23 +957,23 @@ void make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src, u
   SHCI_CUDA(cudaStreamSynchronize(s));
 }
 
-// Emits the members of the pieces for one batch (or set of iterations), appending them to (bu, bd,
-// bv) after the first *bn.  Pieces whose region overflowed are appended to *over with their
+// Emits the members of the pieces for one batch (or set of iterations), appending them to rec
+// after the first *bn.  Pieces whose region overflowed are appended to *over with their
 // exact sizes.  The accumulation is sorted and reduced in place whenever it grows past kCap, to
 // keep it bounded.
 template <int MODE>
 void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSources& S,
-                    const PieceList& L, DevBuf<uint64_t>& bu, DevBuf<uint64_t>& bd,
-                    DevBuf<double>* bv, size_t* bn, int a_bits, PieceRerun* over) {
+                    const PieceList& L, DevBuf<PtRec<n_cols<MODE>()>>& rec, size_t* bn,
+                    int tag_bits, PieceRerun* over) {
   constexpr int NV = n_cols<MODE>();
   cudaStream_t s = c->stream;
   const uint64_t kCap = 1ull << 27;
-  DevBuf<uint64_t> cu, cd, d_dst;
+  DevBuf<PtRec<NV>> out;
+  DevBuf<uint64_t> d_dst;
   DevBuf<uint32_t> d_cnt;
-  DevBuf<double> cv[NV];
-  cu.mt = cd.mt = d_dst.mt = &c->mem;
+  out.mt = &c->mem;
+  d_dst.mt = &c->mem;
   d_cnt.mt = &c->mem;
-  for (int v = 0; v < NV; v++) cv[v].mt = &c->mem;
   const SingleFix F = single_fix(c);
   const size_t smem = sizeof(PtWarp) * kPtWarps;
   SHCI_CUDA(cudaFuncSetAttribute(k_pt_emit<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1014,18 +1006,12 @@ void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSource
     d_cnt.resize((size_t)n + 1);  // (the overflow count after the pieces')
     d_dst.resize((size_t)n + 1);
     SHCI_CUDA(cudaMemsetAsync(d_cnt.p, 0, ((size_t)n + 1) * 4, s));
-    cu.resize(std::max<uint64_t>(tot, 1), 1.25);
-    cd.resize(std::max<uint64_t>(tot, 1), 1.25);
-    OutCols oc{};
-    for (int v = 0; v < NV; v++) {
-      cv[v].resize(std::max<uint64_t>(tot, 1), 1.25);
-      oc.v[v] = cv[v].p;
-    }
+    out.resize(std::max<uint64_t>(tot, 1), 1.25);
     const PtPieces pc{L.src.p + k0, L.begin.p + k0, L.len.p + k0, L.off.p + k0, d_cnt.p, n, base};
     {
       ProfScope ps(c->prof, s, "pt2_emit");
       k_pt_emit<MODE><<<grid_for((size_t)n * 32, kPtWarps * 32, st.grid), kPtWarps * 32, smem, s>>>(
-          st.P, Q, S, F, pc, cu.p, cd.p, oc);
+          st.P, Q, S, F, pc, out.p);
       SHCI_LAUNCH_CHECK();
     }
     uint64_t got = 0;
@@ -1039,17 +1025,10 @@ void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSource
       SHCI_CUDA(cudaMemcpyAsync(&n_over, d_cnt.p + n, 4, cudaMemcpyDeviceToHost, s));
       SHCI_CUDA(cudaStreamSynchronize(s));
       if (got) {
-        bu.n = bd.n = *bn;
-        bu.grow_keep(*bn + got, s);
-        bd.grow_keep(*bn + got, s);
-        OutCols ov{};
-        for (int v = 0; v < NV; v++) {
-          bv[v].n = *bn;
-          bv[v].grow_keep(*bn + got, s);
-          ov.v[v] = bv[v].p + *bn;
-        }
+        rec.n = *bn;
+        rec.grow_keep(*bn + got, s);
         k_pt_collect<NV><<<grid_for((size_t)n * 8, 256), 256, 0, s>>>(
-            pc.off, base, d_dst.p, d_dst.p + n, n, cu.p, cd.p, oc, bu.p + *bn, bd.p + *bn, ov);
+            pc.off, base, d_dst.p, d_dst.p + n, n, out.p, rec.p + *bn);
         SHCI_LAUNCH_CHECK();
         *bn += got;
       }
@@ -1072,27 +1051,24 @@ void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSource
           over->off.push_back(over->off.back() + cnt[k]);
         }
     }
-    if (*bn > kCap) {  // keep the accumulation buffer bounded
-      *bn = sort_unique_pairs(c, bu, bd, *bn, bv, NV, a_bits);
-      bu.n = bd.n = *bn;
-    }
+    if (*bn > kCap)  // keep the accumulation buffer bounded
+      *bn = group_records<NV>(c, rec, *bn, st.P.n_orbs, tag_bits);
     k0 = k1;
     base = end;
   }
 }
 
 // Emits and reduces the members of the pieces for one batch / set of iterations; returns the
-// unique count, keys in (bu, bd) and value columns in bv[0..n_cols).  Pieces whose estimated
+// number of distinct dets, which rec then holds.  Pieces whose estimated
 // region overflowed are emitted again, after the others, with the sizes they turned out to have.
 template <int MODE>
 size_t pt_emit_reduce(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSources& S,
-                      const PieceList& L, DevBuf<uint64_t>& bu, DevBuf<uint64_t>& bd,
-                      DevBuf<double>* bv, int a_bits) {
+                      const PieceList& L, DevBuf<PtRec<n_cols<MODE>()>>& rec, int tag_bits) {
   constexpr int NV = n_cols<MODE>();
   cudaStream_t s = c->stream;
   size_t bn = 0;
   PieceRerun over;
-  pt_emit_append<MODE>(c, st, Q, S, L, bu, bd, bv, &bn, a_bits, &over);
+  pt_emit_append<MODE>(c, st, Q, S, L, rec, &bn, tag_bits, &over);
   if (!over.src.empty()) {
     PieceList again(c);
     const size_t n = again.n = over.src.size();
@@ -1107,14 +1083,13 @@ size_t pt_emit_reduce(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSour
     SHCI_CUDA(cudaMemcpyAsync(again.off.p, over.off.data(), (n + 1) * 8, cudaMemcpyHostToDevice, s));
     SHCI_CUDA(cudaStreamSynchronize(s));
     PieceRerun over2;
-    pt_emit_append<MODE>(c, st, Q, S, again, bu, bd, bv, &bn, a_bits, &over2);
+    pt_emit_append<MODE>(c, st, Q, S, again, rec, &bn, tag_bits, &over2);
     if (!over2.src.empty()) throw std::logic_error("PT2 emission: exact regions overflowed");
   }
   {
     ProfScope ps(c->prof, s, "pt2_reduce");
-    bn = sort_unique_pairs(c, bu, bd, bn, bv, NV, a_bits);
+    bn = group_records<NV>(c, rec, bn, st.P.n_orbs, tag_bits);
   }
-  bu.n = bd.n = bn;
   return bn;
 }
 
@@ -1135,8 +1110,8 @@ void pt_counts(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSources& S,
 
 // Sum and sum of squares of the contributions of one reduced batch (dtm / psto).
 template <int MODE>
-void pt_batch_sums(shci_ctx* c, DevBuf<uint64_t>& bu, DevBuf<uint64_t>& bd, DevBuf<double>* bv,
-                   size_t bn, double e_var, double* sum, double* sumsq) {
+void pt_batch_sums(shci_ctx* c, const DevBuf<PtRec<n_cols<MODE>()>>& rec, size_t bn, double e_var,
+                   double* sum, double* sumsq) {
   *sum = *sumsq = 0.0;
   if (!bn) return;
   cudaStream_t s = c->stream;
@@ -1146,12 +1121,10 @@ void pt_batch_sums(shci_ctx* c, DevBuf<uint64_t>& bu, DevBuf<uint64_t>& bd, DevB
   x.resize(bn);
   out.resize(2);
   starts.resize(2);
-  OutCols oc{};
-  for (int v = 0; v < n_cols<MODE>(); v++) oc.v[v] = bv[v].p;
   {
     ProfScope ps(c->prof, s, "pt2_contrib");
-    k_pt_x<MODE><<<grid_for(bn, 256), 256, 0, s>>>(diag_fix(c), bu.p, bd.p, oc, bn, e_var, 1.0,
-                                                   ~0ull, x.p);
+    k_pt_x<MODE><<<grid_for(bn, 256), 256, 0, s>>>(diag_fix(c), rec.p, bn, e_var, 1.0, ~0ull,
+                                                   x.p);
     SHCI_LAUNCH_CHECK();
     const uint64_t st2[2] = {0, bn};
     SHCI_CUDA(cudaMemcpyAsync(starts.p, st2, 16, cudaMemcpyHostToDevice, s));
@@ -1203,15 +1176,13 @@ Pt2Out pt_batched(shci_ctx* c, double e_var, PtParams Q, size_t n_batches, doubl
   Pt2Out out;
   double esum = 0.0, esq = 0.0;
   size_t n_sum = 0;
-  DevBuf<uint64_t> bu, bd;
-  DevBuf<double> bv[2];
-  bu.mt = bd.mt = bv[0].mt = bv[1].mt = &c->mem;
+  DevBuf<PtRec<n_cols<MODE>()>> rec;
+  rec.mt = &c->mem;
   for (size_t batch = 0; batch < n_batches; batch++) {
     Q.batch = batch;
-    bu.n = bd.n = 0;
-    const size_t bn = pt_emit_reduce<MODE>(c, st, Q, S, pieces, bu, bd, bv, 0);
+    const size_t bn = pt_emit_reduce<MODE>(c, st, Q, S, pieces, rec, 0);
     double bs, bsq;
-    pt_batch_sums<MODE>(c, bu, bd, bv, bn, e_var, &bs, &bsq);
+    pt_batch_sums<MODE>(c, rec, bn, e_var, &bs, &bsq);
     n_sum += bn;
     esum += bs;
     esq += bsq;
@@ -1338,11 +1309,9 @@ size_t pilot_pt_dets(shci_ctx* c, PtSetup& st, const std::vector<size_t>& src, d
   pt_counts<kSto>(c, st, Q, S, n_src, entries);
   PieceList pieces(c);
   make_pieces(c, entries, n_src, 128, nullptr, pieces);
-  DevBuf<uint64_t> bu, bd;
-  DevBuf<double> bv[5];
-  bu.mt = bd.mt = &c->mem;
-  for (auto& b : bv) b.mt = &c->mem;
-  return pt_emit_reduce<kSto>(c, st, Q, S, pieces, bu, bd, bv, shift + 5);
+  DevBuf<PtRec<5>> rec;
+  rec.mt = &c->mem;
+  return pt_emit_reduce<kSto>(c, st, Q, S, pieces, rec, 5);
 }
 
 size_t psto_auto_batches(shci_ctx* c, double eps_pt_psto, double pt_mem_avail, double mem_usage,
@@ -1682,11 +1651,9 @@ Pt2Out pt2_sto(shci_ctx* c, double energy_var, double eps_pt_psto, double eps_pt
     pt_counts<kSto>(c, st, Q, S, n_src, entries);
     PieceList pieces(c);
     make_pieces(c, entries, n_src, n_batches, d_off.p, pieces);
-    DevBuf<uint64_t> bu, bd;
-    DevBuf<double> bv[5];
-    bu.mt = bd.mt = &c->mem;
-    for (auto& b : bv) b.mt = &c->mem;
-    const size_t bn = pt_emit_reduce<kSto>(c, st, Q, S, pieces, bu, bd, bv, shift + 5);
+    DevBuf<PtRec<5>> rec;
+    rec.mt = &c->mem;
+    const size_t bn = pt_emit_reduce<kSto>(c, st, Q, S, pieces, rec, 5);
     // per-iteration sums of the contributions
     std::vector<double> it_sum(n_it, 0.0);
     if (bn) {
@@ -1696,16 +1663,13 @@ Pt2Out pt2_sto(shci_ctx* c, double energy_var, double eps_pt_psto, double eps_pt
       x.resize(bn);
       o.resize(2 * n_it);
       starts.resize(n_it + 1);
-      OutCols oc{};
-      for (int v = 0; v < 5; v++) oc.v[v] = bv[v].p;
       const uint64_t mask = shift == 64 ? ~0ull : ((1ull << shift) - 1ull);
       {
         ProfScope ps(c->prof, s, "pt2_contrib");
-        k_pt_x<kSto><<<grid_for(bn, 256), 256, 0, s>>>(diag_fix(c), bu.p, bd.p, oc, bn,
-                                                       energy_var, static_cast<double>(n_batches),
-                                                       mask, x.p);
+        k_pt_x<kSto><<<grid_for(bn, 256), 256, 0, s>>>(diag_fix(c), rec.p, bn, energy_var,
+                                                       static_cast<double>(n_batches), mask, x.p);
         SHCI_LAUNCH_CHECK();
-        k_iter_starts<<<1, 128, 0, s>>>(bu.p, bn, shift, n_it, starts.p);
+        k_iter_starts<<<1, 128, 0, s>>>(rec.p, bn, shift, n_it, starts.p);
         SHCI_LAUNCH_CHECK();
         seg_reduce2(c, x.p, starts.p, n_it, bn, o.p);
       }

@@ -244,36 +244,11 @@ __global__ void k_max_coef(const double* c0, StatePtrs xs, int n_extra, size_t n
 
 }  // namespace
 
-namespace {
-
-// out[g] = sum of vals[perm[k]] over segment g = [starts[g], starts[g+1]), in input order
-// (one thread per segment: a fixed summation order, independent of scheduling).
-__global__ void k_segsum(const uint32_t* starts, size_t nseg, size_t m, const uint32_t* perm,
-                         const double* vals, double* out) {
-  for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < nseg;
-       g += (size_t)gridDim.x * blockDim.x) {
-    const size_t e = g + 1 < nseg ? starts[g + 1] : m;
-    double acc = 0.0;
-    for (size_t k = starts[g]; k < e; k++) acc += vals[perm[k]];
-    out[g] = acc;
-  }
-}
-
-__global__ void k_seg_starts(const uint32_t* flags, const uint32_t* pos, size_t m,
-                             uint32_t* starts) {
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < m;
-       k += (size_t)gridDim.x * blockDim.x)
-    if (flags[k]) starts[pos[k]] = static_cast<uint32_t>(k);
-}
-
-}  // namespace
-
 // Sorts (up, dn) pairs held in a / b (length m) into ascending (a, b) order and removes
-// duplicates; returns the unique count (left in a / b).  With vals (n_vals columns), the
-// values of equal keys are summed (reduce by key) and left in the columns.  a_bits = bits
-// of the a key (0: n_orbs); b keys always have n_orbs bits.
+// duplicates; returns the unique count (left in a / b).  a_bits = bits of the a key (0: n_orbs);
+// b keys always have n_orbs bits.
 size_t sort_unique_pairs(shci_ctx* c, DevBuf<uint64_t>& a, DevBuf<uint64_t>& b, size_t m,
-                         DevBuf<double>* vals, int n_vals, int a_bits) {
+                         int a_bits) {
   if (m == 0) return 0;
   cudaStream_t s = c->stream;
   const int nb = c->I.n;
@@ -296,43 +271,16 @@ size_t sort_unique_pairs(shci_ctx* c, DevBuf<uint64_t>& a, DevBuf<uint64_t>& b, 
   k_unique_flags<<<grid_for(m, 256), 256, 0, s>>>(key.p, sd.p, m, c->u1.p);
   SHCI_LAUNCH_CHECK();
   const uint32_t nu = exclusive_scan_u32(c->u1.p, c->u2.p, m, s, c->sort);
-  if (vals && n_vals > 0) {
-    DevBuf<uint32_t> starts;
-    starts.mt = &c->mem;
-    starts.resize(nu ? nu : 1);
-    k_seg_starts<<<grid_for(m, 256), 256, 0, s>>>(c->u1.p, c->u2.p, m, starts.p);
-    SHCI_LAUNCH_CHECK();
-    DevBuf<double> sums;
-    sums.mt = &c->mem;
-    sums.resize(nu ? nu : 1);
-    for (int v = 0; v < n_vals; v++) {
-      k_segsum<<<grid_for(nu, 256), 256, 0, s>>>(starts.p, nu, m, c->u0.p, vals[v].p, sums.p);
-      SHCI_LAUNCH_CHECK();
-      SHCI_CUDA(cudaMemcpyAsync(vals[v].p, sums.p, nu * 8, cudaMemcpyDeviceToDevice, s));
-    }
-    SHCI_CUDA(cudaStreamSynchronize(s));
-    c->launches += 1 + n_vals;
-  }
   k_compact2<<<grid_for(m, 256), 256, 0, s>>>(key.p, sd.p, c->u1.p, c->u2.p, m, a.p, b.p);
   SHCI_LAUNCH_CHECK();
   c->launches += 8;
   return nu;
 }
 
-namespace {
-__global__ void k_compact_vals(const double* v, const uint32_t* flags, const uint32_t* pos,
-                               size_t n, double* ov) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    if (flags[i]) ov[pos[i]] = v[i];
-}
-}  // namespace
-
-// Appends the entries of (a, b[, v columns]) whose a != kInvalid to (oa, ob[, ov columns])
-// after *n_out (growing them); *n_out is advanced by the number appended.
-void compact_valid(shci_ctx* c, const uint64_t* a, const uint64_t* b, const double* const* v,
-                   int n_vals, size_t m, DevBuf<uint64_t>& oa, DevBuf<uint64_t>& ob,
-                   DevBuf<double>* ov, size_t* n_out) {
+// Appends the entries of (a, b) whose a != kInvalid to (oa, ob) after *n_out (growing them);
+// *n_out is advanced by the number appended.
+void compact_valid(shci_ctx* c, const uint64_t* a, const uint64_t* b, size_t m,
+                   DevBuf<uint64_t>& oa, DevBuf<uint64_t>& ob, size_t* n_out) {
   if (m == 0) return;
   cudaStream_t s = c->stream;
   c->u1.reserve(m, 1.25);
@@ -348,12 +296,6 @@ void compact_valid(shci_ctx* c, const uint64_t* a, const uint64_t* b, const doub
   ob.grow_keep(at + nv, s);
   k_compact2<<<grid_for(m, 256), 256, 0, s>>>(a, b, c->u1.p, c->u2.p, m, oa.p + at, ob.p + at);
   SHCI_LAUNCH_CHECK();
-  for (int k = 0; k < n_vals && ov; k++) {
-    ov[k].n = at;
-    ov[k].grow_keep(at + nv, s);
-    k_compact_vals<<<grid_for(m, 256), 256, 0, s>>>(v[k], c->u1.p, c->u2.p, m, ov[k].p + at);
-    SHCI_LAUNCH_CHECK();
-  }
   *n_out = at + nv;
 }
 
@@ -548,7 +490,7 @@ size_t select_dets(shci_ctx* c, double eps_var, bool var_sd) {
           }
           // compact valid candidates, then sort + unique
           const size_t before = pass_n;
-          compact_valid(c, cu.p, cd.p, nullptr, 0, tot, pass_up, pass_dn, nullptr, &pass_n);
+          compact_valid(c, cu.p, cd.p, tot, pass_up, pass_dn, &pass_n);
           if (pass_n > before) {
             pass_n = sort_unique_pairs(c, pass_up, pass_dn, pass_n);
             pass_up.n = pass_dn.n = pass_n;

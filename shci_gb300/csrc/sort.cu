@@ -258,19 +258,22 @@ __global__ void k_key_spread(const K* keys, size_t n, unsigned long long* spread
 
 template <class K, class V>
 void radix_sort_impl(DevBuf<K>& keys, DevBuf<V>& vals, size_t n, int begin_bit, int end_bit,
-                     cudaStream_t s, SortScratch& sc, DevBuf<K>& kalt, DevBuf<V>& valt) {
+                     cudaStream_t s, SortScratch& sc, DevBuf<K>& kalt, DevBuf<V>& valt,
+                     bool skip = true) {
   if (n <= 1 || begin_bit >= end_bit) return;
   if (n >= 0xffffffffull) throw ArgError("radix sort: 2^32 or more items");
   end_bit = end_bit > (int)(8 * sizeof(K)) ? (int)(8 * sizeof(K)) : end_bit;
   // Which digits vary at all?
-  sc.part64.reserve(scan_part_size(1));
-  unsigned long long* spread = reinterpret_cast<unsigned long long*>(sc.part64.p);
-  SHCI_CUDA(cudaMemsetAsync(spread, 0, sizeof(unsigned long long), s));
-  k_key_spread<K><<<grid_for(n, 256, 152 * 8), 256, 0, s>>>(keys.p, n, spread);
-  SHCI_LAUNCH_CHECK();
-  unsigned long long sp = 0;
-  SHCI_CUDA(cudaMemcpyAsync(&sp, spread, sizeof(sp), cudaMemcpyDeviceToHost, s));
-  SHCI_CUDA(cudaStreamSynchronize(s));
+  unsigned long long sp = ~0ull;
+  if (skip) {
+    sc.part64.reserve(scan_part_size(1));
+    unsigned long long* spread = reinterpret_cast<unsigned long long*>(sc.part64.p);
+    SHCI_CUDA(cudaMemsetAsync(spread, 0, sizeof(unsigned long long), s));
+    k_key_spread<K><<<grid_for(n, 256, 152 * 8), 256, 0, s>>>(keys.p, n, spread);
+    SHCI_LAUNCH_CHECK();
+    SHCI_CUDA(cudaMemcpyAsync(&sp, spread, sizeof(sp), cudaMemcpyDeviceToHost, s));
+    SHCI_CUDA(cudaStreamSynchronize(s));
+  }
 
   const unsigned n_tiles = static_cast<unsigned>((n + kSortTile - 1) / kSortTile);
   const size_t n_hist = (size_t)256 * n_tiles;
@@ -373,9 +376,9 @@ void radix_sort_pairs64(DevBuf<uint64_t>& keys, DevBuf<uint64_t>& vals, size_t n
 }
 
 void radix_sort_pairs32(DevBuf<uint32_t>& keys, DevBuf<uint32_t>& vals, size_t n,
-                        int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc) {
+                        int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc, bool skip) {
   radix_sort_impl<uint32_t, uint32_t>(keys, vals, n, begin_bit, end_bit, s, sc, sc.kalt32,
-                                      sc.valt32);
+                                      sc.valt32, skip);
 }
 
 void iota_u32(uint32_t* v, size_t n, cudaStream_t s) {

@@ -43,8 +43,10 @@ void radix_sort_pairs(DevBuf<uint64_t>& keys, DevBuf<uint32_t>& vals, size_t n, 
                       int end_bit, cudaStream_t s, SortScratch& sc);
 void radix_sort_pairs64(DevBuf<uint64_t>& keys, DevBuf<uint64_t>& vals, size_t n,
                         int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc);
+// skip = false: every digit is sorted without looking first which ones vary (hash keys).
 void radix_sort_pairs32(DevBuf<uint32_t>& keys, DevBuf<uint32_t>& vals, size_t n,
-                        int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc);
+                        int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc,
+                        bool skip = true);
 
 template <class T>
 inline void swap_storage(DevBuf<T>& a, DevBuf<T>& b) {

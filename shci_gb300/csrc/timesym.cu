@@ -172,10 +172,10 @@ size_t build_time_sym(shci_ctx* c, int precision) {
     rz.mt = &c->mem;
     rz.resize(len);
     SHCI_CUDA(cudaMemsetAsync(rz.p, 0, len * 8, s));
-    compact_valid(c, raw.p, rz.p, nullptr, 0, len, keys, zero, nullptr, &K);
+    compact_valid(c, raw.p, rz.p, len, keys, zero, &K);
     raw.release();
     rz.release();
-    K = sort_unique_pairs(c, keys, zero, K, nullptr, 1, 64);
+    K = sort_unique_pairs(c, keys, zero, K, 64);
     c->launches += 1;
   } catch (...) {
     c->time_sym = true;
