@@ -676,7 +676,9 @@ __global__ void k_pt_x(DiagFix D, const PtRec<n_cols<MODE>()>* __restrict__ rec,
 // partials.  Every partial is a compensated double-double sum (Dd), so the result does not
 // lose accuracy with the number of PT dets (1e8 and more); only the chunking fixes the order,
 // so results are reproducible.
-constexpr uint32_t kRedChunk = 1u << 16;
+// A chunk is 32 elements a thread: chunks of 65,536 elements left two thirds of the chip idle below
+// 10M determinants (0.89 -> 0.57 ms for 12.6M, 0.46 -> 0.11 ms for 1.9M).
+constexpr uint32_t kRedChunk = 1u << 13;
 
 __device__ __forceinline__ void block_sum2(Dd* a, Dd* b) {
   __shared__ Dd s1[8], s2[8];
@@ -708,17 +710,21 @@ __global__ void __launch_bounds__(256)
   const uint64_t b0 = starts[g] + (uint64_t)ch * kRedChunk;
   const uint64_t e = starts[g + 1];
   const uint64_t b1 = b0 + kRedChunk < e ? b0 + kRedChunk : e;
+  // a thread's sums with the rounding errors of their additions kept apart (added up in FP64 and
+  // joined at the end: 16 FP64 operations an element instead of 24)
   Dd a, b;
   for (uint64_t k = b0 + threadIdx.x; k < b1; k += blockDim.x) {
     const double v = x[k];
-    a = dd_add(a, v);
-    // v^2 as an exact product pair: hi = v*v rounded, lo = its FMA error
+    double e;
+    two_sum64(a.hi, v, &a.hi, &e);
+    a.lo += e;
+    // v^2 as an exact product pair: sq rounded, its FMA error
     const double sq = v * v;
-    Dd t;
-    t.hi = sq;
-    t.lo = fma(v, v, -sq);
-    b = dd_add(b, t);
+    two_sum64(b.hi, sq, &b.hi, &e);
+    b.lo += e + fma(v, v, -sq);
   }
+  a = dd_add(a, 0.0);
+  b = dd_add(b, 0.0);
   block_sum2(&a, &b);
   if (threadIdx.x == 0) {
     double* o = part + 4 * ((size_t)g * n_chunks + ch);
