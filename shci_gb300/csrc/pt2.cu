@@ -191,12 +191,18 @@ struct PtPieces {
 constexpr uint32_t kPieceLen = 4096;
 constexpr uint32_t kPtQ = 64;    // queue lengths (< 32 waiting + 32 pushed)
 constexpr uint32_t kPtSlots = 256;  // slots listed at a time
+// Ranges of at least this many entries are walked slot by slot, the others flattened over the lanes:
+// a round of 32 costs about 40 instructions with one slot's strings in registers and about 100
+// when every lane finds its slot (n = 40: 6.4 -> 5.4 ms a pseudo-stochastic batch, 13.4 -> 11.9 ms
+// for six stochastic iterations; a limit of 24 measures the same).
+constexpr uint32_t kPtLong = 12;
 
 struct PtWarp {
-  // slots of the current source with a non-empty range: first entry, entries, code
+  // slots of the current source with a non-empty range: first entry, entries, code; long ranges
+  // from the front, short ones from the back
   uint32_t s_lo[kPtSlots], s_cnt[kPtSlots], s_code[kPtSlots];
-  // stage 1 queue: entries whose targets are free
-  uint32_t a_rs[kPtQ], a_code[kPtQ], a_piece[kPtQ];
+  // stage 1 queue: entries whose targets are free (x: slot code with the targets, y: piece)
+  uint2 a[kPtQ];
   // stage 2 queue (several batches): members
   uint64_t b_u[kPtQ], b_d[kPtQ];
   uint32_t b_piece[kPtQ];
@@ -204,11 +210,12 @@ struct PtWarp {
   uint8_t occ[128];  // electron -> spatial orbital, alpha electrons first
 };
 
-// Slot code: the strings that the targets r and s of an entry must be free in, and the orbitals
-// that the electrons leave.  A queue entry's r | s << 16 holds the targets of the stored pair; a
-// beta-beta pair is stored as its alpha image and an alpha-beta pair p > q as (q, p) (chem_system.cc:
-// 347-361), so the strings follow from the slot alone.
-enum : uint32_t { kADn = 1u << 16, kBDn = 1u << 17, kOne = 1u << 18 };
+// Slot code: the orbitals p and q that the electrons leave, and the strings that the targets r and s
+// of an entry must be free in; a queued entry adds its targets.  A queue entry's r | s << 16 holds
+// the targets of the stored pair; a beta-beta pair is stored as its alpha image and an alpha-beta
+// pair p > q as (q, p) (chem_system.cc:347-361), so the strings follow from the slot alone.
+constexpr int kPBit = 0, kQBit = 6, kRBit = 12, kSBit = 18;
+enum : uint32_t { kADn = 1u << 24, kBDn = 1u << 25, kOne = 1u << 26 };
 
 // Entry range and code of slot `slot`; as slot_range (heatbath.cuh), the orbitals from `occ`.
 __device__ __forceinline__ uint32_t pt_slot(const SelParams& P, const uint8_t* occ, int slot,
@@ -223,7 +230,7 @@ __device__ __forceinline__ uint32_t pt_slot(const SelParams& P, const uint8_t* o
     const uint32_t a = P.s_off[p], b = P.s_off[p + 1];
     *lo = a;
     *cnt = first_below(P.s_S, a, b, eps_min) - a;
-    return p | kOne | (slot < P.n_up ? 0u : kADn);
+    return p << kPBit | kOne | (slot < P.n_up ? 0u : kADn);
   }
   if (P.no_doubles || eps_min > P.max_hci) return 0;
   const uint32_t pr = P.pair_tab[slot - P.n_elecs];
@@ -234,13 +241,13 @@ __device__ __forceinline__ uint32_t pt_slot(const SelParams& P, const uint8_t* o
   size_t pq;
   if (dn1 == dn2) {
     pq = c2(p, q);
-    code = p | (q << 8) | (dn1 ? kADn | kBDn : 0u);
+    code = p << kPBit | q << kQBit | (dn1 ? kADn | kBDn : 0u);
   } else if (p > q) {  // stored as (q, p + n): r goes to beta, s to alpha
     pq = c2(q, p + n);
-    code = p | (q << 8) | kADn;
+    code = p << kPBit | q << kQBit | kADn;
   } else {
     pq = c2(p, q + n);
-    code = p | (q << 8) | kBDn;
+    code = p << kPBit | q << kQBit | kBDn;
   }
   const uint32_t a = static_cast<uint32_t>(P.d_off[pq]), b = static_cast<uint32_t>(P.d_off[pq + 1]);
   const uint32_t s = first_below(P.d_H, a, b, eps_max);
@@ -264,8 +271,8 @@ __device__ __forceinline__ uint32_t bit_of(uint64_t x, uint32_t k) {
 // against the source's strings and queues what passes; stage 2 builds 32 of those determinants and,
 // with several batches, hashes them and queues the members; the last stage evaluates 32 members.
 // Queues carry over from piece to piece.  Members keep their walk order within a piece.
-// At n = 40, 40,000 dets: 19.4 -> 4.6 ms deterministic (297M window entries), 11.3 -> 6.5 ms a
-// pseudo-stochastic batch of 16 (its hash is the work left: 56 % of issue), 21.4 -> 13.4 ms for six
+// At n = 40, 40,000 dets: 19.4 -> 4.6 ms deterministic (297M window entries), 11.3 -> 5.4 ms a
+// pseudo-stochastic batch of 16 (its hash is most of the work left), 21.4 -> 11.9 ms for six
 // stochastic iterations; n = 26, 30,000 dets: 5.3 -> 1.4 ms, of which the heaviest determinant's
 // window on one warp had been half.  (Before: build and hash at the walk, an output slot for
 // every window entry, a warp per source.)
@@ -279,7 +286,7 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
   const unsigned lt = (1u << lane) - 1u;
   const uint32_t wpg = gridDim.x * kPtWarps;
   const int n = P.n_orbs;
-  const uint32_t n_mask_off = static_cast<uint32_t>(n);
+  const uint32_t n_off = static_cast<uint32_t>(n);  // an alpha-beta pair's s is stored as s + n
   uint32_t ah = 0, an = 0, bh = 0, bn = 0;           // warp-uniform ring states
   uint32_t run_piece = 0xffffffffu, run_cnt = 0;      // kept members of the last piece seen
 
@@ -390,8 +397,8 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
     __syncwarp();
     const uint32_t sl = (ah + lane) & (kPtQ - 1);
     const bool act = lane < m;
-    const uint32_t piece = act ? W.a_piece[sl] : 0xffffffffu;
-    const uint32_t code = act ? W.a_code[sl] : 0u, rs = act ? W.a_rs[sl] : 0u;
+    const uint2 entry = W.a[sl];
+    const uint32_t piece = act ? entry.y : 0xffffffffu, code = entry.x;
     __syncwarp();
     ah += m;
     an -= m;
@@ -402,8 +409,8 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
       const uint32_t i = src_det(S, kk, MODE);
       cu = P.up[i];
       cd = P.dn[i];
-      const uint64_t out1 = 1ull << (code & 0xffu), out2 = 1ull << (code >> 8 & 0xffu);
-      const uint64_t in1 = 1ull << (rs & 0xffffu), in2 = 1ull << (rs >> 16);
+      const uint64_t out1 = 1ull << (code >> kPBit & 63u), out2 = 1ull << (code >> kQBit & 63u);
+      const uint64_t in1 = 1ull << (code >> kRBit & 63u), in2 = 1ull << (code >> kSBit & 63u);
       // (targets are in the strings A and B; the electrons that leave: of the first electron's
       // string and the second's, which for a swapped pair are B and A)
       const bool a_dn = code & kADn, b_dn = code & kBDn;
@@ -449,6 +456,15 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
     }
   };
 
+  // Queues the lanes' entries that passed.
+  auto push_a = [&](bool pass, uint32_t x, uint32_t piece) {
+    const unsigned bal = __ballot_sync(kFull, pass);
+    if (!bal) return;
+    if (pass) W.a[(ah + an + __popc(bal & lt)) & (kPtQ - 1)] = make_uint2(x, piece);
+    an += __popc(bal);
+    if (an >= 32u) drain_a(32u);
+  };
+
   for (uint32_t piece = blockIdx.x * kPtWarps + (threadIdx.x >> 5); piece < pc.n; piece += wpg) {
     const uint32_t kk = pc.src[piece];
     uint32_t skip = pc.begin[piece], left = pc.len[piece];
@@ -466,26 +482,56 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
     __syncwarp();
     const int n_slots = P.n_elecs + P.n_pairs;
     for (int f0 = 0; f0 < n_slots && left; f0 += kPtSlots) {
-      // the non-empty slots of this stretch
-      uint32_t m = 0;
+      // the non-empty slots of this stretch (a piece's entries: the long ranges in slot order, then
+      // the short ones)
+      uint32_t n_long = 0, n_short = 0;
       const int f1 = min(n_slots, f0 + (int)kPtSlots);
       for (int s0 = f0; s0 < f1; s0 += 32) {
         uint32_t lo = 0, c = 0, code = 0;
         if (s0 + (int)lane < f1)
           code = pt_slot(P, W.occ, s0 + lane, eps_min, eps_max, &lo, &c);
-        const unsigned bal = __ballot_sync(kFull, c != 0);
+        const unsigned bl = __ballot_sync(kFull, c >= kPtLong);
+        const unsigned bs = __ballot_sync(kFull, c && c < kPtLong);
         if (c) {
-          const uint32_t k = m + __popc(bal & lt);
+          const uint32_t k = c >= kPtLong ? n_long + __popc(bl & lt)
+                                          : kPtSlots - 1u - n_short - __popc(bs & lt);
           W.s_lo[k] = lo;
           W.s_cnt[k] = c;
           W.s_code[k] = code;
         }
-        m += __popc(bal);
+        n_long += __popc(bl);
+        n_short += __popc(bs);
       }
       __syncwarp();
-      for (uint32_t g = 0; g < m && left; g += 32) {
-        const uint32_t k = g + lane;
-        const uint32_t c = k < m ? W.s_cnt[k] : 0u;
+      // long ranges: a slot at a time, its strings in registers
+      for (uint32_t k = 0; k < n_long && left; k++) {
+        const uint32_t c = W.s_cnt[k];
+        if (skip >= c) {
+          skip -= c;
+          continue;
+        }
+        const uint32_t end = min(c, skip + left);
+        left -= end - skip;
+        const uint32_t code = W.s_code[k];
+        const uint64_t A = code & kADn ? bd : bu;
+        const uint64_t B = code & kOne ? 0ull : code & kBDn ? bd : bu;
+        const uint32_t* __restrict__ q = (code & kOne ? P.s_r : P.d_rs) + W.s_lo[k];
+        for (uint32_t t = skip + lane; t < end + lane; t += 64) {
+          const bool v0 = t < end, v1 = t + 32 < end;
+          const uint32_t x0 = v0 ? q[t] : 0u, x1 = v1 ? q[t + 32] : 0u;
+          uint32_t s0 = x0 >> 16, s1 = x1 >> 16;
+          if (s0 >= n_off) s0 -= n_off;
+          if (s1 >= n_off) s1 -= n_off;
+          const uint32_t r0 = x0 & 0xffffu, r1 = x1 & 0xffffu;
+          push_a(v0 && !(bit_of(A, r0) | bit_of(B, s0)), code | r0 << kRBit | s0 << kSBit, piece);
+          push_a(v1 && !(bit_of(A, r1) | bit_of(B, s1)), code | r1 << kRBit | s1 << kSBit, piece);
+        }
+        skip = 0;
+      }
+      // short ranges: 32 slots' entries flattened over the lanes
+      for (uint32_t g = 0; g < n_short && left; g += 32) {
+        const uint32_t k = kPtSlots - 1u - (g + lane);
+        const uint32_t c = g + lane < n_short ? W.s_cnt[k] : 0u;
         uint32_t inc = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -510,33 +556,20 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
           }
           const uint32_t o_first = __shfl_sync(kFull, first, ol);
           bool pass = false;
-          uint32_t rs = 0, code = 0;
+          uint32_t x = 0;
           if (t < end) {
-            code = W.s_code[g + ol];
-            const uint32_t e = W.s_lo[g + ol] + (t - o_first);
+            const uint32_t ok = kPtSlots - 1u - (g + ol);
+            const uint32_t code = W.s_code[ok];
+            const uint32_t e = W.s_lo[ok] + (t - o_first);
             const uint64_t A = code & kADn ? bd : bu;
-            if (code & kOne) {
-              rs = P.s_r[e];
-              pass = !bit_of(A, rs);
-            } else {
-              rs = P.d_rs[e];
-              const uint64_t B = code & kBDn ? bd : bu;
-              uint32_t x = rs >> 16;
-              if (x >= n_mask_off) x -= n_mask_off;
-              rs = (rs & 0xffffu) | (x << 16);
-              pass = !(bit_of(A, rs & 0xffffu) | bit_of(B, x));
-            }
+            const uint64_t B = code & kOne ? 0ull : code & kBDn ? bd : bu;
+            const uint32_t rs = code & kOne ? P.s_r[e] : P.d_rs[e];
+            uint32_t r = rs & 0xffffu, s = rs >> 16;
+            if (s >= n_off) s -= n_off;
+            pass = !(bit_of(A, r) | bit_of(B, s));
+            x = code | r << kRBit | s << kSBit;
           }
-          const unsigned bal = __ballot_sync(kFull, pass);
-          if (!bal) continue;
-          if (pass) {
-            const uint32_t q = (ah + an + __popc(bal & lt)) & (kPtQ - 1);
-            W.a_rs[q] = rs;
-            W.a_code[q] = code;
-            W.a_piece[q] = piece;
-          }
-          an += __popc(bal);
-          if (an >= 32u) drain_a(32u);
+          push_a(pass, x, piece);
         }
         skip = 0;
       }
