@@ -34,7 +34,6 @@ struct SelParams {
   double max_hci, max_singles;
   int n_orbs, n_up, n_elecs, n_pairs;
   int var_sd;
-  uint32_t pass, n_src_total;  // sources are i = pass + 5 k, i < n_src_total
   // second rejection (chem_system.cc:300-308, 318-324, 364-370): off unless rej_on
   int rej_on;
   double rej_factor;  // second_rejection_factor
@@ -167,60 +166,8 @@ __device__ __forceinline__ double src_eps_min(const SelParams& P, uint32_t i) {
 }
 
 
-// Candidate det for entry e of slot `slot` of det (up, dn).  Returns false when the target
-// orbitals are occupied (the reference's occupancy checks).  *single tells the slot kind.
-__device__ __forceinline__ bool make_candidate(const SelParams& P, uint64_t up, uint64_t dn,
-                                               int slot, uint32_t e, uint64_t* cu,
-                                               uint64_t* cd, bool* single) {
-  const int n = P.n_orbs;
-  *cu = up;
-  *cd = dn;
-  if (slot < P.n_elecs) {
-    *single = true;
-    const bool is_up = slot < P.n_up;
-    const int p = is_up ? nth_bit(up, slot) : nth_bit(dn, slot - P.n_up);
-    const int r = static_cast<int>(P.s_r[e]);
-    // an inactive target (active space) fails like an occupied one
-    if (is_up) {
-      if ((up | P.inactive) >> r & 1) return false;
-      *cu = (up & ~(1ull << p)) | (1ull << r);
-    } else {
-      if ((dn | P.inactive) >> r & 1) return false;
-      *cd = (dn & ~(1ull << p)) | (1ull << r);
-    }
-    return true;
-  }
-  *single = false;
-  const uint32_t pr = P.pair_tab[slot - P.n_elecs];
-  const int p = elec_orb(up, dn, pr & 0xffff, P.n_up, n);
-  const int q = elec_orb(up, dn, pr >> 16, P.n_up, n);
-  const uint32_t rs = P.d_rs[e];
-  int r = rs & 0xffff, s = rs >> 16;
-  if (p >= n && q >= n) {
-    r += n;
-    s += n;
-  } else if (p < n && q >= n && p > q - n) {
-    const int tmp = s - n;
-    s = r + n;
-    r = tmp;
-  }
-  // an inactive target (active space) fails like an occupied one
-  const uint64_t bu = up | P.inactive, bd = dn | P.inactive;
-  const bool occ_r = r < n ? (bu >> r & 1) : (bd >> (r - n) & 1);
-  if (occ_r) return false;
-  const bool occ_s = s < n ? (bu >> s & 1) : (bd >> (s - n) & 1);
-  if (occ_s) return false;
-  uint64_t u = up, d = dn;
-  if (p < n) u &= ~(1ull << p); else d &= ~(1ull << (p - n));
-  if (q < n) u &= ~(1ull << q); else d &= ~(1ull << (q - n));
-  if (r < n) u |= 1ull << r; else d |= 1ull << (r - n);
-  if (s < n) u |= 1ull << s; else d |= 1ull << (s - n);
-  *cu = u;
-  *cd = d;
-  return true;
-}
-
-// make_candidate with the slot's electron orbitals already known (from slot_range).
+// Candidate det for entry e of slot `slot` of det (up, dn), with the slot's electron orbitals from
+// slot_range.  Returns false when the target orbitals are occupied (the reference's occupancy checks).
 __device__ __forceinline__ bool make_candidate_at(const SelParams& P, uint64_t up, uint64_t dn,
                                                   int slot, uint32_t orbs, uint32_t e,
                                                   uint64_t* cu, uint64_t* cd) {

@@ -95,7 +95,7 @@ void jacobi_eig(int k, const double* lower, int ld, double* evals, double* evecs
 
 // select.cu
 size_t select_dets(shci_ctx* c, double eps_var, bool var_sd);
-void rebuild_det_set(shci_ctx* c, size_t n_have = 0, bool allow_dup = false);
+void rebuild_det_set(shci_ctx* c, bool allow_dup = false);
 size_t sort_unique_pairs(shci_ctx* c, DevBuf<uint64_t>& a, DevBuf<uint64_t>& b, size_t m,
                          int a_bits = 0);
 void compact_valid(shci_ctx* c, const uint64_t* a, const uint64_t* b, size_t m,

@@ -34,6 +34,7 @@
 #include "group.cuh"
 #include "heatbath.cuh"
 #include "kernels.h"
+#include "walk.cuh"
 
 namespace shci {
 
@@ -186,80 +187,17 @@ struct PtPieces {
   uint64_t base;  // off of the output arrays' first entry
 };
 
-// Entries a warp walks at most before the next piece: the heaviest determinant's window holds
-// 100,000 entries, 3,000 rounds of one warp.
-constexpr uint32_t kPieceLen = 4096;
 constexpr uint32_t kPtQ = 64;    // queue lengths (< 32 waiting + 32 pushed)
-constexpr uint32_t kPtSlots = 256;  // slots listed at a time
-// Ranges of at least this many entries are walked slot by slot, the others flattened over the lanes:
-// a round of 32 costs about 40 instructions with one slot's strings in registers and about 100
-// when every lane finds its slot (n = 40: 6.4 -> 5.4 ms a pseudo-stochastic batch, 13.4 -> 11.9 ms
-// for six stochastic iterations; a limit of 24 measures the same).
-constexpr uint32_t kPtLong = 12;
 
 struct PtWarp {
-  // slots of the current source with a non-empty range: first entry, entries, code; long ranges
-  // from the front, short ones from the back
-  uint32_t s_lo[kPtSlots], s_cnt[kPtSlots], s_code[kPtSlots];
+  WalkWarp w;
   // stage 1 queue: entries whose targets are free (x: slot code with the targets, y: piece)
   uint2 a[kPtQ];
   // stage 2 queue (several batches): members
   uint64_t b_u[kPtQ], b_d[kPtQ];
   uint32_t b_piece[kPtQ];
   uint8_t b_ent[kPtQ];
-  uint8_t occ[128];  // electron -> spatial orbital, alpha electrons first
 };
-
-// Slot code: the orbitals p and q that the electrons leave, and the strings that the targets r and s
-// of an entry must be free in; a queued entry adds its targets.  A queue entry's r | s << 16 holds
-// the targets of the stored pair; a beta-beta pair is stored as its alpha image and an alpha-beta
-// pair p > q as (q, p) (chem_system.cc:347-361), so the strings follow from the slot alone.
-constexpr int kPBit = 0, kQBit = 6, kRBit = 12, kSBit = 18;
-enum : uint32_t { kADn = 1u << 24, kBDn = 1u << 25, kOne = 1u << 26 };
-
-// Entry range and code of slot `slot`; as slot_range (heatbath.cuh), the orbitals from `occ`.
-__device__ __forceinline__ uint32_t pt_slot(const SelParams& P, const uint8_t* occ, int slot,
-                                            double eps_min, double eps_max, uint32_t* lo,
-                                            uint32_t* cnt) {
-  *lo = 0;
-  *cnt = 0;
-  const int n = P.n_orbs;
-  if (slot < P.n_elecs) {
-    if (eps_min > P.max_singles) return 0;
-    const uint32_t p = occ[slot];
-    const uint32_t a = P.s_off[p], b = P.s_off[p + 1];
-    *lo = a;
-    *cnt = first_below(P.s_S, a, b, eps_min) - a;
-    return p << kPBit | kOne | (slot < P.n_up ? 0u : kADn);
-  }
-  if (P.no_doubles || eps_min > P.max_hci) return 0;
-  const uint32_t pr = P.pair_tab[slot - P.n_elecs];
-  const int e1 = pr & 0xffff, e2 = pr >> 16;
-  const uint32_t p = occ[e1], q = occ[e2];
-  const bool dn1 = e1 >= P.n_up, dn2 = e2 >= P.n_up;
-  uint32_t code;
-  size_t pq;
-  if (dn1 == dn2) {
-    pq = c2(p, q);
-    code = p << kPBit | q << kQBit | (dn1 ? kADn | kBDn : 0u);
-  } else if (p > q) {  // stored as (q, p + n): r goes to beta, s to alpha
-    pq = c2(q, p + n);
-    code = p << kPBit | q << kQBit | kADn;
-  } else {
-    pq = c2(p, q + n);
-    code = p << kPBit | q << kQBit | kBDn;
-  }
-  const uint32_t a = static_cast<uint32_t>(P.d_off[pq]), b = static_cast<uint32_t>(P.d_off[pq + 1]);
-  const uint32_t s = first_below(P.d_H, a, b, eps_max);
-  *lo = s;
-  *cnt = first_below(P.d_H, s, b, eps_min) - s;
-  return code;
-}
-
-__device__ __forceinline__ uint32_t bit_of(uint64_t x, uint32_t k) {
-  const uint32_t w = k & 32u ? static_cast<uint32_t>(x >> 32) : static_cast<uint32_t>(x);
-  return w >> (k & 31u) & 1u;
-}
 
 // Emits the members of each piece into its region: the window entries whose targets are free, that
 // fall in the current hash batch, are not variational and have |H_ai c_i| >= eps (the handler's
@@ -285,8 +223,6 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
   const unsigned lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const uint32_t wpg = gridDim.x * kPtWarps;
-  const int n = P.n_orbs;
-  const uint32_t n_off = static_cast<uint32_t>(n);  // an alpha-beta pair's s is stored as s + n
   uint32_t ah = 0, an = 0, bh = 0, bn = 0;           // warp-uniform ring states
   uint32_t run_piece = 0xffffffffu, run_cnt = 0;      // kept members of the last piece seen
 
@@ -409,22 +345,7 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
       const uint32_t i = src_det(S, kk, MODE);
       cu = P.up[i];
       cd = P.dn[i];
-      const uint64_t out1 = 1ull << (code >> kPBit & 63u), out2 = 1ull << (code >> kQBit & 63u);
-      const uint64_t in1 = 1ull << (code >> kRBit & 63u), in2 = 1ull << (code >> kSBit & 63u);
-      // (targets are in the strings A and B; the electrons that leave: of the first electron's
-      // string and the second's, which for a swapped pair are B and A)
-      const bool a_dn = code & kADn, b_dn = code & kBDn;
-      if (code & kOne) {
-        if (a_dn) cd ^= out1 | in1;
-        else cu ^= out1 | in1;
-      } else if (a_dn == b_dn) {
-        const uint64_t x = out1 | out2 | in1 | in2;
-        if (a_dn) cd ^= x;
-        else cu ^= x;
-      } else {
-        cu ^= out1 | (a_dn ? in2 : in1);
-        cd ^= out2 | (a_dn ? in1 : in2);
-      }
+      apply_entry(code, &cu, &cd);
     }
     if (Q.n_batches <= 1) {
       if (MODE != kSto) {
@@ -467,151 +388,17 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
 
   for (uint32_t piece = blockIdx.x * kPtWarps + (threadIdx.x >> 5); piece < pc.n; piece += wpg) {
     const uint32_t kk = pc.src[piece];
-    uint32_t skip = pc.begin[piece], left = pc.len[piece];
+    const uint32_t skip = pc.begin[piece], left = pc.len[piece];
     const uint32_t i = src_det(S, kk, MODE);
     const double ac = fabs(P.coef[i]);
     const double eps_min = Q.eps / ac;
     const double eps_max = 1.0e100 / ac;
     const uint64_t up = P.up[i], dn = P.dn[i];
-    const uint64_t bu = up | P.inactive, bd = dn | P.inactive;  // (inactive targets: active space)
-    __syncwarp();
-    for (int o = lane; o < n; o += 32) {
-      if (up >> o & 1) W.occ[popc64(up & below(o))] = static_cast<uint8_t>(o);
-      if (dn >> o & 1) W.occ[P.n_up + popc64(dn & below(o))] = static_cast<uint8_t>(o);
-    }
-    __syncwarp();
-    const int n_slots = P.n_elecs + P.n_pairs;
-    for (int f0 = 0; f0 < n_slots && left; f0 += kPtSlots) {
-      // the non-empty slots of this stretch (a piece's entries: the long ranges in slot order, then
-      // the short ones)
-      uint32_t n_long = 0, n_short = 0;
-      const int f1 = min(n_slots, f0 + (int)kPtSlots);
-      for (int s0 = f0; s0 < f1; s0 += 32) {
-        uint32_t lo = 0, c = 0, code = 0;
-        if (s0 + (int)lane < f1)
-          code = pt_slot(P, W.occ, s0 + lane, eps_min, eps_max, &lo, &c);
-        const unsigned bl = __ballot_sync(kFull, c >= kPtLong);
-        const unsigned bs = __ballot_sync(kFull, c && c < kPtLong);
-        if (c) {
-          const uint32_t k = c >= kPtLong ? n_long + __popc(bl & lt)
-                                          : kPtSlots - 1u - n_short - __popc(bs & lt);
-          W.s_lo[k] = lo;
-          W.s_cnt[k] = c;
-          W.s_code[k] = code;
-        }
-        n_long += __popc(bl);
-        n_short += __popc(bs);
-      }
-      __syncwarp();
-      // long ranges: a slot at a time, its strings in registers
-      for (uint32_t k = 0; k < n_long && left; k++) {
-        const uint32_t c = W.s_cnt[k];
-        if (skip >= c) {
-          skip -= c;
-          continue;
-        }
-        const uint32_t end = min(c, skip + left);
-        left -= end - skip;
-        const uint32_t code = W.s_code[k];
-        const uint64_t A = code & kADn ? bd : bu;
-        const uint64_t B = code & kOne ? 0ull : code & kBDn ? bd : bu;
-        const uint32_t* __restrict__ q = (code & kOne ? P.s_r : P.d_rs) + W.s_lo[k];
-        for (uint32_t t = skip + lane; t < end + lane; t += 64) {
-          const bool v0 = t < end, v1 = t + 32 < end;
-          const uint32_t x0 = v0 ? q[t] : 0u, x1 = v1 ? q[t + 32] : 0u;
-          uint32_t s0 = x0 >> 16, s1 = x1 >> 16;
-          if (s0 >= n_off) s0 -= n_off;
-          if (s1 >= n_off) s1 -= n_off;
-          const uint32_t r0 = x0 & 0xffffu, r1 = x1 & 0xffffu;
-          push_a(v0 && !(bit_of(A, r0) | bit_of(B, s0)), code | r0 << kRBit | s0 << kSBit, piece);
-          push_a(v1 && !(bit_of(A, r1) | bit_of(B, s1)), code | r1 << kRBit | s1 << kSBit, piece);
-        }
-        skip = 0;
-      }
-      // short ranges: 32 slots' entries flattened over the lanes
-      for (uint32_t g = 0; g < n_short && left; g += 32) {
-        const uint32_t k = kPtSlots - 1u - (g + lane);
-        const uint32_t c = g + lane < n_short ? W.s_cnt[k] : 0u;
-        uint32_t inc = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(kFull, inc, o);
-          if (lane >= (unsigned)o) inc += t;
-        }
-        const uint32_t total = __shfl_sync(kFull, inc, 31);
-        if (skip >= total) {
-          skip -= total;
-          continue;
-        }
-        const uint32_t end = min(total, skip + left);
-        left -= end - skip;
-        const uint32_t first = inc - c;  // of this lane's slot
-        for (uint32_t t0 = skip; t0 < end; t0 += 32) {
-          const uint32_t t = t0 + lane;
-          uint32_t ol = 0;  // owner: the number of slots that end at or before t
-#pragma unroll
-          for (uint32_t step = 16; step; step >>= 1) {
-            const uint32_t v = __shfl_sync(kFull, inc, ol + step - 1);
-            if (v <= t) ol += step;
-          }
-          const uint32_t o_first = __shfl_sync(kFull, first, ol);
-          bool pass = false;
-          uint32_t x = 0;
-          if (t < end) {
-            const uint32_t ok = kPtSlots - 1u - (g + ol);
-            const uint32_t code = W.s_code[ok];
-            const uint32_t e = W.s_lo[ok] + (t - o_first);
-            const uint64_t A = code & kADn ? bd : bu;
-            const uint64_t B = code & kOne ? 0ull : code & kBDn ? bd : bu;
-            const uint32_t rs = code & kOne ? P.s_r[e] : P.d_rs[e];
-            uint32_t r = rs & 0xffffu, s = rs >> 16;
-            if (s >= n_off) s -= n_off;
-            pass = !(bit_of(A, r) | bit_of(B, s));
-            x = code | r << kRBit | s << kSBit;
-          }
-          push_a(pass, x, piece);
-        }
-        skip = 0;
-      }
-      __syncwarp();
-    }
+    walk_window(P, W.w, up, dn, eps_min, eps_max, skip, left,
+                [&](bool, bool free, uint32_t x, uint32_t) { push_a(free, x, piece); });
   }
   while (an) drain_a(an < 32u ? an : 32u);
   while (bn) drain_b(bn < 32u ? bn : 32u);
-}
-
-// Pieces per source, and the pieces with their region sizes (into off[p], to be scanned): every
-// entry with one batch; with several, a piece's members are a binomial(len, 1 / n_batches) count
-// per entry of the source (a det walked once for several iterations), and len / n_batches * slack +
-// pad exceeds its mean by many standard deviations (pieces that overflow are emitted again).
-__global__ void k_piece_count(const uint64_t* __restrict__ entries, uint32_t n_src, uint32_t* np) {
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src; k += gridDim.x * blockDim.x)
-    np[k] = static_cast<uint32_t>((entries[k] + kPieceLen - 1) / kPieceLen);
-}
-__global__ void k_piece_fill(const uint64_t* __restrict__ entries, const uint32_t* __restrict__ first,
-                             uint32_t n_src, uint64_t n_batches, double slack, double pad,
-                             const uint32_t* __restrict__ ent_off, uint32_t* __restrict__ src,
-                             uint32_t* __restrict__ begin, uint32_t* __restrict__ len,
-                             uint64_t* __restrict__ off) {
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src;
-       k += gridDim.x * blockDim.x) {
-    const uint64_t m = entries[k];
-    const uint64_t mult = ent_off ? ent_off[k + 1] - ent_off[k] : 1u;
-    uint32_t p = first[k];
-    for (uint64_t b = 0; b < m; b += kPieceLen, p++) {
-      const uint64_t l = min(static_cast<unsigned long long>(kPieceLen),
-                             static_cast<unsigned long long>(m - b));
-      uint64_t r = l * mult;
-      if (n_batches > 1) {
-        const double est = ceil(static_cast<double>(r) / static_cast<double>(n_batches) * slack + pad);
-        if (est < static_cast<double>(r)) r = est > 0.0 ? static_cast<uint64_t>(est) : 0ull;
-      }
-      src[p] = k;
-      begin[p] = static_cast<uint32_t>(b);  // (a source's windows hold fewer than 2^32 entries)
-      len[p] = static_cast<uint32_t>(l);
-      off[p] = r;
-    }
-  }
 }
 
 // Members of each piece that were written: none of one whose region was too small (*over counts
@@ -947,53 +734,19 @@ void pt_setup(shci_ctx* c, PtSetup& st) {
   st.grid = static_cast<unsigned>(sms) * 8u;
 }
 
-// Pieces of a set of sources (on the device); piece p's region is [off[p], off[p + 1]).
-struct PieceList {
-  DevBuf<uint32_t> src, begin, len;
-  DevBuf<uint64_t> off;
-  size_t n = 0;
-  uint64_t tot = 0;
-  explicit PieceList(shci_ctx* c) {
-    src.mt = begin.mt = len.mt = &c->mem;
-    off.mt = &c->mem;
-  }
-};
 // Pieces by host arrays (those to be emitted again), with exact sizes.
 struct PieceRerun {
   std::vector<uint32_t> src, begin, len;
   std::vector<uint64_t> off{0};
 };
 
-// Pieces of the sources with `entries` window entries each (device; ent_off as in StoSources).
-// SHCI_PT_SLOTS="slack,pad" replaces the region estimate's 1.3 and 64.
-void make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src, uint64_t n_batches,
-                 const uint32_t* ent_off, PieceList& L) {
+// Region estimate with several batches: SHCI_PT_SLOTS="slack,pad" replaces 1.3 and 64.
+void make_pt_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src,
+                    uint64_t n_batches, const uint32_t* ent_off, PieceList& L) {
   double slack = 1.3, pad = 64.0;
   if (const char* e = std::getenv("SHCI_PT_SLOTS")) std::sscanf(e, "%lf,%lf", &slack, &pad);
-  cudaStream_t s = c->stream;
-  L.n = 0;
-  L.tot = 0;
-  if (n_src == 0) return;
   HostScope hs(c->prof, "pt2_host_offsets");
-  DevBuf<uint32_t> first;
-  first.mt = &c->mem;
-  first.resize(n_src);
-  k_piece_count<<<grid_for(n_src, 256), 256, 0, s>>>(entries.p, n_src, first.p);
-  SHCI_LAUNCH_CHECK();
-  L.n = exclusive_scan_u32(first.p, first.p, n_src, s, c->sort);
-  c->launches += 4;
-  if (L.n == 0) return;
-  L.src.resize(L.n);
-  L.begin.resize(L.n);
-  L.len.resize(L.n);
-  L.off.resize(L.n + 1);
-  k_piece_fill<<<grid_for(n_src, 256), 256, 0, s>>>(entries.p, first.p, n_src, n_batches, slack,
-                                                    pad, ent_off, L.src.p, L.begin.p, L.len.p,
-                                                    L.off.p);
-  SHCI_LAUNCH_CHECK();
-  exclusive_scan_u64_async(L.off.p, L.off.p, L.n, s, c->sort, L.off.p + L.n);
-  SHCI_CUDA(cudaMemcpyAsync(&L.tot, L.off.p + L.n, 8, cudaMemcpyDeviceToHost, s));
-  SHCI_CUDA(cudaStreamSynchronize(s));
+  make_pieces(c, entries, n_src, n_batches, slack, pad, ent_off, L);
 }
 
 // Emits the members of the pieces for one batch (or set of iterations), appending them to rec
@@ -1019,27 +772,9 @@ void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSource
                                  static_cast<int>(smem)));
   size_t k0 = 0;
   uint64_t base = 0;  // off[k0]
-  auto off_at = [&](size_t k) {
-    uint64_t v = 0;
-    SHCI_CUDA(cudaMemcpyAsync(&v, L.off.p + k, 8, cudaMemcpyDeviceToHost, s));
-    SHCI_CUDA(cudaStreamSynchronize(s));
-    return v;
-  };
   while (k0 < L.n) {
-    // the pieces whose regions fit kCap together: all of them, or up to the last whose end does
-    // (one at least)
-    size_t k1 = L.n;
-    uint64_t end = L.tot;
-    if (end - base > kCap) {
-      size_t lo = k0 + 1, hi = L.n;  // off[lo] is taken in any case; off[hi] - base > kCap
-      while (lo + 1 < hi) {
-        const size_t mid = lo + (hi - lo) / 2;
-        if (off_at(mid) - base <= kCap) lo = mid;
-        else hi = mid;
-      }
-      k1 = lo;
-      end = off_at(k1);
-    }
+    uint64_t end = 0;
+    const size_t k1 = piece_run(c, L, k0, base, kCap, &end);
     const uint64_t tot = end - base;
     const uint32_t n = static_cast<uint32_t>(k1 - k0);
     d_cnt.resize((size_t)n + 1);  // (the overflow count after the pieces')
@@ -1210,7 +945,7 @@ Pt2Out pt_batched(shci_ctx* c, double e_var, PtParams Q, size_t n_batches, doubl
   }
   set_batches(Q, n_batches);
   PieceList pieces(c);
-  make_pieces(c, entries, n_var, n_batches, nullptr, pieces);
+  make_pt_pieces(c, entries, n_var, n_batches, nullptr, pieces);
   entries.release();
   Pt2Out out;
   double esum = 0.0, esq = 0.0;
@@ -1347,7 +1082,7 @@ size_t pilot_pt_dets(shci_ctx* c, PtSetup& st, const std::vector<size_t>& src, d
   DevBuf<uint64_t> entries;
   pt_counts<kSto>(c, st, Q, S, n_src, entries);
   PieceList pieces(c);
-  make_pieces(c, entries, n_src, 128, nullptr, pieces);
+  make_pt_pieces(c, entries, n_src, 128, nullptr, pieces);
   DevBuf<PtRec<5>> rec;
   rec.mt = &c->mem;
   return pt_emit_reduce<kSto>(c, st, Q, S, pieces, rec, 5);
@@ -1689,7 +1424,7 @@ Pt2Out pt2_sto(shci_ctx* c, double energy_var, double eps_pt_psto, double eps_pt
     DevBuf<uint64_t> entries;
     pt_counts<kSto>(c, st, Q, S, n_src, entries);
     PieceList pieces(c);
-    make_pieces(c, entries, n_src, n_batches, d_off.p, pieces);
+    make_pt_pieces(c, entries, n_src, n_batches, d_off.p, pieces);
     DevBuf<PtRec<5>> rec;
     rec.mt = &c->mem;
     const size_t bn = pt_emit_reduce<kSto>(c, st, Q, S, pieces, rec, 5);

@@ -235,7 +235,7 @@ void rdm1_dev(shci_ctx* c, double* res_dev) {
   const uint32_t n_dets = static_cast<uint32_t>(c->up.size());
   const int n = c->I.n;
   cudaStream_t s = c->stream;
-  rebuild_det_set(c, 0, true);
+  rebuild_det_set(c, true);
   SelParams P{};
   P.up = c->d_up.p;
   P.dn = c->d_dn.p;

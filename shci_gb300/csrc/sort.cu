@@ -364,9 +364,9 @@ uint32_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, cudaStr
 }
 
 void radix_sort_pairs(DevBuf<uint64_t>& keys, DevBuf<uint32_t>& vals, size_t n, int begin_bit,
-                      int end_bit, cudaStream_t s, SortScratch& sc) {
+                      int end_bit, cudaStream_t s, SortScratch& sc, bool skip) {
   radix_sort_impl<uint64_t, uint32_t>(keys, vals, n, begin_bit, end_bit, s, sc, sc.kalt,
-                                      sc.valt32);
+                                      sc.valt32, skip);
 }
 
 void radix_sort_pairs64(DevBuf<uint64_t>& keys, DevBuf<uint64_t>& vals, size_t n,

@@ -39,11 +39,11 @@ void exclusive_scan_u32_async(const uint32_t* in, uint32_t* out, size_t n, cudaS
 // Stable sort of the first n (keys, vals) by key bits [begin_bit, end_bit).  When the
 // result ends up in the scratch ping-pong buffers, their storage is swapped into `keys` /
 // `vals`, so the caller's buffers always hold the sorted data on return.
+// skip = false: every digit is sorted without looking first which ones vary.
 void radix_sort_pairs(DevBuf<uint64_t>& keys, DevBuf<uint32_t>& vals, size_t n, int begin_bit,
-                      int end_bit, cudaStream_t s, SortScratch& sc);
+                      int end_bit, cudaStream_t s, SortScratch& sc, bool skip = true);
 void radix_sort_pairs64(DevBuf<uint64_t>& keys, DevBuf<uint64_t>& vals, size_t n,
                         int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc);
-// skip = false: every digit is sorted without looking first which ones vary (hash keys).
 void radix_sort_pairs32(DevBuf<uint32_t>& keys, DevBuf<uint32_t>& vals, size_t n,
                         int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc,
                         bool skip = true);

@@ -1,0 +1,91 @@
+// Pieces of the heat-bath windows (walk.cuh).
+#include "walk.cuh"
+
+#include "kernels.h"
+
+namespace shci {
+
+namespace {
+
+__global__ void k_piece_count(const uint64_t* __restrict__ entries, uint32_t n_src, uint32_t* np) {
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src; k += gridDim.x * blockDim.x)
+    np[k] = static_cast<uint32_t>((entries[k] + kPieceLen - 1) / kPieceLen);
+}
+
+// Region sizes go into off[p], to be scanned.
+__global__ void k_piece_fill(const uint64_t* __restrict__ entries, const uint32_t* __restrict__ first,
+                             uint32_t n_src, uint64_t n_batches, double slack, double pad,
+                             const uint32_t* __restrict__ ent_off, uint32_t* __restrict__ src,
+                             uint32_t* __restrict__ begin, uint32_t* __restrict__ len,
+                             uint64_t* __restrict__ off) {
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src;
+       k += gridDim.x * blockDim.x) {
+    const uint64_t m = entries[k];
+    const uint64_t mult = ent_off ? ent_off[k + 1] - ent_off[k] : 1u;
+    uint32_t p = first[k];
+    for (uint64_t b = 0; b < m; b += kPieceLen, p++) {
+      const uint64_t l = min(static_cast<unsigned long long>(kPieceLen),
+                             static_cast<unsigned long long>(m - b));
+      uint64_t r = l * mult;
+      if (n_batches > 1) {
+        const double est = ceil(static_cast<double>(r) / static_cast<double>(n_batches) * slack + pad);
+        if (est < static_cast<double>(r)) r = est > 0.0 ? static_cast<uint64_t>(est) : 0ull;
+      }
+      src[p] = k;
+      begin[p] = static_cast<uint32_t>(b);  // (a source's windows hold fewer than 2^32 entries)
+      len[p] = static_cast<uint32_t>(l);
+      off[p] = r;
+    }
+  }
+}
+
+}  // namespace
+
+void make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src, uint64_t n_batches,
+                 double slack, double pad, const uint32_t* ent_off, PieceList& L) {
+  cudaStream_t s = c->stream;
+  L.n = 0;
+  L.tot = 0;
+  if (n_src == 0) return;
+  DevBuf<uint32_t> first;
+  first.mt = &c->mem;
+  first.resize(n_src);
+  k_piece_count<<<grid_for(n_src, 256), 256, 0, s>>>(entries.p, n_src, first.p);
+  SHCI_LAUNCH_CHECK();
+  L.n = exclusive_scan_u32(first.p, first.p, n_src, s, c->sort);
+  c->launches += 4;
+  if (L.n == 0) return;
+  L.src.resize(L.n);
+  L.begin.resize(L.n);
+  L.len.resize(L.n);
+  L.off.resize(L.n + 1);
+  k_piece_fill<<<grid_for(n_src, 256), 256, 0, s>>>(entries.p, first.p, n_src, n_batches, slack,
+                                                    pad, ent_off, L.src.p, L.begin.p, L.len.p,
+                                                    L.off.p);
+  SHCI_LAUNCH_CHECK();
+  exclusive_scan_u64_async(L.off.p, L.off.p, L.n, s, c->sort, L.off.p + L.n);
+  SHCI_CUDA(cudaMemcpyAsync(&L.tot, L.off.p + L.n, 8, cudaMemcpyDeviceToHost, s));
+  SHCI_CUDA(cudaStreamSynchronize(s));
+}
+
+size_t piece_run(shci_ctx* c, const PieceList& L, size_t k0, uint64_t base, uint64_t cap,
+                 uint64_t* end) {
+  *end = L.tot;
+  if (L.tot - base <= cap) return L.n;
+  auto off_at = [&](size_t k) {
+    uint64_t v = 0;
+    SHCI_CUDA(cudaMemcpyAsync(&v, L.off.p + k, 8, cudaMemcpyDeviceToHost, c->stream));
+    SHCI_CUDA(cudaStreamSynchronize(c->stream));
+    return v;
+  };
+  size_t lo = k0 + 1, hi = L.n;  // off[lo] is taken in any case; off[hi] - base > cap
+  while (lo + 1 < hi) {
+    const size_t mid = lo + (hi - lo) / 2;
+    if (off_at(mid) - base <= cap) lo = mid;
+    else hi = mid;
+  }
+  *end = off_at(lo);
+  return lo;
+}
+
+}  // namespace shci

@@ -1,0 +1,247 @@
+// Walking the heat-bath windows of determinants (PT2 emission and selection).
+//
+// ChemSystem::find_connected_dets (src/chem/chem_system.cc:289-402) walks, for each electron and each
+// electron pair of a determinant (a slot), the entries of one queue from eps_max down to eps_min.
+// The windows of all determinants are cut into pieces of at most kPieceLen entries; a warp takes
+// a piece at a time.
+#pragma once
+
+#include "ctx.h"
+#include "heatbath.cuh"
+
+namespace shci {
+
+// Entries a warp walks at most before the next piece: the heaviest determinant's window holds
+// 100,000 entries, 3,000 rounds of one warp.
+constexpr uint32_t kPieceLen = 4096;
+constexpr uint32_t kWalkSlots = 256;  // slots listed at a time
+// Ranges of at least this many entries are walked slot by slot, the others flattened over the lanes:
+// a round of 32 costs about 40 instructions with one slot's strings in registers and about 100
+// when every lane finds its slot (PT2 at n = 40: 6.4 -> 5.4 ms a pseudo-stochastic batch, 13.4 ->
+// 11.9 ms for six stochastic iterations; a limit of 24 measures the same).
+constexpr uint32_t kWalkLong = 12;
+
+// A warp's shared memory.
+struct WalkWarp {
+  // slots of the current source with a non-empty range: first entry, entries, code; long ranges
+  // from the front, short ones from the back
+  uint32_t s_lo[kWalkSlots], s_cnt[kWalkSlots], s_code[kWalkSlots];
+  uint8_t occ[128];  // electron -> spatial orbital, alpha electrons first
+};
+
+// Slot code: the orbitals p and q that the electrons leave, and the strings that the targets r and s
+// of an entry must be free in; a queued entry adds its targets.  A queue entry's r | s << 16 holds
+// the targets of the stored pair; a beta-beta pair is stored as its alpha image and an alpha-beta
+// pair p > q as (q, p) (chem_system.cc:347-361), so the strings follow from the slot alone.
+constexpr int kPBit = 0, kQBit = 6, kRBit = 12, kSBit = 18;
+enum : uint32_t { kADn = 1u << 24, kBDn = 1u << 25, kOne = 1u << 26 };
+
+// Entry range and code of slot `slot`; as slot_range (heatbath.cuh), the orbitals from `occ`.
+__device__ __forceinline__ uint32_t walk_slot(const SelParams& P, const uint8_t* occ, int slot,
+                                            double eps_min, double eps_max, uint32_t* lo,
+                                            uint32_t* cnt) {
+  *lo = 0;
+  *cnt = 0;
+  const int n = P.n_orbs;
+  if (slot < P.n_elecs) {
+    if (eps_min > P.max_singles) return 0;
+    const uint32_t p = occ[slot];
+    const uint32_t a = P.s_off[p], b = P.s_off[p + 1];
+    *lo = a;
+    *cnt = first_below(P.s_S, a, b, eps_min) - a;
+    return p << kPBit | kOne | (slot < P.n_up ? 0u : kADn);
+  }
+  if (P.no_doubles || eps_min > P.max_hci) return 0;
+  const uint32_t pr = P.pair_tab[slot - P.n_elecs];
+  const int e1 = pr & 0xffff, e2 = pr >> 16;
+  const uint32_t p = occ[e1], q = occ[e2];
+  const bool dn1 = e1 >= P.n_up, dn2 = e2 >= P.n_up;
+  uint32_t code;
+  size_t pq;
+  if (dn1 == dn2) {
+    pq = c2(p, q);
+    code = p << kPBit | q << kQBit | (dn1 ? kADn | kBDn : 0u);
+  } else if (p > q) {  // stored as (q, p + n): r goes to beta, s to alpha
+    pq = c2(q, p + n);
+    code = p << kPBit | q << kQBit | kADn;
+  } else {
+    pq = c2(p, q + n);
+    code = p << kPBit | q << kQBit | kBDn;
+  }
+  const uint32_t a = static_cast<uint32_t>(P.d_off[pq]), b = static_cast<uint32_t>(P.d_off[pq + 1]);
+  const uint32_t s = first_below(P.d_H, a, b, eps_max);
+  *lo = s;
+  *cnt = first_below(P.d_H, s, b, eps_min) - s;
+  return code;
+}
+
+__device__ __forceinline__ uint32_t bit_of(uint64_t x, uint32_t k) {
+  const uint32_t w = k & 32u ? static_cast<uint32_t>(x >> 32) : static_cast<uint32_t>(x);
+  return w >> (k & 31u) & 1u;
+}
+
+// The determinant that entry `code` (with its targets) makes of (*u, *d).
+__device__ __forceinline__ void apply_entry(uint32_t code, uint64_t* u, uint64_t* d) {
+  const uint64_t out1 = 1ull << (code >> kPBit & 63u), out2 = 1ull << (code >> kQBit & 63u);
+  const uint64_t in1 = 1ull << (code >> kRBit & 63u), in2 = 1ull << (code >> kSBit & 63u);
+  // (targets are in the strings A and B; the electrons that leave: of the first electron's string
+  // and the second's, which for a swapped pair are B and A)
+  const bool a_dn = code & kADn, b_dn = code & kBDn;
+  if (code & kOne) {
+    if (a_dn) *d ^= out1 | in1;
+    else *u ^= out1 | in1;
+  } else if (a_dn == b_dn) {
+    const uint64_t x = out1 | out2 | in1 | in2;
+    if (a_dn) *d ^= x;
+    else *u ^= x;
+  } else {
+    *u ^= out1 | (a_dn ? in2 : in1);
+    *d ^= out2 | (a_dn ? in1 : in2);
+  }
+}
+
+// Entries [skip, skip + left) of det (up, dn)'s windows [eps_min, eps_max), 32 at a time: all lanes
+// call push(valid, free, x, e) with x = slot code and targets, e = queue entry, free = both
+// targets are free (valid lanes only).
+template <class Push>
+__device__ __forceinline__ void walk_window(const SelParams& P, WalkWarp& W, uint64_t up,
+                                            uint64_t dn, double eps_min, double eps_max,
+                                            uint32_t skip, uint32_t left, Push&& push) {
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int n = P.n_orbs;
+  const uint32_t n_off = static_cast<uint32_t>(n);  // an alpha-beta pair's s is stored as s + n
+  const uint64_t bu = up | P.inactive, bd = dn | P.inactive;  // (inactive targets: active space)
+  __syncwarp();
+  for (int o = lane; o < n; o += 32) {
+    if (up >> o & 1) W.occ[popc64(up & below(o))] = static_cast<uint8_t>(o);
+    if (dn >> o & 1) W.occ[P.n_up + popc64(dn & below(o))] = static_cast<uint8_t>(o);
+  }
+  __syncwarp();
+  const int n_slots = P.n_elecs + P.n_pairs;
+  for (int f0 = 0; f0 < n_slots && left; f0 += kWalkSlots) {
+    // the non-empty slots of this stretch (a piece's entries: the long ranges in slot order, then
+    // the short ones)
+    uint32_t n_long = 0, n_short = 0;
+    const int f1 = min(n_slots, f0 + (int)kWalkSlots);
+    for (int s0 = f0; s0 < f1; s0 += 32) {
+      uint32_t lo = 0, c = 0, code = 0;
+      if (s0 + (int)lane < f1)
+        code = walk_slot(P, W.occ, s0 + lane, eps_min, eps_max, &lo, &c);
+      const unsigned bl = __ballot_sync(kFull, c >= kWalkLong);
+      const unsigned bs = __ballot_sync(kFull, c && c < kWalkLong);
+      if (c) {
+        const uint32_t k = c >= kWalkLong ? n_long + __popc(bl & lt)
+                                        : kWalkSlots - 1u - n_short - __popc(bs & lt);
+        W.s_lo[k] = lo;
+        W.s_cnt[k] = c;
+        W.s_code[k] = code;
+      }
+      n_long += __popc(bl);
+      n_short += __popc(bs);
+    }
+    __syncwarp();
+    // long ranges: a slot at a time, its strings in registers
+    for (uint32_t k = 0; k < n_long && left; k++) {
+      const uint32_t c = W.s_cnt[k];
+      if (skip >= c) {
+        skip -= c;
+        continue;
+      }
+      const uint32_t end = min(c, skip + left);
+      left -= end - skip;
+      const uint32_t code = W.s_code[k];
+      const uint64_t A = code & kADn ? bd : bu;
+      const uint64_t B = code & kOne ? 0ull : code & kBDn ? bd : bu;
+      const uint32_t lo = W.s_lo[k];
+      const uint32_t* __restrict__ q = (code & kOne ? P.s_r : P.d_rs) + lo;
+      for (uint32_t t = skip + lane; t < end + lane; t += 64) {
+        const bool v0 = t < end, v1 = t + 32 < end;
+        const uint32_t x0 = v0 ? q[t] : 0u, x1 = v1 ? q[t + 32] : 0u;
+        uint32_t s0 = x0 >> 16, s1 = x1 >> 16;
+        if (s0 >= n_off) s0 -= n_off;
+        if (s1 >= n_off) s1 -= n_off;
+        const uint32_t r0 = x0 & 0xffffu, r1 = x1 & 0xffffu;
+        push(v0, v0 && !(bit_of(A, r0) | bit_of(B, s0)), code | r0 << kRBit | s0 << kSBit, lo + t);
+        push(v1, v1 && !(bit_of(A, r1) | bit_of(B, s1)), code | r1 << kRBit | s1 << kSBit,
+             lo + t + 32);
+      }
+      skip = 0;
+    }
+    // short ranges: 32 slots' entries flattened over the lanes
+    for (uint32_t g = 0; g < n_short && left; g += 32) {
+      const uint32_t k = kWalkSlots - 1u - (g + lane);
+      const uint32_t c = g + lane < n_short ? W.s_cnt[k] : 0u;
+      uint32_t inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, inc, o);
+        if (lane >= (unsigned)o) inc += t;
+      }
+      const uint32_t total = __shfl_sync(kFull, inc, 31);
+      if (skip >= total) {
+        skip -= total;
+        continue;
+      }
+      const uint32_t end = min(total, skip + left);
+      left -= end - skip;
+      const uint32_t first = inc - c;  // of this lane's slot
+      for (uint32_t t0 = skip; t0 < end; t0 += 32) {
+        const uint32_t t = t0 + lane;
+        uint32_t ol = 0;  // owner: the number of slots that end at or before t
+#pragma unroll
+        for (uint32_t step = 16; step; step >>= 1) {
+          const uint32_t v = __shfl_sync(kFull, inc, ol + step - 1);
+          if (v <= t) ol += step;
+        }
+        const uint32_t o_first = __shfl_sync(kFull, first, ol);
+        bool free = false;
+        uint32_t x = 0, e = 0;
+        if (t < end) {
+          const uint32_t ok = kWalkSlots - 1u - (g + ol);
+          const uint32_t code = W.s_code[ok];
+          e = W.s_lo[ok] + (t - o_first);
+          const uint64_t A = code & kADn ? bd : bu;
+          const uint64_t B = code & kOne ? 0ull : code & kBDn ? bd : bu;
+          const uint32_t rs = code & kOne ? P.s_r[e] : P.d_rs[e];
+          uint32_t r = rs & 0xffffu, s = rs >> 16;
+          if (s >= n_off) s -= n_off;
+          free = !(bit_of(A, r) | bit_of(B, s));
+          x = code | r << kRBit | s << kSBit;
+        }
+        push(t < end, free, x, e);
+      }
+      skip = 0;
+    }
+    __syncwarp();
+  }
+}
+
+// ---- pieces -------------------------------------------------------------------------------------
+
+// Pieces of a set of sources (on the device); piece p's region is [off[p], off[p + 1]).
+struct PieceList {
+  DevBuf<uint32_t> src, begin, len;
+  DevBuf<uint64_t> off;
+  size_t n = 0;
+  uint64_t tot = 0;
+  explicit PieceList(shci_ctx* c) {
+    src.mt = begin.mt = len.mt = &c->mem;
+    off.mt = &c->mem;
+  }
+};
+
+// walk.cu: pieces of the sources with `entries` window entries each (device).  A piece's region: its
+// length with one batch; with several, a piece's members are a binomial(len, 1 / n_batches) count
+// per entry of the source (ent_off: a det walked once for several entries), and len / n_batches *
+// slack + pad exceeds its mean by many standard deviations (pieces that overflow are emitted
+// again).
+void make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src, uint64_t n_batches,
+                 double slack, double pad, const uint32_t* ent_off, PieceList& L);
+
+// walk.cu: the end of the run of pieces from k0 whose regions together hold at most `cap` (one piece
+// at least); base = off[k0], *end = off[result].
+size_t piece_run(shci_ctx* c, const PieceList& L, size_t k0, uint64_t base, uint64_t cap,
+                 uint64_t* end);
+
+}  // namespace shci
