@@ -15,6 +15,7 @@
 
 #include "ctx.h"
 #include "kernels.h"
+#include "spmv.cuh"
 
 namespace shci {
 
@@ -43,29 +44,45 @@ struct Ptrs6 {
   const double* p[6];
 };
 
-// partial[m * kDotBlocks + b] = block b's share of <x, ys[m]> (ys[m] null: of sum x)
+// Ends a reduction over the grid: every block leaves its m partial sums, and the block that arrives
+// last adds them up in block order into out[0, m) (so the result does not depend on timing) and
+// resets the counter.  A second launch for that sum cost as much as the sum itself.
+__device__ __forceinline__ void grid_sums(const double* acc, int m, double* __restrict__ partial,
+                                          unsigned* __restrict__ counter,
+                                          double* __restrict__ out) {
+  __shared__ bool last;
+  for (int k = 0; k < m; k++) {
+    const double t = block_sum(acc[k]);
+    if (threadIdx.x == 0) partial[k * kDotBlocks + blockIdx.x] = t;
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(counter, 1u) + 1u == gridDim.x;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int k = 0; k < m; k++) {
+    double v = 0.0;
+    for (int b = threadIdx.x; b < static_cast<int>(gridDim.x); b += blockDim.x)
+      v += __ldcg(partial + k * kDotBlocks + b);
+    const double t = block_sum(v);
+    if (threadIdx.x == 0) out[k] = t;
+  }
+  if (threadIdx.x == 0) *counter = 0u;
+}
+
+// out[k] = <x, ys[k]> (ys[k] null: sum of x), k < m <= 6
 __global__ void __launch_bounds__(kDotThreads)
-    k_mdot_partial(const double* __restrict__ x, Ptrs6 ys, int m, size_t n,
-                   double* __restrict__ partial) {
+    k_mdot(const double* __restrict__ x, Ptrs6 ys, int m, size_t n, double* __restrict__ partial,
+           unsigned* __restrict__ counter, double* __restrict__ out) {
   double acc[6] = {0, 0, 0, 0, 0, 0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const double xi = x[i];
     for (int k = 0; k < m; k++) acc[k] += ys.p[k] ? xi * ys.p[k][i] : xi;
   }
-  for (int k = 0; k < m; k++) {
-    const double t = block_sum(acc[k]);
-    if (threadIdx.x == 0) partial[k * kDotBlocks + blockIdx.x] = t;
-  }
-}
-
-__global__ void k_mdot_final(const double* __restrict__ partial, int m, double* out) {
-  for (int k = 0; k < m; k++) {
-    double v = 0.0;
-    for (int b = threadIdx.x; b < kDotBlocks; b += blockDim.x) v += partial[k * kDotBlocks + b];
-    const double t = block_sum(v);
-    if (threadIdx.x == 0) out[k] = t;
-  }
+  grid_sums(acc, m, partial, counter, out);
 }
 
 // v -= (*coef) * u
@@ -134,12 +151,90 @@ __global__ void k_combine_n(double* __restrict__ w, double* __restrict__ hw, Com
   }
 }
 
+// One step of davidson() up to the product: the Ritz vector of the last subspace solve (cb.k > 0), the
+// preconditioned residual (davidson.cc:135-143), Gram-Schmidt (:146-152) and the norm, each sum in
+// the pass that forms its vector.  A step was 9 to 11 + 3 ic launches and two synchronisations around
+// the product; now 4 + ic and one (n = 16 FP64 variation, 33 products: 9.7 -> 7.7 ms; n = 26 mixed, 48
+// products: 27.8 -> 25.3 ms).
+//
+// w = sum_k e_k v_k, hw = sum_k e_k hv_k; v = (hw - lambda w) / (lambda - d), 0 where |lambda - d| <
+// 1e-8; out[0] = <v, next> (next null: <v, v>).  *xmax (mixed products) is cleared.
+__global__ void __launch_bounds__(kDotThreads)
+    k_ritz_precond(double* __restrict__ w, double* __restrict__ hw, Comb cb,
+                   double* __restrict__ v, const double* __restrict__ diag, double lambda,
+                   const double* __restrict__ next, size_t n, double* __restrict__ partial,
+                   unsigned* __restrict__ counter, double* __restrict__ out,
+                   double* __restrict__ xmax) {
+  if (xmax && blockIdx.x == 0 && threadIdx.x == 0) *xmax = 0.0;
+  double acc = 0.0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    double a, b;
+    if (cb.k) {
+      a = b = 0.0;
+      for (int k = 0; k < cb.k; k++) {
+        a += cb.v[k][i] * cb.e[k];
+        b += cb.hv[k][i] * cb.e[k];
+      }
+      w[i] = a;
+      hw[i] = b;
+    } else {
+      a = w[i];
+      b = hw[i];
+    }
+    const double d = lambda - diag[i];
+    const double x = fabs(d) < 1.0e-8 ? 0.0 : (b - lambda * a) / d;
+    v[i] = x;
+    acc += x * (next ? next[i] : x);
+  }
+  grid_sums(&acc, 1, partial, counter, out);
+}
+
+// v -= (*coef) * u; out[0] = <v, next> (next null: <v, v>)
+__global__ void __launch_bounds__(kDotThreads)
+    k_axpy_dot(double* __restrict__ v, const double* __restrict__ u,
+               const double* __restrict__ coef, const double* __restrict__ next, size_t n,
+               double* __restrict__ partial, unsigned* __restrict__ counter,
+               double* __restrict__ out) {
+  const double a = *coef;
+  double acc = 0.0;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const double x = v[i] - a * u[i];
+    v[i] = x;
+    acc += x * (next ? next[i] : x);
+  }
+  grid_sums(&acc, 1, partial, counter, out);
+}
+
+// The mixed product's end (spmv.cu, k_fix_out) and its dots: hv = yfix * 2^-s + diag * v, out[k] =
+// <hv, ys[k]>.
+__global__ void __launch_bounds__(kDotThreads)
+    k_fix_rows(const unsigned long long* __restrict__ yfix, const double* __restrict__ scal,
+               const double* __restrict__ diag, const double* __restrict__ v,
+               double* __restrict__ hv, Ptrs6 ys, int m, size_t n, double* __restrict__ partial,
+               unsigned* __restrict__ counter, double* __restrict__ out) {
+  const double inv = ldexp(1.0, -fix_scale_of(scal));
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    const double x = static_cast<double>(static_cast<long long>(yfix[i])) * inv + diag[i] * v[i];
+    hv[i] = x;
+    for (int k = 0; k < m; k++) acc[k] += x * ys.p[k][i];
+  }
+  grid_sums(acc, m, partial, counter, out);
+}
+
 class Dots {
  public:
   Dots(shci_ctx* c) : c_(c) {
     c->dav.partial.reserve(6 * kDotBlocks);
-    c->dav.scal.reserve(16);
+    c->dav.scal.reserve(kScal + 1);
+    counter = reinterpret_cast<unsigned*>(c->dav.scal.p + kScal);
+    SHCI_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), c->stream));
   }
+  static constexpr int kScal = 32;  // scalars, then the reductions' block counter
+  unsigned* counter;
   // out_dev[k] = <x, ys[k]>, k < m (stays on the device)
   void mdot(const double* x, std::initializer_list<const double*> ys, size_t n, double* out_dev) {
     Ptrs6 p{};
@@ -148,12 +243,13 @@ class Dots {
     mdot(x, p, m, n, out_dev);
   }
   void mdot(const double* x, const Ptrs6& p, int m, size_t n, double* out_dev) {
-    k_mdot_partial<<<kDotBlocks, kDotThreads, 0, c_->stream>>>(x, p, m, n, c_->dav.partial.p);
+    k_mdot<<<grid(n), kDotThreads, 0, c_->stream>>>(x, p, m, n, c_->dav.partial.p, counter,
+                                                    out_dev);
     SHCI_LAUNCH_CHECK();
-    k_mdot_final<<<1, kDotThreads, 0, c_->stream>>>(c_->dav.partial.p, m, out_dev);
-    SHCI_LAUNCH_CHECK();
-    c_->launches += 2;
+    c_->launches += 1;
   }
+  // (a fixed function of n: the order of a sum follows from the length alone)
+  static unsigned grid(size_t n) { return grid_for(n, kDotThreads, kDotBlocks); }
   double dot_host(const double* a, const double* b, size_t n) {
     mdot(a, {b}, n, c_->dav.scal.p);
     double r = 0.0;
@@ -261,64 +357,86 @@ DavidsonOut davidson(shci_ctx* c, double tol) {
   double lambda = dots.dot_host(D.v[0].p, D.Hv[0].p, n);
   double hk[5 * 5] = {0};
   hk[0] = lambda;
-  SHCI_CUDA(cudaMemcpyAsync(D.w.p, D.v[0].p, n * 8, cudaMemcpyDeviceToDevice, s));
-  SHCI_CUDA(cudaMemcpyAsync(D.Hw.p, D.Hv[0].p, n * 8, cudaMemcpyDeviceToDevice, s));
+  // the Ritz vector still to be formed from the stored vectors: at the next step, or at the end
+  Comb cb{};
+  cb.k = 1;
+  cb.v[0] = D.v[0].p;
+  cb.hv[0] = D.Hv[0].p;
+  cb.e[0] = 1.0;
+  auto form_ritz = [&]() {
+    if (!cb.k) return;
+    k_combine<<<g, 256, 0, s>>>(D.w.p, D.Hw.p, cb, n);
+    SHCI_LAUNCH_CHECK();
+    c->launches += 1;
+    cb.k = 0;
+  };
   out.trace.push_back(lambda);
   double lambda_prev = lambda;
   bool converged = false;
-  double* scal = D.scal.p;
+  double* scal = D.scal.p;       // [0, ic): <v, v_i>, [ic]: <v, v>
+  double* row_dev = scal + 8;    // [0, ic]: <H v, v_i>
+  const unsigned gd = Dots::grid(n);
+  double* xmax = spmv_xmax(c);
   for (size_t it = 1; it < store * 2; it++) {
     const size_t ic = it % store;
     if (it >= store && ic == 0) {  // restart (davidson.cc:115-131)
+      form_ritz();
       SHCI_CUDA(cudaMemcpyAsync(D.v[0].p, D.w.p, n * 8, cudaMemcpyDeviceToDevice, s));
       SHCI_CUDA(cudaMemcpyAsync(D.Hv[0].p, D.Hw.p, n * 8, cudaMemcpyDeviceToDevice, s));
       lambda = dots.dot_host(D.v[0].p, D.Hv[0].p, n);
       hk[0] = lambda;
       continue;
     }
-    k_precond<<<g, 256, 0, s>>>(D.v[ic].p, D.Hw.p, D.w.p, c->H.diag.p, lambda, n);
+    double* v = D.v[ic].p;
+    k_ritz_precond<<<gd, kDotThreads, 0, s>>>(D.w.p, D.Hw.p, cb, v, c->H.diag.p, lambda,
+                                              ic ? D.v[0].p : nullptr, n, D.partial.p,
+                                              dots.counter, scal, xmax);
     SHCI_LAUNCH_CHECK();
+    cb.k = 0;
     for (size_t i = 0; i < ic; i++) {  // Gram-Schmidt (davidson.cc:146-152)
-      dots.mdot(D.v[ic].p, {D.v[i].p}, n, scal);
-      k_axpy_dev<<<g, 256, 0, s>>>(D.v[ic].p, D.v[i].p, scal, n);
+      k_axpy_dot<<<gd, kDotThreads, 0, s>>>(v, D.v[i].p, scal + i,
+                                            i + 1 < ic ? D.v[i + 1].p : nullptr, n, D.partial.p,
+                                            dots.counter, scal + i + 1);
       SHCI_LAUNCH_CHECK();
     }
-    nrm = std::sqrt(dots.dot_host(D.v[ic].p, D.v[ic].p, n));
-    if (nrm < 1e-12) {
+    spmv_normalized(c, v, scal + ic, D.Hv[ic].p);
+    Ptrs6 p{};
+    for (size_t i = 0; i <= ic; i++) p.p[i] = D.v[i].p;
+    if (xmax) {
+      k_fix_rows<<<gd, kDotThreads, 0, s>>>(c->H.yfix.p, c->H.scal.p, c->H.diag.p, v, D.Hv[ic].p,
+                                            p, (int)ic + 1, n, D.partial.p, dots.counter, row_dev);
+      SHCI_LAUNCH_CHECK();
+    } else {
+      dots.mdot(D.Hv[ic].p, p, (int)ic + 1, n, row_dev);
+    }
+    // the norm comes back with the row: a vector without one has cost a product that is dropped
+    double back[16];
+    SHCI_CUDA(cudaMemcpyAsync(back, scal, sizeof(back), cudaMemcpyDeviceToHost, s));
+    SHCI_CUDA(cudaStreamSynchronize(s));
+    if (std::sqrt(back[ic]) < 1e-12) {
       converged = true;
       break;
     }
-    k_scale<<<g, 256, 0, s>>>(D.v[ic].p, nrm, n);
-    SHCI_LAUNCH_CHECK();
-    spmv(c, D.v[ic].p, D.Hv[ic].p, false);
     out.n_matvec++;
-    Ptrs6 p{};
-    for (size_t i = 0; i <= ic; i++) p.p[i] = D.v[i].p;
-    dots.mdot(D.Hv[ic].p, p, (int)ic + 1, n, scal);
-    double row[6];
-    SHCI_CUDA(cudaMemcpyAsync(row, scal, (ic + 1) * 8, cudaMemcpyDeviceToHost, s));
-    SHCI_CUDA(cudaStreamSynchronize(s));
-    for (size_t i = 0; i <= ic; i++) hk[ic * 5 + i] = row[i];
+    for (size_t i = 0; i <= ic; i++) hk[ic * 5 + i] = back[8 + i];
     const int k = static_cast<int>(ic + 1);
     double ev[5], evec[25];
     jacobi_eig(k, hk, 5, ev, evec);
     lambda = ev[0];
     const double factor = evec[0] < 0 ? -1.0 : 1.0;
-    Comb cb{};
     cb.k = k;
     for (int i = 0; i < k; i++) {
       cb.v[i] = D.v[i].p;
       cb.hv[i] = D.Hv[i].p;
       cb.e[i] = evec[i * k] * factor;
     }
-    k_combine<<<g, 256, 0, s>>>(D.w.p, D.Hw.p, cb, n);
-    SHCI_LAUNCH_CHECK();
-    c->launches += 4 + 2 * ic;
+    c->launches += 2 + ic;
     out.trace.push_back(lambda);
     if (std::fabs(lambda - lambda_prev) <= tol) converged = true;
     if (!converged) lambda_prev = lambda;
     if (converged) break;
   }
+  form_ritz();
   SHCI_CUDA(cudaMemcpyAsync(c->d_coef.p, D.w.p, n * 8, cudaMemcpyDeviceToDevice, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
   D.ritz = true;
@@ -505,7 +623,7 @@ double rayleigh_fp64(shci_ctx* c) {
   Dots dots(c);
   if (n > 1 && D.ritz && D.ritz_h == c->H.build_id && c->H.precision != SHCI_PREC_FP64 &&
       D.w.n == n && c->d_coef.n >= n) {
-    D.scal.reserve(8);
+    D.scal.reserve(Dots::kScal + 1);
     SHCI_CUDA(cudaMemsetAsync(D.scal.p, 0, 8, s));
     k_vec_differs<<<grid_for(n, 256, 152 * 8), 256, 0, s>>>(c->d_coef.p, D.w.p, n, D.scal.p);
     SHCI_LAUNCH_CHECK();
@@ -515,10 +633,13 @@ double rayleigh_fp64(shci_ctx* c) {
     if (differs == 0.0) {
       D.rt.mt = &c->mem;
       const size_t len = residual_rows(c, D.w.p, D.rt);
-      const double num = dots.dot_host(D.w.p, D.Hw.p, n) + 2.0 * dots.dot_host(D.rt.p, nullptr, len);
-      const double den = dots.dot_host(D.w.p, D.w.p, n);
+      double r[3];  // w^T Hw, w^T w, w^T R w / 2
+      dots.mdot(D.w.p, {D.Hw.p, D.w.p}, n, D.scal.p);
+      dots.mdot(D.rt.p, {nullptr}, len, D.scal.p + 2);
+      SHCI_CUDA(cudaMemcpyAsync(r, D.scal.p, sizeof(r), cudaMemcpyDeviceToHost, s));
+      SHCI_CUDA(cudaStreamSynchronize(s));
       c->launches += 1;
-      return num / den;
+      return (r[0] + 2.0 * r[2]) / r[1];
     }
   }
   return rayleigh_fp64_of(c, c->d_coef.p);

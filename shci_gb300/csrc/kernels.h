@@ -62,6 +62,11 @@ void build_items(shci_ctx* c);
 
 // spmv.cu: y = H x (FP64 vectors on the device); residual adds the FP32 residual store.
 void spmv(shci_ctx* c, const double* x, double* y, bool residual);
+// Davidson's product: v /= sqrt(*norm2), then y = H v; with a mixed store y is left in the fixed-point
+// sums H.yfix (scale from H.scal), for the caller to add diag * v to.  A mixed product needs
+// *spmv_xmax(c) (null for FP64) set to 0 before.
+double* spmv_xmax(shci_ctx* c);
+void spmv_normalized(shci_ctx* c, double* v, const double* norm2, double* y);
 // out[k] = w_i sum_j R_ij w_j over work item k of row i of the residual store R (mixed H, upper
 // elements; unused entries 0).  Returns the length of out.
 size_t residual_rows(shci_ctx* c, const double* w, DevBuf<double>& out);

@@ -29,6 +29,7 @@
 #include "ctx.h"
 #include "items.cuh"
 #include "kernels.h"
+#include "spmv.cuh"
 
 namespace shci {
 
@@ -116,20 +117,18 @@ __device__ __forceinline__ void prod2(float v, float r, float xh, float xl, floa
   *e = t;
 }
 
-// Scale exponent s with B * 2^s < 2^61 (B > 0), from the bound's binary exponent.
-__device__ __forceinline__ int fix_scale(double B) {
-  if (!(B > 0.0)) return 0;
-  const int e = static_cast<int>((__double_as_longlong(B) >> 52) & 0x7ff) - 1022;  // B < 2^e
-  return 61 - e;
-}
-
 // x -> float pairs; max |x| (as ordered bits of a non-negative double) into *xmax_bits; the
-// fixed-point accumulators (when given) cleared.
+// fixed-point accumulators (when given) cleared.  norm2 (when given): x is divided by its root first,
+// in place.
+template <bool NORM>
 __global__ void k_split_x(const double* __restrict__ x, uint32_t n, float2* xs,
-                          unsigned long long* xmax_bits, unsigned long long* yfix) {
+                          unsigned long long* xmax_bits, unsigned long long* yfix,
+                          const double* __restrict__ norm2, double* __restrict__ x_out) {
   unsigned long long mx = 0;
+  const double nrm = NORM ? sqrt(*norm2) : 1.0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double v = x[i];
+    const double v = NORM ? x_out[i] / nrm : x[i];
+    if (NORM) x_out[i] = v;
     const float h = static_cast<float>(v);
     const float l = static_cast<float>(v - static_cast<double>(h));
     xs[i] = make_float2(h, l);
@@ -143,6 +142,18 @@ __global__ void k_split_x(const double* __restrict__ x, uint32_t n, float2* xs,
     mx = t > mx ? t : mx;
   }
   if ((threadIdx.x & 31) == 0) atomicMax(xmax_bits, mx);
+}
+
+// v /= sqrt(*norm2), y = diag * v
+__global__ void k_normalize_diag(double* __restrict__ v, const double* __restrict__ norm2,
+                                 const double* __restrict__ diag, double* __restrict__ y,
+                                 uint32_t n) {
+  const double s = sqrt(*norm2);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double x = v[i] / s;
+    v[i] = x;
+    y[i] = diag[i] * x;
+  }
 }
 
 // Off-diagonal row abs sums of the full symmetric matrix, in float.
@@ -184,8 +195,7 @@ template <bool RES>
 __global__ void __launch_bounds__(256)
     k_spmv_fix(const __grid_constant__ ItemTab T, const float2* __restrict__ xs,
                const double* __restrict__ scal, unsigned long long* __restrict__ yfix) {
-  const int s = fix_scale(scal[0] * __longlong_as_double(static_cast<long long>(
-                                        reinterpret_cast<const unsigned long long*>(scal)[1])));
+  const int s = fix_scale_of(scal);
   const unsigned lane = threadIdx.x & 31;
   for_items(T, [&](const ItemSeg& S, uint64_t, uint32_t i, uint64_t rs, uint32_t len) {
     const float2 xi = xs[i];
@@ -223,8 +233,7 @@ __global__ void __launch_bounds__(256)
 __global__ void k_fix_out(const unsigned long long* __restrict__ yfix,
                           const double* __restrict__ diag, const double* __restrict__ x,
                           const double* __restrict__ scal, double* __restrict__ y, uint32_t n) {
-  const int s = fix_scale(scal[0] * __longlong_as_double(static_cast<long long>(
-                                        reinterpret_cast<const unsigned long long*>(scal)[1])));
+  const int s = fix_scale_of(scal);
   const double inv = ldexp(1.0, -s);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     y[i] = static_cast<double>(static_cast<long long>(yfix[i])) * inv + diag[i] * x[i];
@@ -355,9 +364,8 @@ size_t residual_rows(shci_ctx* c, const double* w, DevBuf<double>& out) {
   H.xs.resize(2 * (size_t)n, 1.1);
   float2* ws = reinterpret_cast<float2*>(H.xs.p);
   SHCI_CUDA(cudaMemsetAsync(H.scal.p + 1, 0, 8, s));
-  k_split_x<<<grid_for(n, 256), 256, 0, s>>>(w, n, ws,
-                                             reinterpret_cast<unsigned long long*>(H.scal.p + 1),
-                                             nullptr);
+  k_split_x<false><<<grid_for(n, 256), 256, 0, s>>>(
+      w, n, ws, reinterpret_cast<unsigned long long*>(H.scal.p + 1), nullptr, nullptr, nullptr);
   SHCI_LAUNCH_CHECK();
   SHCI_CUDA(cudaMemsetAsync(out.p, 0, len * 8, s));
   k_res_rows<<<item_grid(c, len), 256, 0, s>>>(T, ws, w, out.p);
@@ -389,8 +397,8 @@ void spmv(shci_ctx* c, const double* x, double* y, bool residual) {
   ProfScope ps(c->prof, s, "spmv");
   SHCI_CUDA(cudaMemsetAsync(H.scal.p + 1, 0, 8, s));
   float2* xs = reinterpret_cast<float2*>(H.xs.p);
-  k_split_x<<<grid_for(n, 256), 256, 0, s>>>(
-      x, n, xs, reinterpret_cast<unsigned long long*>(H.scal.p + 1), H.yfix.p);
+  k_split_x<false><<<grid_for(n, 256), 256, 0, s>>>(
+      x, n, xs, reinterpret_cast<unsigned long long*>(H.scal.p + 1), H.yfix.p, nullptr, nullptr);
   SHCI_LAUNCH_CHECK();
   if (residual) k_spmv_fix<true><<<grid, 256, 0, s>>>(T, xs, H.scal.p, H.yfix.p);
   else k_spmv_fix<false><<<grid, 256, 0, s>>>(T, xs, H.scal.p, H.yfix.p);
@@ -398,6 +406,38 @@ void spmv(shci_ctx* c, const double* x, double* y, bool residual) {
   k_fix_out<<<grid_for(n, 256), 256, 0, s>>>(H.yfix.p, H.diag.p, x, H.scal.p, y, n);
   SHCI_LAUNCH_CHECK();
   c->launches += 3;
+}
+
+double* spmv_xmax(shci_ctx* c) {
+  auto& H = c->H;
+  if (H.precision == SHCI_PREC_FP64) return nullptr;
+  if (!H.bound_valid) mixed_bound(c, item_grid(c, H.n));
+  return H.scal.p + 1;
+}
+
+void spmv_normalized(shci_ctx* c, double* v, const double* norm2, double* y) {
+  auto& H = c->H;
+  cudaStream_t s = c->stream;
+  const uint32_t n = static_cast<uint32_t>(H.n);
+  size_t len = 0;
+  const ItemTab T = item_tab(H, &len);
+  const unsigned grid = item_grid(c, len);
+  ProfScope ps(c->prof, s, "spmv");
+  if (H.precision == SHCI_PREC_FP64) {
+    k_normalize_diag<<<grid_for(n, 256), 256, 0, s>>>(v, norm2, H.diag.p, y, n);
+    SHCI_LAUNCH_CHECK();
+    k_spmv<<<grid, 256, 0, s>>>(T, v, y);
+  } else {
+    H.xs.resize(2 * (size_t)n, 1.1);
+    H.yfix.resize(n, 1.1);
+    float2* xs = reinterpret_cast<float2*>(H.xs.p);
+    k_split_x<true><<<grid_for(n, 256), 256, 0, s>>>(
+        nullptr, n, xs, reinterpret_cast<unsigned long long*>(H.scal.p + 1), H.yfix.p, norm2, v);
+    SHCI_LAUNCH_CHECK();
+    k_spmv_fix<false><<<grid, 256, 0, s>>>(T, xs, H.scal.p, H.yfix.p);
+  }
+  SHCI_LAUNCH_CHECK();
+  c->launches += 2;
 }
 
 }  // namespace shci
