@@ -25,6 +25,31 @@ __global__ void k_elems(DevIntegrals I, const uint64_t* ui, const uint64_t* di, 
   }
 }
 
+// A few pairs come as kernel arguments (32 bytes a pair, at most 32,764 bytes of arguments): a call of
+// 200 pairs spent 16 of its 47 us on four small copies.
+constexpr size_t kArgElems = 1000;
+template <int N>
+struct ElemArgs {
+  uint64_t v[4][N];  // up_i, dn_i, up_j, dn_j
+};
+template <int N>
+__global__ void k_elems_args(const __grid_constant__ DevIntegrals I,
+                             const __grid_constant__ ElemArgs<N> a, uint32_t n, double* out) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const uint64_t ui = a.v[0][k], di = a.v[1][k], uj = a.v[2][k], dj = a.v[3][k];
+  out[k] = ui == uj && di == dj ? h_diag(I, ui, di) : h_offdiag(I, ui, di, uj, dj);
+}
+
+template <int N>
+void launch_elems_args(shci_ctx* c, const uint64_t* const* in, size_t n, double* out) {
+  ElemArgs<N> a;
+  for (int q = 0; q < 4; q++) std::memcpy(a.v[q], in[q], n * 8);
+  k_elems_args<N><<<static_cast<unsigned>((n + 63) / 64), 64, 0, c->stream>>>(
+      c->dI, a, static_cast<uint32_t>(n), out);
+  SHCI_LAUNCH_CHECK();
+}
+
 // Packed copy of the element store: row i of the source [row_ptr[i], + row_len[i]) goes to
 // [ptr[i], ptr[i+1]); values as FP64 (FP64 store, or FP32 value + FP32 residual).
 __global__ void k_pack_rows(const uint64_t* __restrict__ row_ptr, const uint32_t* __restrict__ row_len,
@@ -253,18 +278,26 @@ void hamiltonian_elems(shci_ctx* c, const uint64_t* ui, const uint64_t* di, cons
                        const uint64_t* dj, size_t n, double* out) {
   if (n == 0) return;
   cudaStream_t s = c->stream;
-  DevBuf<uint64_t> b;
-  b.mt = &c->mem;
-  b.resize(4 * n);
   DevBuf<double> o;
   o.mt = &c->mem;
   o.resize(n);
-  SHCI_CUDA(cudaMemcpyAsync(b.p, ui, n * 8, cudaMemcpyHostToDevice, s));
-  SHCI_CUDA(cudaMemcpyAsync(b.p + n, di, n * 8, cudaMemcpyHostToDevice, s));
-  SHCI_CUDA(cudaMemcpyAsync(b.p + 2 * n, uj, n * 8, cudaMemcpyHostToDevice, s));
-  SHCI_CUDA(cudaMemcpyAsync(b.p + 3 * n, dj, n * 8, cudaMemcpyHostToDevice, s));
-  k_elems<<<grid_for(n, 128), 128, 0, s>>>(c->dI, b.p, b.p + n, b.p + 2 * n, b.p + 3 * n, n, o.p);
-  SHCI_LAUNCH_CHECK();
+  DevBuf<uint64_t> b;
+  b.mt = &c->mem;
+  if (n <= kArgElems) {
+    const uint64_t* in[4] = {ui, di, uj, dj};
+    if (n <= 64) launch_elems_args<64>(c, in, n, o.p);
+    else if (n <= 256) launch_elems_args<256>(c, in, n, o.p);
+    else launch_elems_args<kArgElems>(c, in, n, o.p);
+  } else {
+    b.resize(4 * n);
+    SHCI_CUDA(cudaMemcpyAsync(b.p, ui, n * 8, cudaMemcpyHostToDevice, s));
+    SHCI_CUDA(cudaMemcpyAsync(b.p + n, di, n * 8, cudaMemcpyHostToDevice, s));
+    SHCI_CUDA(cudaMemcpyAsync(b.p + 2 * n, uj, n * 8, cudaMemcpyHostToDevice, s));
+    SHCI_CUDA(cudaMemcpyAsync(b.p + 3 * n, dj, n * 8, cudaMemcpyHostToDevice, s));
+    k_elems<<<grid_for(n, 128), 128, 0, s>>>(c->dI, b.p, b.p + n, b.p + 2 * n, b.p + 3 * n, n,
+                                             o.p);
+    SHCI_LAUNCH_CHECK();
+  }
   SHCI_CUDA(cudaMemcpyAsync(out, o.p, n * 8, cudaMemcpyDeviceToHost, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
   c->launches += 1;
