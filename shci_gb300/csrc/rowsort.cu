@@ -37,7 +37,11 @@ namespace shci {
 namespace {
 
 constexpr int kTile = 2048;          // elements per sorted tile
-constexpr int kSortWarps = 16;
+// Eight warps, three CTAs per SM: a tile's phases are separated by about ten barriers, and more,
+// smaller CTAs fill each other's waits (19.7 ms against 21.2 ms for two CTAs of sixteen warps at n = 40,
+// 1.25G elements; 1.34 against 1.68 ms over the seven builds of an n = 26 variation; four CTAs of
+// eight measure the same, six of four warps 36 ms).
+constexpr int kSortWarps = 8;
 constexpr int kSortThreads = kSortWarps * 32;
 constexpr int kBinWords = 2048;      // 65,536-bin bitmap
 constexpr int kPer = kTile / kSortThreads;
@@ -106,7 +110,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 }
 
 template <bool MIXED>
-__global__ void __launch_bounds__(kSortThreads, 2)
+__global__ void __launch_bounds__(kSortThreads, 3)
     k_sort_rows(const uint64_t* __restrict__ row_ptr, const uint32_t* __restrict__ row_len,
                 uint32_t n, uint32_t* col, double* v64, float* v32, float* r32, unsigned* work,
                 int mask_max_s) {
