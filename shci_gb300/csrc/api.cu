@@ -166,6 +166,7 @@ shci_status shci_create(shci_ctx** out, int device, size_t hbm_budget_bytes) {
       b->mt = &c->mem;
     for (auto* b : {&ix.am_dn, &ix.ad_dn, &ix.bd_up, &ix.ua, &ix.ub, &ix.bs_str}) b->mt = &c->mem;
     c->join.pairs.mt = c->join.jdet.mt = &c->mem;
+    c->join.dets.mt = &c->mem;
     c->join.keys.mt = c->join.span.mt = c->join.keys32.mt = &c->mem;
     c->join.scan.mt = c->join.bstart.mt = &c->mem;
     auto& H = c->H;

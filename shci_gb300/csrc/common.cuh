@@ -37,8 +37,8 @@ __device__ __forceinline__ int ctz64(uint64_t x) { return __ffsll((long long)x) 
 __device__ __forceinline__ uint64_t below(int b) { return (1ull << b) - 1ull; }
 
 __device__ __forceinline__ double g2at(const DevIntegrals& I, int p, int q, int r, int s) {
-  const int n = I.n;
-  return I.g2[((size_t)(p * n + q) * n + r) * n + s];
+  const int n = I.n;  // n <= 64: n^4 fits 32 bits
+  return I.g2[static_cast<unsigned>(((p * n + q) * n + r) * n + s)];
 }
 
 // Diagonal element (chem_system.cc:426-432, 444-457, 495-542 without the cache).
@@ -113,8 +113,9 @@ __device__ __forceinline__ double h_single(const DevIntegrals& I, uint64_t same,
                                            int oi, int oj, int odd) {
   const int n = I.n;
   const double ob = flip_sign(I.h1[oi * n + oj], odd);
-  const double* D = I.dtab + (size_t)(oi * n + oj) * n;
-  const double* X = I.xtab + (size_t)(oi * n + oj) * n;
+  const unsigned row = static_cast<unsigned>((oi * n + oj) * n);
+  const double* D = I.dtab + row;
+  const double* X = I.xtab + row;
   double e = 0.0;
   for (uint64_t m = same & ~(1ull << oi) & ~(1ull << oj); m; m &= m - 1) {
     const int o = ctz64(m);

@@ -39,8 +39,9 @@ struct DetIndex {
 // its electrons; entries are sorted by a hash of the det minus that pair.
 struct JoinIndex {
   uint32_t K = 0;               // entries per det = C(n_up + n_dn, 2)
-  int n_up = 0, n_dn = 0;
+  int n_up = 0, n_elecs = 0;
   size_t m = 0;                 // n * K entries
+  DevBuf<ulonglong2> dets;      // [n] (up, dn)
   DevBuf<uint32_t> pairs;       // [K] electron ranks r1 | r2 << 16 (r1 < r2)
   int bits = 0, key_bytes = 0;  // hash bits kept; key width used by the last index
   DevBuf<uint64_t> keys;        // [m] core hashes (sort keys; released after bucketing)

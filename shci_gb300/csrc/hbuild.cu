@@ -442,34 +442,42 @@ namespace {
 // Bound of sum_j |H_ij| over every excitation of det i (both triangles of its row): the singles
 // queue values of its electrons' orbitals (each S_pr bounds |H| of p -> r for any det) plus
 // the doubles queue values of its electron pairs (the exact |H| of each pq -> rs), summed per
-// orbital / pair ahead (s_tot, d_tot); a warp per det, lanes over its electrons.  The mixed
-// H*v only needs a valid bound for its fixed-point scale, and one per det, independent of the
-// det list, saves the fill an FP32 atomic per stored element.
+// orbital / pair ahead (s_tot, d_tot); a warp per det, its electrons listed once in shared memory
+// and its pairs over the lanes.  The mixed H*v only needs a valid bound for its fixed-point
+// scale, and one per det, independent of the det list, saves the fill an FP32 atomic per stored
+// element.
 __global__ void k_hb_row_bound(const uint64_t* __restrict__ up, const uint64_t* __restrict__ dn,
                                uint32_t begin, uint32_t end, int n, int n_up, int n_elecs,
                                const double* __restrict__ stot, const double* __restrict__ dtot,
                                float* __restrict__ rowabs) {
+  __shared__ uint8_t s_occ[8][128];  // spin-orbitals / electron, alpha first (spatial orbital)
   const unsigned lane = threadIdx.x & 31;
+  uint8_t* occ = s_occ[threadIdx.x >> 5];
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const int n_pairs = n_elecs * (n_elecs - 1) / 2;
   for (uint32_t i = begin + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < end;
        i += warps) {
     const uint64_t u = up[i], d = dn[i];
+    __syncwarp();
+    for (int e = lane; e < n_elecs; e += 32) occ[e] = 0;
+    __syncwarp();
+    for (int o = lane; o < n; o += 32) {
+      if (u >> o & 1) occ[popc64(u & below(o))] = static_cast<uint8_t>(o);
+      if (d >> o & 1) occ[n_up + popc64(d & below(o))] = static_cast<uint8_t>(o);
+    }
+    __syncwarp();
     double acc = 0.0;
-    for (int a = static_cast<int>(lane); a < n_elecs; a += 32) {
-      const int p = elec_orb(u, d, a, n_up, n);
-      acc += stot[p < n ? p : p - n];
-      for (int b = a + 1; b < n_elecs; b++) {
-        const int q = elec_orb(u, d, b, n_up, n);
-        int p2 = p, q2 = q;
-        if (p >= n && q >= n) {
-          p2 -= n;
-          q2 -= n;
-        } else if (p < n && q >= n && p > q - n) {
-          p2 = q - n;
-          q2 = p + n;
-        }
-        acc += dtot[c2(p2, q2)];
-      }
+    for (int e = lane; e < n_elecs; e += 32) acc += stot[occ[e]];
+    // pairs (a, b), a < b, by their index in the triangle b (b - 1) / 2 + a
+    for (int t = lane; t < n_pairs; t += 32) {
+      int b = static_cast<int>((1.0f + sqrtf(1.0f + 8.0f * static_cast<float>(t))) * 0.5f);
+      while (b * (b - 1) / 2 > t) b--;
+      while (b * (b + 1) / 2 <= t) b++;
+      const int a = t - b * (b - 1) / 2;
+      const int p = occ[a], q = occ[b];
+      // (stored pairs: both strings' images alpha; an alpha-beta pair p > q as (q, p))
+      const bool same = (a < n_up) == (b < n_up);
+      acc += dtot[same ? c2(p, q) : p > q ? c2(q, p + n) : c2(p, q + n)];
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);

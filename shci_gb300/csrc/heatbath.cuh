@@ -48,11 +48,26 @@ struct SelParams {
 
 constexpr double kSqrt2 = 1.4142135623730951;  // Util::SQRT2 (src/util.h:58)
 
+// Position of the k-th set bit of x (k from 0, below the number of bits): halves by population
+// count, a third of the instructions of __fns.
 __device__ __forceinline__ int nth_bit(uint64_t x, int k) {
-  const unsigned lo = static_cast<unsigned>(x), hi = static_cast<unsigned>(x >> 32);
-  const int cl = __popc(lo);
-  if (k < cl) return __fns(lo, 0, k + 1);
-  return 32 + __fns(hi, 0, k - cl + 1);
+  unsigned w = static_cast<unsigned>(x);
+  int pos = 0, c = __popc(w);
+  if (k >= c) {
+    k -= c;
+    w = static_cast<unsigned>(x >> 32);
+    pos = 32;
+  }
+#pragma unroll
+  for (int h = 16; h; h >>= 1) {
+    c = __popc(w & ((1u << h) - 1u));
+    if (k >= c) {
+      k -= c;
+      w >>= h;
+      pos += h;
+    }
+  }
+  return pos;
 }
 
 // spin-orbital index of electron e (up electrons first, then dn + n)

@@ -57,6 +57,39 @@ __device__ __forceinline__ void pair_masks(uint32_t pr, uint64_t u, uint64_t d, 
   *rd = b;
 }
 
+// The electrons of one det over a warp's lanes: lane e holds the orbital of electron e (alpha
+// electrons first), so that a pair's masks are two shuffles.  More than 32 electrons: every lane
+// looks its pair up in the strings.  Core keys of 1.2 million dets of 20 electrons: 0.70 ms; 1.7
+// with two bit searches a pair.
+struct LaneElecs {
+  uint64_t u, d;
+  int n_up;
+  bool wide;
+  int orb;  // of electron `lane`; beta orbitals + 64
+  __device__ __forceinline__ LaneElecs(uint64_t u_, uint64_t d_, int n_up_, int ne)
+      : u(u_), d(d_), n_up(n_up_), wide(ne > 32), orb(0) {
+    const int e = threadIdx.x & 31;
+    if (!wide && e < ne) orb = e < n_up ? nth_bit(u, e) : nth_bit(d, e - n_up) + 64;
+  }
+  // Masks of pair pr (all lanes call; lanes without a pair pass any valid one).
+  __device__ __forceinline__ void masks(uint32_t pr, uint64_t* ru, uint64_t* rd) const {
+    if (wide) {
+      pair_masks(pr, u, d, n_up, ru, rd);
+      return;
+    }
+    const int a = __shfl_sync(kFull, orb, pr & 0xffffu), b = __shfl_sync(kFull, orb, pr >> 16);
+    const uint64_t x = 1ull << (a & 63), y = 1ull << (b & 63);
+    *ru = (a < 64 ? x : 0ull) | (b < 64 ? y : 0ull);
+    *rd = (a < 64 ? 0ull : x) | (b < 64 ? 0ull : y);
+  }
+};
+
+__global__ void k_pack_dets(const uint64_t* __restrict__ up, const uint64_t* __restrict__ dn,
+                            uint32_t n, ulonglong2* __restrict__ out) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    out[i] = make_ulonglong2(up[i], dn[i]);
+}
+
 // Entries in det order: key = top `bits` bits of the core hash, value = entry index.
 template <class KT>
 __global__ void k_core_keys(const uint64_t* __restrict__ up, const uint64_t* __restrict__ dn,
@@ -71,9 +104,12 @@ __global__ void k_core_keys(const uint64_t* __restrict__ up, const uint64_t* __r
       if (lane == 0) atomicOr(err, (unsigned)kDevCheck);
       continue;
     }
-    for (uint32_t k = lane; k < K; k += 32) {
+    const LaneElecs el(u, d, n_up, n_up + n_dn);
+    for (uint32_t k0 = 0; k0 < K; k0 += 32) {
+      const uint32_t k = k0 + lane;
       uint64_t ru, rd;
-      pair_masks(pairs[k], u, d, n_up, &ru, &rd);
+      el.masks(pairs[min(k, K - 1u)], &ru, &rd);
+      if (k >= K) continue;
       const size_t t = (size_t)i * K + k;
       keys[t] = static_cast<KT>(core_hash(u & ~ru, d & ~rd) >> (64 - bits));
       vals[t] = static_cast<uint32_t>(t);
@@ -124,7 +160,8 @@ namespace {
 
 struct JoinView {
   uint32_t K;
-  int n_up;
+  int n_up, n_elecs;
+  const ulonglong2* dets;  // (up, dn): one 16-byte read a candidate
   const uint32_t* pairs;
   const uint64_t* span;
   const uint32_t* jdet;
@@ -152,13 +189,14 @@ __device__ __forceinline__ uint32_t member_start(const uint32_t* __restrict__ jd
 // Row kernel of the join (MODE as in RowSink).  A warp per row: lanes take the row's entries
 // 32 at a time, the members after each entry are flattened over the lanes, and every member
 // that passes the canonical-core test goes to the row's queues.
-// Five CTAs per SM (48 registers, a few spilled): 144 ms for the n = 40 fill against 151 ms
-// at the register-limited four (64 registers) and 156 ms at six (40 registers).
+// Bound by the integer pipe (population counts, compares and shuffles per candidate).  1.2 million
+// dets of n = 40 (1.86 G candidates, 1.25 G elements): 25.6 ms; 27.6 with every pair's masks by
+// bit searches in the strings and a candidate's two strings from two arrays.  Five CTAs per SM
+// (48 registers): 25.6 ms, four (64 registers): 27.1, six (40 registers): 25.8.
 template <int MODE>
 __global__ void __launch_bounds__(kJoinWarps * 32, 5)
-    k_hjoin(DevIntegrals I, const uint64_t* __restrict__ up, const uint64_t* __restrict__ dn,
-            uint32_t n, JoinView jv, uint32_t* row_cnt, const uint64_t* row_ptr, uint32_t* col,
-            double* v64, float* v32, float* r32, unsigned* work, float* absacc) {
+    k_hjoin(DevIntegrals I, uint32_t n, JoinView jv, uint32_t* row_cnt, const uint64_t* row_ptr,
+            uint32_t* col, double* v64, float* v32, float* r32, unsigned* work, float* absacc) {
   __shared__ RowQueues qs[kJoinWarps];
   RowQueues& q = qs[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31;
@@ -168,19 +206,21 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 5)
     if (lane == 0) i = atomicAdd(work, 1u);
     i = __shfl_sync(kFull, i, 0);
     if (i >= n) break;
-    const uint64_t ui = up[i], di = dn[i];
+    const ulonglong2 det_i = __ldg(jv.dets + i);
+    const uint64_t ui = det_i.x, di = det_i.y;
+    const LaneElecs el(ui, di, jv.n_up, jv.n_elecs);
     RowSink<MODE> sink(q, I, ui, di, MODE ? row_ptr[i] : 0, col, v64, v32, r32);
     if (absacc) sink.track_abs(absacc, i);
     uint64_t n_cand = 0;
     for (uint32_t k0 = 0; k0 < K; k0 += 32) {
       const uint32_t k = k0 + lane;
       uint32_t p = 0, len = 0;
-      uint64_t ru = 0, rd = 0;
+      uint64_t ru, rd;
+      el.masks(jv.pairs[min(k, K - 1u)], &ru, &rd);
       if (k < K) {
         const uint64_t sp = jv.span[(size_t)i * K + k];
         p = member_start(jv.jdet, sp, i, jv.n_prev);
         len = static_cast<uint32_t>(sp >> 32) - p - 1u;
-        pair_masks(jv.pairs[k], ui, di, jv.n_up, &ru, &rd);
       }
       const uint32_t inc = warp_inclusive_u32(len);
       const uint32_t total = __shfl_sync(kFull, inc, 31);
@@ -203,8 +243,9 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 5)
           // the first; take j once
           const bool repeat = pos > o_p + 1u && jv.jdet[pos - 1u] == j;
           if (!repeat) {
-            uj = up[j];
-            dj = dn[j];
+            const ulonglong2 det_j = __ldg(jv.dets + j);
+            uj = det_j.x;
+            dj = det_j.y;
             const uint64_t xu = ui ^ uj, xd = di ^ dj;
             const int x2 = popc64(xu) + popc64(xd);
             const uint64_t iu = ui & xu, id = di & xd;  // electrons of i absent from j
@@ -334,9 +375,13 @@ bool join_prepare(shci_ctx* c) {
   if (static_cast<double>(m) * 26.0 > 0.85 * static_cast<double>(avail)) return false;
   J.K = static_cast<uint32_t>(K);
   J.n_up = n_up;
-  J.n_dn = n_dn;
+  J.n_elecs = ne;
   J.m = m;
   try {
+    J.dets.resize(n);
+    k_pack_dets<<<grid_for(n, 256), 256, 0, s>>>(c->d_up.p, c->d_dn.p, static_cast<uint32_t>(n),
+                                                 J.dets.p);
+    SHCI_LAUNCH_CHECK();
     std::vector<uint32_t> pr;
     pr.reserve(K);
     for (int r1 = 0; r1 < ne; r1++)
@@ -362,18 +407,19 @@ void join_rows(shci_ctx* c, int mode, uint32_t* row_cnt, const uint64_t* row_ptr
                unsigned grid, float* absacc, uint32_t n_prev) {
   const auto& J = c->join;
   const uint32_t n = static_cast<uint32_t>(c->up.size());
-  JoinView v{J.K, J.n_up, J.pairs.p, J.span.p, J.jdet.p, n_prev};
+  if (!J.dets.p || !J.span.p || J.dets.n != n) throw std::logic_error("join rows without an index");
+  JoinView v{J.K, J.n_up, J.n_elecs, J.dets.p, J.pairs.p, J.span.p, J.jdet.p, n_prev};
   cudaStream_t s = c->stream;
   if (mode == 0)
-    k_hjoin<0><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, c->d_up.p, c->d_dn.p, n, v, row_cnt,
+    k_hjoin<0><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt,
                                                  nullptr, nullptr, nullptr, nullptr, nullptr,
                                                  work, absacc);
   else if (mode == 1)
-    k_hjoin<1><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, c->d_up.p, c->d_dn.p, n, v, row_cnt,
+    k_hjoin<1><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt,
                                                  row_ptr, col, v64, nullptr, nullptr, work,
                                                  absacc);
   else
-    k_hjoin<2><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, c->d_up.p, c->d_dn.p, n, v, row_cnt,
+    k_hjoin<2><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt,
                                                  row_ptr, col, nullptr, v32, r32, work,
                                                  absacc);
   SHCI_LAUNCH_CHECK();
@@ -402,6 +448,7 @@ void join_release(shci_ctx* c) {
   J.bstart.release();
   J.jdet.release();
   J.span.release();
+  J.dets.release();
   J.m = 0;
 }
 
