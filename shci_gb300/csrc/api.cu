@@ -168,7 +168,6 @@ shci_status shci_create(shci_ctx** out, int device, size_t hbm_budget_bytes) {
     c->join.pairs.mt = c->join.jdet.mt = &c->mem;
     c->join.dets.mt = &c->mem;
     c->join.keys.mt = c->join.span.mt = c->join.keys32.mt = &c->mem;
-    c->join.scan.mt = c->join.bstart.mt = &c->mem;
     auto& H = c->H;
     H.row_ptr.mt = H.col.mt = H.row_cnt.mt = &c->mem;
     H.val64.mt = H.diag.mt = &c->mem;

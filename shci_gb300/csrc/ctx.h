@@ -46,8 +46,6 @@ struct JoinIndex {
   int bits = 0, key_bytes = 0;  // hash bits kept; key width used by the last index
   DevBuf<uint64_t> keys;        // [m] core hashes (sort keys; released after bucketing)
   DevBuf<uint32_t> keys32;      //     the same when at most 32 hash bits are kept
-  DevBuf<uint32_t> scan;        // [m] bucket index of each sorted position (while bucketing)
-  DevBuf<uint32_t> bstart;      // [buckets + 1] bucket start positions (while bucketing)
   DevBuf<uint32_t> jdet;        // [m] det id of each sorted entry
   DevBuf<uint64_t> span;        // [m] per entry (in det order): sorted position | bucket end << 32
 };
