@@ -35,6 +35,8 @@ namespace shci {
 namespace {
 
 constexpr int kJoinWarps = 8;
+constexpr int kPlaceStretch = 1024;
+constexpr size_t kSplitEntries = 16u << 20;  // 128 MB of spans
 
 __device__ __forceinline__ uint64_t core_hash(uint64_t cu, uint64_t cd) {
   uint64_t h = cu * 0x9E3779B97F4A7C15ull ^ (cd + 0x632BE59BD9B4E019ull) * 0xC2B2AE3D27D4EB4Full;
@@ -141,15 +143,16 @@ __device__ __forceinline__ uint32_t warp_run_end(const KT* __restrict__ keys, KT
   }
 }
 
-// After the sort every position p of a bucket of equal keys writes span[entry] = p | end << 32 and
-// jdet[p] = det id (over the entry index).  A warp per 32 positions: a bucket that ends among them
-// ends at the next lane whose successor differs; only the one that runs on is searched for.
-// Bound by the scattered 8-byte writes of the spans.  228 million entries: 9.3 ms, and 11.4 with
-// flags of the bucket starts, their scan and an array of starts (five launches and a wait more:
-// 0.05 against 0.25 ms over the six builds of an n = 16 variation).
-template <class KT>
-__global__ void k_bucket_spans(const KT* __restrict__ keys, uint32_t* vals, uint32_t m, uint32_t K,
-                               uint64_t* span) {
+// After the sort every position p of a bucket of equal keys makes a span p | end << 32 and the det
+// id of its entry.  A warp per 32 positions: a bucket that ends among them ends at the next lane
+// whose successor differs; only the one that runs on is searched for.  ENTRY: the span goes to its
+// entry's place, else to position p (jdet and ents apart).
+// To entries, this is bound by the scattered 8-byte writes: 228 million entries 9.3 ms, and 11.4
+// with flags of the bucket starts, their scan and an array of starts (five launches and a wait
+// more: 0.05 against 0.25 ms over the six builds of an n = 16 variation).
+template <class KT, bool ENTRY>
+__global__ void k_bucket_spans(const KT* __restrict__ keys, const uint32_t* ents, uint32_t m,
+                               uint32_t K, uint64_t* span, uint32_t* jdet) {
   const unsigned lane = threadIdx.x & 31;
   const uint32_t n_tiles = m / 32u + (m % 32u != 0u);
   for (uint32_t tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile < n_tiles;
@@ -163,11 +166,32 @@ __global__ void k_bucket_spans(const KT* __restrict__ keys, uint32_t* vals, uint
     const unsigned mine = lasts >> lane;
     if (mine) end = static_cast<uint32_t>(p) + __ffs(mine);
     if (p < m) {
-      const uint32_t v = vals[p];
-      span[v] = p | (static_cast<uint64_t>(end) << 32);
-      vals[p] = v / K;
+      const uint32_t v = ents[p];
+      span[ENTRY ? v : p] = p | (static_cast<uint64_t>(end) << 32);
+      jdet[p] = v / K;
     }
   }
+}
+
+// out[ents[p]] = span[p], the entries split by their leading bits: the writes of a while fall in a
+// window that L2 holds, so that a sector goes to memory once and whole.  A block per stretch of
+// positions, in order (a grid that strides over the array writes to every window at once: 8.6 ms
+// against 1.7 at 228 million entries).
+__global__ void __launch_bounds__(256)
+    k_place_spans(const uint32_t* __restrict__ ents, const uint64_t* __restrict__ span, uint32_t m,
+                  uint64_t* __restrict__ out) {
+  const uint64_t p0 = (uint64_t)blockIdx.x * kPlaceStretch + threadIdx.x;
+  uint32_t e[kPlaceStretch / 256];
+  uint64_t v[kPlaceStretch / 256];
+#pragma unroll
+  for (int k = 0; k < kPlaceStretch / 256; k++) {
+    const uint64_t p = p0 + k * 256;
+    e[k] = p < m ? ents[p] : 0u;
+    v[k] = p < m ? span[p] : 0u;
+  }
+#pragma unroll
+  for (int k = 0; k < kPlaceStretch / 256; k++)
+    if (p0 + k * 256 < m) out[e[k]] = v[k];
 }
 
 }  // namespace
@@ -321,7 +345,8 @@ void sort_keys(DevBuf<uint64_t>& k, DevBuf<uint32_t>& v, size_t m, int bits, shc
 
 // Entries -> sorted buckets -> spans; keys of type KT hold `bits` hash bits.
 template <class KT>
-void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int n_dn) {
+void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int n_dn,
+                bool split) {
   auto& J = c->join;
   cudaStream_t s = c->stream;
   const size_t m = J.m;
@@ -349,9 +374,33 @@ void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int
   J.span.resize(m);
   {
     ProfScope ps(c->prof, s, "join_buckets");
-    k_bucket_spans<KT><<<grid_for(m, 256), 256, 0, s>>>(keys.p, J.jdet.p, static_cast<uint32_t>(m),
-                                                        J.K, J.span.p);
-    SHCI_LAUNCH_CHECK();
+    const uint32_t m32 = static_cast<uint32_t>(m);
+    if (!split) {
+      k_bucket_spans<KT, true><<<grid_for(m, 256), 256, 0, s>>>(keys.p, J.jdet.p, m32, J.K,
+                                                                J.span.p, J.jdet.p);
+      SHCI_LAUNCH_CHECK();
+    } else {
+      DevBuf<uint32_t> ents;
+      ents.mt = &c->mem;
+      ents.swap(J.jdet);
+      J.jdet.mt = &c->mem;
+      J.jdet.resize(m);
+      k_bucket_spans<KT, false><<<grid_for(m, 256), 256, 0, s>>>(keys.p, ents.p, m32, J.K,
+                                                                 J.span.p, J.jdet.p);
+      SHCI_LAUNCH_CHECK();
+      keys.release();
+      int top = 0;  // bits of an entry index
+      while (top < 32 && (m32 - 1u) >> top) top++;
+      radix_sort_pairs32_64(ents, J.span, m, std::max(0, top - 8), top, s, c->sort, false);
+      c->sort.valt64.resize(m);
+      k_place_spans<<<static_cast<unsigned>((m + kPlaceStretch - 1) / kPlaceStretch), 256, 0, s>>>(
+          ents.p, J.span.p, m32, c->sort.valt64.p);
+      SHCI_LAUNCH_CHECK();
+      swap_storage(J.span, c->sort.valt64);
+      c->launches += 6;
+      SHCI_CUDA(cudaStreamSynchronize(s));
+      release_sort_pingpong(c);
+    }
   }
   SHCI_CUDA(cudaStreamSynchronize(s));
   keys.release();
@@ -399,8 +448,15 @@ bool join_prepare(shci_ctx* c) {
     // SHCI_JOIN_BITS (4..40) narrows it, so tests can force colliding buckets.
     int bits = m <= (1ull << 30) ? 32 : 40;
     if (const char* e = std::getenv("SHCI_JOIN_BITS")) bits = std::min(40, std::max(4, std::atoi(e)));
-    if (bits <= 32) join_index(c, J.keys32, bits, n, n_up, n_dn);
-    else join_index(c, J.keys, bits, n, n_up, n_dn);
+    // Spans by way of their entries' leading bits where they outgrow L2 and the storage of that
+    // (34 bytes an entry) is there.  Straight against by leading bits: 9.5 million entries 0.14
+    // against 0.21 ms, 17 million 0.43 against 0.35, 76 million 2.9 against 1.4, 228 million 9.3
+    // against 4.3.  SHCI_JOIN_SPLIT=0 or 1 takes the one or the other at any size.
+    const double want = static_cast<double>(m) * 34.0;
+    bool split = m > kSplitEntries && want < 0.85 * static_cast<double>(avail);
+    if (const char* e = std::getenv("SHCI_JOIN_SPLIT")) split = std::atoi(e) != 0;
+    if (bits <= 32) join_index(c, J.keys32, bits, n, n_up, n_dn, split);
+    else join_index(c, J.keys, bits, n, n_up, n_dn, split);
   } catch (const OomError&) {
     join_release(c);
     release_sort_pingpong(c);

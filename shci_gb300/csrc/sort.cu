@@ -381,6 +381,13 @@ void radix_sort_pairs32(DevBuf<uint32_t>& keys, DevBuf<uint32_t>& vals, size_t n
                                       sc.valt32, skip);
 }
 
+void radix_sort_pairs32_64(DevBuf<uint32_t>& keys, DevBuf<uint64_t>& vals, size_t n,
+                           int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc,
+                           bool skip) {
+  radix_sort_impl<uint32_t, uint64_t>(keys, vals, n, begin_bit, end_bit, s, sc, sc.kalt32,
+                                      sc.valt64, skip);
+}
+
 void iota_u32(uint32_t* v, size_t n, cudaStream_t s) {
   k_iota<<<grid_for(n, 256), 256, 0, s>>>(v, n);
   SHCI_LAUNCH_CHECK();

@@ -47,6 +47,9 @@ void radix_sort_pairs64(DevBuf<uint64_t>& keys, DevBuf<uint64_t>& vals, size_t n
 void radix_sort_pairs32(DevBuf<uint32_t>& keys, DevBuf<uint32_t>& vals, size_t n,
                         int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc,
                         bool skip = true);
+void radix_sort_pairs32_64(DevBuf<uint32_t>& keys, DevBuf<uint64_t>& vals, size_t n,
+                           int begin_bit, int end_bit, cudaStream_t s, SortScratch& sc,
+                           bool skip = true);
 
 template <class T>
 inline void swap_storage(DevBuf<T>& a, DevBuf<T>& b) {

@@ -1,5 +1,6 @@
-"""Ends of the core join's buckets (runs of equal hash bits): runs inside a group of 32 positions,
-runs of thousands of positions and one run of all entries give the same matrix."""
+"""Ends of the core join's buckets (runs of equal hash bits): runs inside a group of 32 positions
+and runs of hundreds of positions, the spans written straight to their entries or by way of the
+entries' leading bits, give the same matrix."""
 import numpy as np
 import pytest
 
@@ -21,8 +22,9 @@ def test_bucket_lengths(monkeypatch, count):
     dn = np.array([sum(1 << int(o) for o in b) for _, b in occ], dtype=np.uint64)
     got = []
     for env in ({}, {"SHCI_JOIN_BITS": "4"}, {"SHCI_JOIN_BITS": "9"}, {"SHCI_JOIN_BITS": "40"},
-                {"SHCI_HBUILD": "scan"}):
-        for k in ("SHCI_HBUILD", "SHCI_JOIN_BITS"):
+                {"SHCI_JOIN_SPLIT": "1"}, {"SHCI_JOIN_SPLIT": "1", "SHCI_JOIN_BITS": "4"},
+                {"SHCI_JOIN_SPLIT": "1", "SHCI_JOIN_BITS": "40"}, {"SHCI_HBUILD": "scan"}):
+        for k in ("SHCI_HBUILD", "SHCI_JOIN_BITS", "SHCI_JOIN_SPLIT"):
             monkeypatch.delenv(k, raising=False)
         for k, v in env.items():
             monkeypatch.setenv(k, v)
