@@ -102,10 +102,7 @@ __global__ void k_core_keys(const uint64_t* __restrict__ up, const uint64_t* __r
   const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t i = warp0; i < n; i += n_warps) {
     const uint64_t u = up[i], d = dn[i];
-    if (popc64(u) != n_up || popc64(d) != n_dn) {
-      if (lane == 0) atomicOr(err, (unsigned)kDevCheck);
-      continue;
-    }
+    if ((popc64(u) != n_up || popc64(d) != n_dn) && lane == 0) atomicOr(err, (unsigned)kDevCheck);
     const LaneElecs el(u, d, n_up, n_up + n_dn);
     for (uint32_t k0 = 0; k0 < K; k0 += 32) {
       const uint32_t k = k0 + lane;
@@ -337,10 +334,10 @@ void release_sort_pingpong(shci_ctx* c) {
 }
 
 void sort_keys(DevBuf<uint32_t>& k, DevBuf<uint32_t>& v, size_t m, int bits, shci_ctx* c) {
-  radix_sort_pairs32(k, v, m, 0, bits, c->stream, c->sort);
+  radix_sort_pairs32(k, v, m, 0, bits, c->stream, c->sort, false);
 }
 void sort_keys(DevBuf<uint64_t>& k, DevBuf<uint32_t>& v, size_t m, int bits, shci_ctx* c) {
-  radix_sort_pairs(k, v, m, 0, bits, c->stream, c->sort);
+  radix_sort_pairs(k, v, m, 0, bits, c->stream, c->sort, false);
 }
 
 // Entries -> sorted buckets -> spans; keys of type KT hold `bits` hash bits.
@@ -361,10 +358,6 @@ void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int
         keys.p, J.jdet.p, c->err_word.p);
     SHCI_LAUNCH_CHECK();
   }
-  unsigned err = 0;
-  SHCI_CUDA(cudaMemcpyAsync(&err, c->err_word.p, 4, cudaMemcpyDeviceToHost, s));
-  SHCI_CUDA(cudaStreamSynchronize(s));
-  if (err) throw ArgError("dets do not all have the electron counts of the first det");
   {
     ProfScope ps(c->prof, s, "join_sort");
     sort_keys(keys, J.jdet, m, bits, c);
@@ -402,8 +395,11 @@ void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int
       release_sort_pingpong(c);
     }
   }
+  unsigned err = 0;
+  SHCI_CUDA(cudaMemcpyAsync(&err, c->err_word.p, 4, cudaMemcpyDeviceToHost, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
   keys.release();
+  if (err) throw ArgError("dets do not all have the electron counts of the first det");
   J.key_bytes = sizeof(KT);
   J.bits = bits;
   c->launches += 7;

@@ -74,8 +74,7 @@ __global__ void k_tile_scan(const T* in, T* out, size_t n, const T* offsets, T* 
     acc += items[k];
   }
   T tot;
-  T pre = block_exclusive(acc, &tot);
-  if (offsets) pre += offsets[blockIdx.x];
+  T pre = block_exclusive(acc, &tot) + offsets[blockIdx.x];
 #pragma unroll
   for (int k = 0; k < kScanItems; k++) {
     if (base + k < n) {
@@ -86,14 +85,66 @@ __global__ void k_tile_scan(const T* in, T* out, size_t n, const T* offsets, T* 
   }
 }
 
+// Up to kOneChunks * 4,096 values by one block: a thread holds four consecutive values of every
+// chunk of 4,096, all loaded before the first is used.  A scan of this size is bound by latency:
+// one launch of about 4 us for three of 3 us each (and the gaps between them).
+constexpr int kOneThreads = 1024;
+constexpr int kOneChunks = 4;
+constexpr size_t kOneMax = (size_t)kOneThreads * 4 * kOneChunks;
+
+template <class T>
+__global__ void __launch_bounds__(kOneThreads)
+    k_scan_one(const T* in, T* out, unsigned n, T* total_dev) {
+  __shared__ T s_w[kOneChunks * 32];  // sums of the warps of each chunk, then the sums before them
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  T v[kOneChunks][4], before[kOneChunks];
+#pragma unroll
+  for (int c = 0; c < kOneChunks; c++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned t = (c * kOneThreads + threadIdx.x) * 4 + k;
+      v[c][k] = t < n ? in[t] : T(0);
+    }
+#pragma unroll
+  for (int c = 0; c < kOneChunks; c++) {
+    const T sum = v[c][0] + v[c][1] + v[c][2] + v[c][3];
+    const T inc = warp_inclusive(sum);
+    before[c] = inc - sum;
+    if (lane == 31) s_w[c * 32 + warp] = inc;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    T run = 0;
+#pragma unroll
+    for (int c = 0; c < kOneChunks; c++) {
+      const T w = s_w[c * 32 + lane];
+      const T inc = warp_inclusive(w);
+      s_w[c * 32 + lane] = run + inc - w;
+      run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0 && total_dev) *total_dev = run;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < kOneChunks; c++) {
+    T run = s_w[c * 32 + warp] + before[c];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned t = (c * kOneThreads + threadIdx.x) * 4 + k;
+      if (t < n) out[t] = run;
+      run += v[c][k];
+    }
+  }
+}
+
 template <class T>
 void scan_rec(const T* in, T* out, size_t n, cudaStream_t s, T* part, T* total_dev) {
-  const size_t nb = (n + kScanTile - 1) / kScanTile;
-  if (nb <= 1) {
-    k_tile_scan<T><<<1, kScanThreads, 0, s>>>(in, out, n, nullptr, total_dev);
+  if (n <= kOneMax) {
+    k_scan_one<T><<<1, kOneThreads, 0, s>>>(in, out, static_cast<unsigned>(n), total_dev);
     SHCI_LAUNCH_CHECK();
     return;
   }
+  const size_t nb = (n + kScanTile - 1) / kScanTile;
   k_tile_sums<T><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, part);
   SHCI_LAUNCH_CHECK();
   scan_rec<T>(part, part, nb, s, part + nb, nullptr);
