@@ -167,6 +167,7 @@ shci_status shci_create(shci_ctx** out, int device, size_t hbm_budget_bytes) {
     for (auto* b : {&ix.am_dn, &ix.ad_dn, &ix.bd_up, &ix.ua, &ix.ub, &ix.bs_str}) b->mt = &c->mem;
     c->join.pairs.mt = c->join.jdet.mt = &c->mem;
     c->join.dets.mt = &c->mem;
+    c->join.lists.mt = c->join.units.mt = c->join.long_rows.mt = c->join.unit_cnt.mt = &c->mem;
     c->join.keys.mt = c->join.span.mt = c->join.keys32.mt = &c->mem;
     auto& H = c->H;
     H.row_ptr.mt = H.col.mt = H.row_cnt.mt = &c->mem;

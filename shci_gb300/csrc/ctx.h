@@ -42,6 +42,10 @@ struct JoinIndex {
   int n_up = 0, n_elecs = 0;
   size_t m = 0;                 // n * K entries
   DevBuf<ulonglong2> dets;      // [n] (up, dn)
+  DevBuf<uint32_t> lists;       // parts of long rows, long rows; candidates of the longest
+  DevBuf<uint2> units;          // (row, part)
+  DevBuf<uint2> long_rows;      // (row, its first unit)
+  DevBuf<uint32_t> unit_cnt;    // elements a part kept
   DevBuf<uint32_t> pairs;       // [K] electron ranks r1 | r2 << 16 (r1 < r2)
   int bits = 0, key_bytes = 0;  // hash bits kept; key width used by the last index
   DevBuf<uint64_t> keys;        // [m] core hashes (sort keys; released after bucketing)

@@ -595,14 +595,15 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
   uint64_t nnz = 0;
   bool one_pass = false;
   if (H.join && !two_pass) {
-    const uint64_t cap = join_row_caps(c, H.row_ptr.p, static_cast<uint32_t>(n_prev));
+    const JoinCaps caps = join_row_caps(c, H.row_ptr.p, static_cast<uint32_t>(n_prev));
+    const uint64_t cap = caps.total;
     one_pass = static_cast<double>(cap) * 12.0 * 1.1 < 0.9 * static_cast<double>(store_room(c));
     if (one_pass) {
       alloc_store(c, precision, cap);
       {
         ProfScope ps(c->prof, s, "hbuild_fill");
         join_rows(c, fill_mode, H.row_cnt.p, H.row_ptr.p, H.col.p, H.val64.p, H.val32.p,
-                  H.res32.p, work, grid, absacc, static_cast<uint32_t>(n_prev));
+                  H.res32.p, work, grid, absacc, static_cast<uint32_t>(n_prev), caps);
       }
       c->k0.resize(n, 1.25);
       widen_u32_u64(H.row_cnt.p, c->k0.p, n, s);
@@ -615,7 +616,7 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
       ProfScope ps(c->prof, s, "hbuild_count");
       if (H.join) {
         join_rows(c, 0, H.row_cnt.p, nullptr, nullptr, nullptr, nullptr, nullptr, work, grid,
-                  absacc, static_cast<uint32_t>(n_prev));
+                  absacc, static_cast<uint32_t>(n_prev), {});
       } else {
         k_hbuild<0><<<grid, kWarps * 32, 0, s>>>(c->dI, c->d_up.p, c->d_dn.p, (uint32_t)n, v,
                                                  H.row_cnt.p, nullptr, nullptr, nullptr,
@@ -648,7 +649,7 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
       ProfScope ps(c->prof, s, "hbuild_fill");
       if (H.join) {
         join_rows(c, fill_mode, nullptr, H.row_ptr.p, H.col.p, H.val64.p, H.val32.p, H.res32.p,
-                  work, grid, nullptr, static_cast<uint32_t>(n_prev));
+                  work, grid, nullptr, static_cast<uint32_t>(n_prev), {});
       } else if (precision == SHCI_PREC_FP64) {
         k_hbuild<1><<<grid, kWarps * 32, 0, s>>>(c->dI, c->d_up.p, c->d_dn.p, (uint32_t)n, v,
                                                  nullptr, H.row_ptr.p, H.col.p, H.val64.p,

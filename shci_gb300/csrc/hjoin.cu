@@ -34,8 +34,10 @@ namespace shci {
 
 namespace {
 
-constexpr int kJoinWarps = 8;
+constexpr int kJoinWarps = 8, kJoinCtas = 5;
 constexpr int kPlaceStretch = 1024;
+constexpr uint32_t kMinPart = 256;
+constexpr int kCloseThreads = 256, kClosePer = 4;
 constexpr size_t kSplitEntries = 16u << 20;  // 128 MB of spans
 
 __device__ __forceinline__ uint64_t core_hash(uint64_t cu, uint64_t cd) {
@@ -203,6 +205,10 @@ struct JoinView {
   const uint64_t* span;
   const uint32_t* jdet;
   uint32_t n_prev;  // incremental update: rows < n_prev take only members >= n_prev
+  uint32_t part;  // parts of long rows
+  const uint32_t* lists;
+  const uint2* units;
+  uint32_t* unit_cnt;
 };
 
 // Members of entry sp = (position p | bucket end << 32) of row i: positions (p', end) with
@@ -213,6 +219,7 @@ __device__ __forceinline__ uint32_t member_start(const uint32_t* __restrict__ jd
   uint32_t p = static_cast<uint32_t>(sp);
   if (i < n_prev) {
     uint32_t lo = p + 1u, hi = static_cast<uint32_t>(sp >> 32);
+    if (jdet[hi - 1u] < n_prev) return hi - 1u;  // (most buckets have no new member)
     while (lo < hi) {
       const uint32_t mid = (lo + hi) >> 1;
       if (jdet[mid] < n_prev) lo = mid + 1u;
@@ -223,33 +230,121 @@ __device__ __forceinline__ uint32_t member_start(const uint32_t* __restrict__ jd
   return p;
 }
 
-// Row kernel of the join (MODE as in RowSink).  A warp per row: lanes take the row's entries
-// 32 at a time, the members after each entry are flattened over the lanes, and every member
-// that passes the canonical-core test goes to the row's queues.
+// Rows of more than two parts of `part` candidates, cut into parts (in the order of the traversal)
+// that different warps take: units[slot + k] = (row, part k), lists[0] units and lists[1] rows in
+// all, rows[.] = (row, slot).  A part fills its own stretch of the row's storage, which holds one
+// place per candidate; k_close_rows closes the gaps.
+__global__ void k_long_rows(const uint64_t* __restrict__ row_ptr, uint32_t n, uint32_t part,
+                            uint32_t* lists, uint2* __restrict__ units, uint2* __restrict__ rows) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t cand = static_cast<uint32_t>(row_ptr[i + 1] - row_ptr[i]);
+    if (cand <= 2u * part) continue;
+    const uint32_t parts = (cand - 1u) / part + 1u;
+    const uint32_t slot = atomicAdd(&lists[0], parts);
+    rows[atomicAdd(&lists[1], 1u)] = make_uint2(i, slot);
+    for (uint32_t k = 0; k < parts; k++) units[slot + k] = make_uint2(i, k);
+  }
+}
+
+// A CTA per long row moves its parts together, a stretch (held in registers between two barriers)
+// after the other, and writes the row's length.
+template <int MODE>
+__global__ void __launch_bounds__(kCloseThreads)
+    k_close_rows(const uint64_t* __restrict__ row_ptr, uint32_t part,
+                 const uint32_t* __restrict__ lists, const uint2* __restrict__ rows,
+                 const uint32_t* __restrict__ unit_cnt, uint32_t* row_cnt, uint32_t* col,
+                 double* v64, float* v32, float* r32) {
+  __shared__ uint32_t s_cnt[kCloseThreads];
+  const uint32_t n_rows = lists[1];
+  for (uint32_t r = blockIdx.x; r < n_rows; r += gridDim.x) {
+    const uint32_t i = rows[r].x, slot = rows[r].y;
+    const uint64_t base = row_ptr[i];
+    const uint32_t cand = static_cast<uint32_t>(row_ptr[i + 1] - base);
+    const uint32_t parts = (cand - 1u) / part + 1u;
+    uint32_t len = 0;
+    for (uint32_t k = 0; k < parts; k++) {
+      if (k % kCloseThreads == 0) {
+        __syncthreads();
+        if (k + threadIdx.x < parts) s_cnt[threadIdx.x] = unit_cnt[slot + k + threadIdx.x];
+        __syncthreads();
+      }
+      const uint32_t c = s_cnt[k % kCloseThreads];
+      const uint64_t src = base + (uint64_t)k * part, dst = base + len;
+      len += c;
+      if (src == dst) continue;
+      for (uint32_t t0 = 0; t0 < c; t0 += kCloseThreads * kClosePer) {
+        uint32_t j[kClosePer];
+        double a[kClosePer];
+        float b[kClosePer], e[kClosePer];
+#pragma unroll
+        for (int x = 0; x < kClosePer; x++) {
+          const uint32_t t = t0 + threadIdx.x + x * kCloseThreads;
+          if (t >= c) continue;
+          j[x] = col[src + t];
+          if (MODE == 1) a[x] = v64[src + t];
+          if (MODE == 2) {
+            b[x] = v32[src + t];
+            e[x] = r32[src + t];
+          }
+        }
+        __syncthreads();  // (what the stores below write over has been read)
+#pragma unroll
+        for (int x = 0; x < kClosePer; x++) {
+          const uint32_t t = t0 + threadIdx.x + x * kCloseThreads;
+          if (t >= c) continue;
+          col[dst + t] = j[x];
+          if (MODE == 1) v64[dst + t] = a[x];
+          if (MODE == 2) {
+            v32[dst + t] = b[x];
+            r32[dst + t] = e[x];
+          }
+        }
+      }
+    }
+    if (threadIdx.x == 0) row_cnt[i] = len;
+  }
+}
+
+// Row kernel of the join (MODE as in RowSink).  A warp per row or, PARTS, part of a long row
+// (these first): lanes take the row's entries 32 at a time, the members after each entry are flattened over the
+// lanes, and every member that passes the canonical-core test goes to the row's queues.
 // Bound by the integer pipe (population counts, compares and shuffles per candidate).  1.2 million
 // dets of n = 40 (1.86 G candidates, 1.25 G elements): 25.6 ms; 27.6 with every pair's masks by
 // bit searches in the strings and a candidate's two strings from two arrays.  Five CTAs per SM
 // (48 registers): 25.6 ms, four (64 registers): 27.1, six (40 registers): 25.8.
-template <int MODE>
-__global__ void __launch_bounds__(kJoinWarps * 32, 5)
+template <int MODE, bool PARTS>
+__global__ void __launch_bounds__(kJoinWarps * 32, kJoinCtas)
     k_hjoin(DevIntegrals I, uint32_t n, JoinView jv, uint32_t* row_cnt, const uint64_t* row_ptr,
             uint32_t* col, double* v64, float* v32, float* r32, unsigned* work, float* absacc) {
   __shared__ RowQueues qs[kJoinWarps];
   RowQueues& q = qs[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31;
   const uint32_t K = jv.K;
+  const uint32_t n_units = PARTS ? jv.lists[0] : 0u;
   while (true) {
-    uint32_t i = 0;
-    if (lane == 0) i = atomicAdd(work, 1u);
-    i = __shfl_sync(kFull, i, 0);
-    if (i >= n) break;
+    uint32_t w = 0;
+    if (lane == 0) w = atomicAdd(work, 1u);
+    w = __shfl_sync(kFull, w, 0);
+    uint32_t i = w - n_units, t_lo = 0, t_hi = 0xffffffffu;  // the row's candidates [t_lo, t_hi)
+    uint64_t base = 0;
+    if (PARTS && w < n_units) {
+      const uint2 x = jv.units[w];
+      i = x.x;
+      t_lo = x.y * jv.part;
+      t_hi = t_lo + jv.part;
+      base = row_ptr[i] + t_lo;
+    } else {
+      if (i >= n) break;
+      if (MODE) base = row_ptr[i];
+      if (PARTS && row_ptr[i + 1] - base > 2u * jv.part) continue;
+    }
     const ulonglong2 det_i = __ldg(jv.dets + i);
     const uint64_t ui = det_i.x, di = det_i.y;
     const LaneElecs el(ui, di, jv.n_up, jv.n_elecs);
-    RowSink<MODE> sink(q, I, ui, di, MODE ? row_ptr[i] : 0, col, v64, v32, r32);
+    RowSink<MODE> sink(q, I, ui, di, base, col, v64, v32, r32);
     if (absacc) sink.track_abs(absacc, i);
-    uint64_t n_cand = 0;
-    for (uint32_t k0 = 0; k0 < K; k0 += 32) {
+    uint32_t n_cand = 0;  // up to the current entries
+    for (uint32_t k0 = 0; k0 < K && (!PARTS || n_cand < t_hi); k0 += 32) {
       const uint32_t k = k0 + lane;
       uint32_t p = 0, len = 0;
       uint64_t ru, rd;
@@ -261,8 +356,10 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 5)
       }
       const uint32_t inc = warp_inclusive_u32(len);
       const uint32_t total = __shfl_sync(kFull, inc, 31);
+      const uint32_t first = PARTS && t_lo > n_cand ? t_lo - n_cand : 0u;
+      const uint32_t end = PARTS ? min(total, t_hi - n_cand) : total;
       n_cand += total;
-      for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+      for (uint32_t t0 = first; t0 < end; t0 += 32) {
         const uint32_t t = t0 + lane;
         const uint32_t o = owner_lane(inc, t);
         const uint32_t o_inc = __shfl_sync(kFull, inc, o);
@@ -273,7 +370,7 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 5)
         bool cand = false, single = false;
         uint32_t j = 0;
         uint64_t uj = 0, dj = 0;
-        if (t < total) {
+        if (t < end) {
           const uint32_t pos = o_p + 1u + (t - (o_inc - o_len));
           j = jv.jdet[pos];
           // a second entry of j in this bucket (its two cores hashed alike) sits right after
@@ -302,8 +399,10 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 5)
     }
     const uint32_t cnt = sink.finish();
     if (lane == 0) {
-      if (row_cnt) row_cnt[i] = cnt;
-      atomicAdd(reinterpret_cast<unsigned long long*>(work + 2), (unsigned long long)n_cand);
+      if (PARTS && w < n_units) jv.unit_cnt[w] = cnt;
+      else if (row_cnt) row_cnt[i] = cnt;
+      atomicAdd(reinterpret_cast<unsigned long long*>(work + 2),
+                (unsigned long long)(PARTS ? min(n_cand, t_hi) - t_lo : n_cand));
     }
   }
 }
@@ -311,8 +410,10 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 5)
 // Row capacity of a single-pass build: the candidates of row i (members after each of its
 // entries), an upper bound on the elements it keeps.
 __global__ void k_join_caps(const uint64_t* __restrict__ span, const uint32_t* __restrict__ jdet,
-                            uint32_t n, uint32_t K, uint32_t n_prev, uint64_t* caps) {
+                            uint32_t n, uint32_t K, uint32_t n_prev, uint64_t* caps,
+                            uint32_t* longest) {
   const unsigned lane = threadIdx.x & 31;
+  uint32_t most = 0;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
     uint64_t c = 0;
@@ -323,7 +424,9 @@ __global__ void k_join_caps(const uint64_t* __restrict__ span, const uint32_t* _
 #pragma unroll
     for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
     if (lane == 0) caps[i] = c;
+    most = max(most, static_cast<uint32_t>(c));
   }
+  if (lane == 0) atomicMax(longest, most);
 }
 
 void release_sort_pingpong(shci_ctx* c) {
@@ -461,42 +564,99 @@ bool join_prepare(shci_ctx* c) {
   return true;
 }
 
-void join_rows(shci_ctx* c, int mode, uint32_t* row_cnt, const uint64_t* row_ptr,
-               uint32_t* col, double* v64, float* v32, float* r32, unsigned* work,
-               unsigned grid, float* absacc, uint32_t n_prev) {
-  const auto& J = c->join;
-  const uint32_t n = static_cast<uint32_t>(c->up.size());
-  if (!J.dets.p || !J.span.p || J.dets.n != n) throw std::logic_error("join rows without an index");
-  JoinView v{J.K, J.n_up, J.n_elecs, J.dets.p, J.pairs.p, J.span.p, J.jdet.p, n_prev};
+namespace {
+
+template <bool PARTS>
+void launch_hjoin(shci_ctx* c, int mode, uint32_t n, const JoinView& v, uint32_t* row_cnt,
+                  const uint64_t* row_ptr, uint32_t* col, double* v64, float* v32, float* r32,
+                  unsigned* work, unsigned grid, float* absacc) {
   cudaStream_t s = c->stream;
-  if (mode == 0)
-    k_hjoin<0><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt,
-                                                 nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                 work, absacc);
-  else if (mode == 1)
-    k_hjoin<1><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt,
-                                                 row_ptr, col, v64, nullptr, nullptr, work,
-                                                 absacc);
+  if (mode == 1)
+    k_hjoin<1, PARTS><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt, row_ptr, col, v64,
+                                                        nullptr, nullptr, work, absacc);
   else
-    k_hjoin<2><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt,
-                                                 row_ptr, col, nullptr, v32, r32, work,
-                                                 absacc);
+    k_hjoin<2, PARTS><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt, row_ptr, col, nullptr,
+                                                        v32, r32, work, absacc);
   SHCI_LAUNCH_CHECK();
   c->launches += 1;
 }
 
-uint64_t join_row_caps(shci_ctx* c, uint64_t* row_start, uint32_t n_prev) {
-  const auto& J = c->join;
+}  // namespace
+
+void join_rows(shci_ctx* c, int mode, uint32_t* row_cnt, const uint64_t* row_ptr,
+               uint32_t* col, double* v64, float* v32, float* r32, unsigned* work,
+               unsigned grid, float* absacc, uint32_t n_prev, const JoinCaps& caps) {
+  auto& J = c->join;
+  const uint32_t n = static_cast<uint32_t>(c->up.size());
+  if (!J.dets.p || !J.span.p || J.dets.n != n) throw std::logic_error("join rows without an index");
+  cudaStream_t s = c->stream;
+  JoinView v{J.K,      J.n_up, J.n_elecs, J.dets.p, J.pairs.p, J.span.p,
+             J.jdet.p, n_prev, 0,         nullptr,  nullptr,   nullptr};
+  if (mode == 0) {
+    k_hjoin<0, false><<<grid, kJoinWarps * 32, 0, s>>>(c->dI, n, v, row_cnt, nullptr, nullptr,
+                                                        nullptr, nullptr, nullptr, work, absacc);
+    SHCI_LAUNCH_CHECK();
+    c->launches += 1;
+    return;
+  }
+  // A warp takes about 75 ns a candidate however few others there are, so rows go to one warp each
+  // only while the longest is no longer than a resident warp's share of all candidates, else in
+  // parts of a quarter of that share.  30,000 dets of n = 40 (24 million candidates): 0.43 ms in
+  // parts, 1.69 by rows; 120,000 (134 million): 1.96 and 4.95, most of it the longest row's warp
+  // alone; 1.2 million (1.86 G): 26.1 in parts of 8,192, 25.5 by rows.  SHCI_JOIN_PART sets the
+  // candidates of a part (0: whole rows).
+  int dev_sms = 0;
+  SHCI_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device));
+  const uint64_t share = caps.total / (static_cast<uint64_t>(dev_sms) * kJoinWarps * kJoinCtas);
+  if (caps.longest > share)
+    v.part = static_cast<uint32_t>(std::max<uint64_t>(kMinPart, std::min<uint64_t>(share / 4, 1u << 30)));
+  if (const char* e = std::getenv("SHCI_JOIN_PART"))
+    v.part = caps.longest ? static_cast<uint32_t>(std::max(0, std::atoi(e))) : 0u;
+  if (v.part == 0 || caps.longest <= 2ull * v.part) {
+    launch_hjoin<false>(c, mode, n, v, row_cnt, row_ptr, col, v64, v32, r32, work, grid, absacc);
+    return;
+  }
+  // (a long row has more than two parts of the candidates, and at most one part that is not full)
+  const size_t long_max = std::min<size_t>(n, caps.total / (2ull * v.part));
+  J.long_rows.resize(long_max);
+  J.units.resize(caps.total / v.part + long_max);
+  J.unit_cnt.resize(J.units.n);
+  v.lists = J.lists.p;
+  v.units = J.units.p;
+  v.unit_cnt = J.unit_cnt.p;
+  SHCI_CUDA(cudaMemsetAsync(J.lists.p, 0, 2 * sizeof(uint32_t), s));
+  k_long_rows<<<grid_for(n, 256), 256, 0, s>>>(row_ptr, n, v.part, J.lists.p, J.units.p,
+                                               J.long_rows.p);
+  SHCI_LAUNCH_CHECK();
+  launch_hjoin<true>(c, mode, n, v, row_cnt, row_ptr, col, v64, v32, r32, work, grid, absacc);
+  if (mode == 1)
+    k_close_rows<1><<<grid, kCloseThreads, 0, s>>>(row_ptr, v.part, J.lists.p, J.long_rows.p,
+                                                   J.unit_cnt.p, row_cnt, col, v64, nullptr,
+                                                   nullptr);
+  else
+    k_close_rows<2><<<grid, kCloseThreads, 0, s>>>(row_ptr, v.part, J.lists.p, J.long_rows.p,
+                                                   J.unit_cnt.p, row_cnt, col, nullptr, v32, r32);
+  SHCI_LAUNCH_CHECK();
+  c->launches += 2;
+}
+
+JoinCaps join_row_caps(shci_ctx* c, uint64_t* row_start, uint32_t n_prev) {
+  auto& J = c->join;
   const uint32_t n = static_cast<uint32_t>(c->up.size());
   cudaStream_t s = c->stream;
+  J.lists.resize(3);
+  SHCI_CUDA(cudaMemsetAsync(J.lists.p + 2, 0, sizeof(uint32_t), s));
   k_join_caps<<<grid_for((size_t)n * 32, 256), 256, 0, s>>>(J.span.p, J.jdet.p, n, J.K, n_prev,
-                                                           row_start);
+                                                           row_start, J.lists.p + 2);
   SHCI_LAUNCH_CHECK();
-  const uint64_t tot = exclusive_scan_u64(row_start, row_start, n, s, c->sort);
-  SHCI_CUDA(cudaMemcpyAsync(row_start + n, &tot, 8, cudaMemcpyHostToDevice, s));
+  exclusive_scan_u64_async(row_start, row_start, n, s, c->sort, row_start + n);
+  uint64_t total = 0;
+  uint32_t longest = 0;
+  SHCI_CUDA(cudaMemcpyAsync(&total, row_start + n, 8, cudaMemcpyDeviceToHost, s));
+  SHCI_CUDA(cudaMemcpyAsync(&longest, J.lists.p + 2, 4, cudaMemcpyDeviceToHost, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
   c->launches += 1;
-  return tot;
+  return {total, longest};
 }
 
 void join_release(shci_ctx* c) {
@@ -506,6 +666,10 @@ void join_release(shci_ctx* c) {
   J.jdet.release();
   J.span.release();
   J.dets.release();
+  J.lists.release();
+  J.units.release();
+  J.long_rows.release();
+  J.unit_cnt.release();
   J.m = 0;
 }
 

@@ -43,14 +43,19 @@ size_t build_time_sym(shci_ctx* c, int precision);
 // cannot be used for the current dets; join_rows runs one pass (mode as the row kernels;
 // every mode writes each row's kept count to row_cnt when given).
 bool join_prepare(shci_ctx* c);
-// n_prev > 0 (incremental update): rows < n_prev take only columns >= n_prev.
+// Candidates of a single-pass build: all of them, and those of the row that has the most.
+struct JoinCaps {
+  uint64_t total = 0, longest = 0;
+};
+// n_prev > 0 (incremental update): rows < n_prev take only columns >= n_prev.  caps: of
+// join_row_caps where row_ptr holds its row starts (long rows are then cut over warps), else none.
 void join_rows(shci_ctx* c, int mode, uint32_t* row_cnt, const uint64_t* row_ptr,
                uint32_t* col, double* v64, float* v32, float* r32, unsigned* work,
-               unsigned grid, float* absacc, uint32_t n_prev);
+               unsigned grid, float* absacc, uint32_t n_prev, const JoinCaps& caps);
 void join_release(shci_ctx* c);
 // Row starts of a single-pass build: row_start[i] = sum of the candidate counts of rows < i
-// (row_start has n + 1 entries); returns the total capacity.
-uint64_t join_row_caps(shci_ctx* c, uint64_t* row_start, uint32_t n_prev);
+// (row_start has n + 1 entries).
+JoinCaps join_row_caps(shci_ctx* c, uint64_t* row_start, uint32_t n_prev);
 
 // rowsort.cu: sorts each row of the element store by column (tiles of 2048 elements), so
 // that H*v's scattered accesses share sectors; SHCI_ROW_SORT=0 turns the pass off.
