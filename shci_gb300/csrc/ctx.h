@@ -188,6 +188,7 @@ struct shci_ctx {
   // PT2 diagonals in 64-bit fixed point (pt2.cu): h_oo, J - K (same spin), J (opposite spin)
   shci::DevBuf<long long> dfix;
   int dfix_scale = 0;
+  unsigned long long dfix_ref = 0;  // the lowest filling in the same fixed point
   bool dfix_valid = false;
   // PT2 single-excitation elements in 64-bit fixed point (pt2.cu): h_pq, (pq|oo), (po|oq)
   shci::DevBuf<long long> sfix;
