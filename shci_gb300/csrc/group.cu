@@ -7,8 +7,8 @@
 // with one hash (about m^2 / 2^33 pairs of m) stay apart.  The sums are formed in an order that the
 // records fix.  An order by determinant is not needed (the contributions are summed afterwards, in a
 // compensated fixed order).  The sort by determinant that this replaces took a radix sort for each
-// string, ten passes over 12-byte items and a gather per array: 13.4 -> 8.4 ms over the three stages
-// of an n = 40 run (40,000 dets, 50M records in the first), 1.89 -> 1.28 ms at n = 26 (20M records).
+// string, ten passes over 12-byte items and a gather per array: 13.4 -> 7.6 ms over the three stages
+// of an n = 40 run (40,000 dets, 50M records in the first), 1.89 -> 1.20 ms at n = 26 (20M records).
 #include <algorithm>
 
 #include "group.cuh"
@@ -96,10 +96,11 @@ __global__ void __launch_bounds__(kGroupWarps * 32)
 // The sums, to out[pos[k / 32] + heads before k in its word] for every head k.  A warp per 32
 // records: a run of one determinant is summed by halving distances among its lanes; the run that
 // goes on behind the warp's records is followed by all lanes, and a determinant that shares its
-// key with others by its head's lane.  Bound by the FP64 pipe and
-// the latency of a warp's loads.  Over the stages of an n = 40 run (50M, 2 x 10M and 14M records):
-// 0.94 + 0.83 + 1.25 ms, against 1.04 + 1.11 + 1.40 for a thread per determinant, which waits in each
-// warp for the longest run of 32, and another 1.1 ms of passes for its list of heads.
+// key with others by its head's lane.  Bound by the FP64 pipe (a warp's addition takes 16 cycles
+// however few lanes need it), so no step is taken that no head needs.  Over the stages of an n = 40
+// run (50M, 2 x 10M and 14M records): 0.67 + 0.64 + 0.88 ms (0.94 + 0.83 + 1.25 when every run was
+// summed over five steps), against 1.04 + 1.11 + 1.40 for a thread per determinant, which waits in
+// each warp for the longest run of 32, and another 1.1 ms of passes for its list of heads.
 template <int NV>
 __global__ void __launch_bounds__(kGroupWarps * 32)
     k_group_sum(const uint32_t* __restrict__ key, const PtRec<NV>* __restrict__ rec,
@@ -121,9 +122,11 @@ __global__ void __launch_bounds__(kGroupWarps * 32)
     const unsigned runs = __ballot_sync(kFull, starts);
     const unsigned later = lane == 31 ? 0u : runs >> (lane + 1);
     const int end = later ? lane + __ffs(later) : 32;  // the lane behind this one's run
+    const int begin = 31 - __clz(runs & (0xffffffffu >> (31 - lane)));
+    const int stop = (heads >> begin) & 1u ? end : 0;  // (runs that began before are not summed here)
 #pragma unroll
     for (int h = 1; h < 32; h <<= 1) {
-      const bool take = lane + h < end;
+      const bool take = lane + h < stop;
       if (!__any_sync(kFull, take)) break;
 #pragma unroll
       for (int v = 0; v < NV; v++) {
@@ -137,9 +140,9 @@ __global__ void __launch_bounds__(kGroupWarps * 32)
     if ((heads >> last & 1u) && w * 32 + 32 < m) {  // the last run goes on?
       const uint32_t lx = __shfl_sync(kFull, x, last);
       const uint64_t lu = __shfl_sync(kFull, r.u, last), ld = __shfl_sync(kFull, r.d, last);
-      double acc[NV] = {};
+      double acc[NV];
       size_t p0 = w * 32 + 32;
-      int more;
+      int more, width = 0;  // lanes that hold a sum
       do {
         const size_t p = p0 + lane;
         const bool in = p < m && key[p] == lx && rec[p].u == lu && rec[p].d == ld;
@@ -147,16 +150,23 @@ __global__ void __launch_bounds__(kGroupWarps * 32)
         more = out_of ? __ffs(out_of) - 1 : 32;
         if (lane < more) {
 #pragma unroll
-          for (int v = 0; v < NV; v++) acc[v] += rec[p].v[v];
+          for (int v = 0; v < NV; v++) acc[v] = width ? acc[v] + rec[p].v[v] : rec[p].v[v];
         }
+        width = max(width, more);
         p0 += more;
       } while (more == 32);
-      if (p0 > w * 32 + 32) {
+      if (width) {
+        for (int h = 1; h < width; h <<= 1) {
+#pragma unroll
+          for (int v = 0; v < NV; v++) {
+            const double t = __shfl_down_sync(kFull, acc[v], h);
+            if (lane + h < width) acc[v] += t;
+          }
+        }
 #pragma unroll
         for (int v = 0; v < NV; v++) {
-#pragma unroll
-          for (int h = 16; h; h >>= 1) acc[v] += __shfl_xor_sync(kFull, acc[v], h);
-          if (lane == last) r.v[v] += acc[v];
+          const double t = __shfl_sync(kFull, acc[v], 0);
+          if (lane == last) r.v[v] += t;
         }
       }
       if (lane == last) q = p0;
@@ -172,7 +182,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32)
     }
 #pragma unroll
     for (int v = 0; v < NV; v++)
-      if (r.v[v] == 0.0) r.v[v] = 0.0;  // (no -0)
+      if (static_cast<uint64_t>(__double_as_longlong(r.v[v])) == 1ull << 63) r.v[v] = 0.0;
     out[at + __popc(heads & ((1u << lane) - 1u))] = r;
   }
 }
