@@ -42,7 +42,7 @@ struct JoinIndex {
   int n_up = 0, n_elecs = 0;
   size_t m = 0;                 // n * K entries
   DevBuf<ulonglong2> dets;      // [n] (up, dn)
-  DevBuf<uint32_t> lists;       // parts of long rows, long rows; candidates of the longest
+  DevBuf<uint32_t> lists;       // parts of long rows, long rows; most candidates of a row; error; total
   DevBuf<uint2> units;          // (row, part)
   DevBuf<uint2> long_rows;      // (row, its first unit)
   DevBuf<uint32_t> unit_cnt;    // elements a part kept

@@ -94,6 +94,13 @@ __global__ void k_axpy_dev(double* __restrict__ v, const double* __restrict__ u,
     v[i] -= a * u[i];
 }
 
+__global__ void k_normalize(double* __restrict__ v, const double* __restrict__ norm2, size_t n) {
+  const double s = sqrt(*norm2);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x)
+    v[i] = v[i] / s;
+}
+
 __global__ void k_scale(double* __restrict__ v, double s, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
@@ -349,8 +356,8 @@ DavidsonOut davidson(shci_ctx* c, double tol) {
   D.Hw.resize(n, 1.1);
   // v0 = init / |init|
   SHCI_CUDA(cudaMemcpyAsync(D.v[0].p, c->d_coef.p, n * 8, cudaMemcpyDeviceToDevice, s));
-  double nrm = std::sqrt(dots.dot_host(D.v[0].p, D.v[0].p, n));
-  k_scale<<<g, 256, 0, s>>>(D.v[0].p, nrm, n);
+  dots.mdot(D.v[0].p, {D.v[0].p}, n, D.scal.p);
+  k_normalize<<<g, 256, 0, s>>>(D.v[0].p, D.scal.p, n);
   SHCI_LAUNCH_CHECK();
   spmv(c, D.v[0].p, D.Hv[0].p, false);
   out.n_matvec++;

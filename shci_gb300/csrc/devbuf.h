@@ -161,7 +161,8 @@ struct DevBuf {
     reserve(k, slack);
     n = k;
   }
-  // Grows capacity keeping the first n elements.
+  // Grows capacity keeping the first n elements (the old block is released behind the copy on the
+  // context's one stream).
   void grow_keep(size_t k, cudaStream_t s, double slack = 1.5) {
     if (k <= cap) {
       n = k;
@@ -171,7 +172,6 @@ struct DevBuf {
     nb.mt = mt;
     nb.reserve(k, slack);
     if (n) SHCI_CUDA(cudaMemcpyAsync(nb.p, p, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
-    SHCI_CUDA(cudaStreamSynchronize(s));
     std::swap(p, nb.p);
     std::swap(cap, nb.cap);
     nb.n = 0;

@@ -514,6 +514,7 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
   H.bound_valid = false;
   H.join = !scan_only && join_prepare(c);
   if (!H.join) n_prev = 0;  // the group scan builds whole matrices only
+  else if (two_pass) join_check(c);
   if (n_prev) {
     // keep the current store as an older segment
     auto seg = std::make_unique<HSeg>();
@@ -547,8 +548,9 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
   H.row_ptr.resize(n + 1, 1.25);
   H.row_cnt.resize(n + 1, 1.25);
   H.diag.resize(n, 1.25);
-  // err_word layout: [0] row work counter, [1] unused, [2..7] three u64 candidate counters
-  c->err_word.resize(8);
+  // err_word layout: [0] row work counter, [1] unused, [2..7] three u64 candidate counters, [8..9]
+  // the elements of a single-pass build
+  c->err_word.resize(10);
   IndexView v{ix.det_aid.p, ix.det_bid.p, ix.a_start.p, ix.b_start.p, ix.am_idx.p,
               ix.ad_idx.p,  ix.bd_idx.p,  ix.am_dn.p,   ix.ad_dn.p,   ix.bd_up.p,
               ix.ua.p,      ix.as_off.p,  ix.as_list.p, ix.bs_off.p,  ix.bs_str.p};
@@ -607,7 +609,8 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
       }
       c->k0.resize(n, 1.25);
       widen_u32_u64(H.row_cnt.p, c->k0.p, n, s);
-      nnz = exclusive_scan_u64(c->k0.p, c->k0.p, n, s, c->sort);
+      exclusive_scan_u64_async(c->k0.p, c->k0.p, n, s, c->sort,
+                               reinterpret_cast<uint64_t*>(work + 8));
       H.packed = false;
     }
   }
@@ -629,9 +632,10 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
     nnz = exclusive_scan_u64(H.row_ptr.p, H.row_ptr.p, n, s, c->sort);
     SHCI_CUDA(cudaMemcpyAsync(H.row_ptr.p + n, &nnz, 8, cudaMemcpyHostToDevice, s));
   }
-  unsigned long long cand[3] = {0, 0, 0};
-  SHCI_CUDA(cudaMemcpyAsync(cand, work + 2, 24, cudaMemcpyDeviceToHost, s));
+  unsigned long long cand[4] = {0, 0, 0, 0};
+  SHCI_CUDA(cudaMemcpyAsync(cand, work + 2, sizeof(cand), cudaMemcpyDeviceToHost, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
+  if (one_pass) nnz = cand[3];
   if (absacc || hb_bound) finish_mixed_bound(c);
   H.nnz_current = nnz;
   H.nnz = nnz;
@@ -662,8 +666,8 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
       SHCI_LAUNCH_CHECK();
     }
     H.packed = true;
+    SHCI_CUDA(cudaStreamSynchronize(s));
   }
-  SHCI_CUDA(cudaStreamSynchronize(s));
   if (H.join) join_release(c);
   if (row_sort_enabled()) sort_rows(c);
   build_items(c);

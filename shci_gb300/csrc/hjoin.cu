@@ -36,6 +36,7 @@ namespace {
 
 constexpr int kJoinWarps = 8, kJoinCtas = 5;
 constexpr int kPlaceStretch = 1024;
+constexpr const char* kBadCounts = "dets do not all have the electron counts of the first det";
 constexpr uint32_t kMinPart = 256;
 constexpr int kCloseThreads = 256, kClosePer = 4;
 constexpr size_t kSplitEntries = 16u << 20;  // 128 MB of spans
@@ -452,13 +453,11 @@ void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int
   const size_t m = J.m;
   keys.resize(m);
   J.jdet.resize(m);
-  c->err_word.resize(8);
   {
     ProfScope ps(c->prof, s, "join_keys");
-    SHCI_CUDA(cudaMemsetAsync(c->err_word.p, 0, 4, s));
     k_core_keys<KT><<<grid_for(n * 32, 256), 256, 0, s>>>(
         c->d_up.p, c->d_dn.p, static_cast<uint32_t>(n), J.pairs.p, J.K, n_up, n_dn, bits,
-        keys.p, J.jdet.p, c->err_word.p);
+        keys.p, J.jdet.p, J.lists.p + 3);
     SHCI_LAUNCH_CHECK();
   }
   {
@@ -494,15 +493,10 @@ void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int
       SHCI_LAUNCH_CHECK();
       swap_storage(J.span, c->sort.valt64);
       c->launches += 6;
-      SHCI_CUDA(cudaStreamSynchronize(s));
       release_sort_pingpong(c);
     }
   }
-  unsigned err = 0;
-  SHCI_CUDA(cudaMemcpyAsync(&err, c->err_word.p, 4, cudaMemcpyDeviceToHost, s));
-  SHCI_CUDA(cudaStreamSynchronize(s));
   keys.release();
-  if (err) throw ArgError("dets do not all have the electron counts of the first det");
   J.key_bytes = sizeof(KT);
   J.bits = bits;
   c->launches += 7;
@@ -533,6 +527,8 @@ bool join_prepare(shci_ctx* c) {
   J.n_elecs = ne;
   J.m = m;
   try {
+    J.lists.resize(6);
+    SHCI_CUDA(cudaMemsetAsync(J.lists.p, 0, 6 * sizeof(uint32_t), s));
     J.dets.resize(n);
     k_pack_dets<<<grid_for(n, 256), 256, 0, s>>>(c->d_up.p, c->d_dn.p, static_cast<uint32_t>(n),
                                                  J.dets.p);
@@ -644,19 +640,25 @@ JoinCaps join_row_caps(shci_ctx* c, uint64_t* row_start, uint32_t n_prev) {
   auto& J = c->join;
   const uint32_t n = static_cast<uint32_t>(c->up.size());
   cudaStream_t s = c->stream;
-  J.lists.resize(3);
-  SHCI_CUDA(cudaMemsetAsync(J.lists.p + 2, 0, sizeof(uint32_t), s));
   k_join_caps<<<grid_for((size_t)n * 32, 256), 256, 0, s>>>(J.span.p, J.jdet.p, n, J.K, n_prev,
                                                            row_start, J.lists.p + 2);
   SHCI_LAUNCH_CHECK();
-  exclusive_scan_u64_async(row_start, row_start, n, s, c->sort, row_start + n);
-  uint64_t total = 0;
-  uint32_t longest = 0;
-  SHCI_CUDA(cudaMemcpyAsync(&total, row_start + n, 8, cudaMemcpyDeviceToHost, s));
-  SHCI_CUDA(cudaMemcpyAsync(&longest, J.lists.p + 2, 4, cudaMemcpyDeviceToHost, s));
+  uint64_t* total = reinterpret_cast<uint64_t*>(J.lists.p + 4);
+  exclusive_scan_u64_async(row_start, row_start, n, s, c->sort, total);
+  SHCI_CUDA(cudaMemcpyAsync(row_start + n, total, 8, cudaMemcpyDeviceToDevice, s));
+  uint32_t h[4];  // one wait: most candidates of a row, error, total
+  SHCI_CUDA(cudaMemcpyAsync(h, J.lists.p + 2, sizeof(h), cudaMemcpyDeviceToHost, s));
   SHCI_CUDA(cudaStreamSynchronize(s));
   c->launches += 1;
-  return {total, longest};
+  if (h[1]) throw ArgError(kBadCounts);
+  return {h[2] | static_cast<uint64_t>(h[3]) << 32, h[0]};
+}
+
+void join_check(shci_ctx* c) {
+  uint32_t err = 0;
+  SHCI_CUDA(cudaMemcpyAsync(&err, c->join.lists.p + 3, 4, cudaMemcpyDeviceToHost, c->stream));
+  SHCI_CUDA(cudaStreamSynchronize(c->stream));
+  if (err) throw ArgError(kBadCounts);
 }
 
 void join_release(shci_ctx* c) {

@@ -53,6 +53,9 @@ void join_rows(shci_ctx* c, int mode, uint32_t* row_cnt, const uint64_t* row_ptr
                uint32_t* col, double* v64, float* v32, float* r32, unsigned* work,
                unsigned grid, float* absacc, uint32_t n_prev, const JoinCaps& caps);
 void join_release(shci_ctx* c);
+// Throws if join_prepare's pass met a det of other electron counts (join_row_caps does so too, with
+// the wait that it has anyway).
+void join_check(shci_ctx* c);
 // Row starts of a single-pass build: row_start[i] = sum of the candidate counts of rows < i
 // (row_start has n + 1 entries).
 JoinCaps join_row_caps(shci_ctx* c, uint64_t* row_start, uint32_t n_prev);
@@ -106,6 +109,10 @@ void jacobi_eig(int k, const double* lower, int ld, double* evals, double* evecs
 // select.cu
 size_t select_dets(shci_ctx* c, double eps_var, bool var_sd);
 void rebuild_det_set(shci_ctx* c, bool allow_dup = false);
+// The same in two halves: the set, and its check with a wait that the caller has anyway.  The first
+// half returns a device word that is not 0 when the list contains duplicates.
+const unsigned* build_det_set(shci_ctx* c);
+void check_det_set(unsigned flag);
 size_t sort_unique_pairs(shci_ctx* c, DevBuf<uint64_t>& a, DevBuf<uint64_t>& b, size_t m,
                          int a_bits = 0);
 void compact_valid(shci_ctx* c, const uint64_t* a, const uint64_t* b, size_t m,

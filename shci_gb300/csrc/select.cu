@@ -417,7 +417,7 @@ __global__ void k_hash_insert(const uint64_t* __restrict__ up, const uint64_t* _
 // of two >= 2n slots.  allow_dup: the set holds one of each group of equal dets instead of refusing
 // the list.  (The set used to come with a sorted copy of the list that only the duplicate check
 // read: two radix sorts per call.)
-void rebuild_det_set(shci_ctx* c, bool allow_dup) {
+const unsigned* build_det_set(shci_ctx* c) {
   const size_t n = c->up.size();
   cudaStream_t s = c->stream;
   c->err_word.resize(8);
@@ -432,11 +432,20 @@ void rebuild_det_set(shci_ctx* c, bool allow_dup) {
   k_hash_insert<<<grid_for(n, 256), 256, 0, s>>>(c->d_up.p, c->d_dn.p, n, c->set_hash.p,
                                                  c->set_hash_mask, dup);
   SHCI_LAUNCH_CHECK();
-  unsigned bad = 0;
-  SHCI_CUDA(cudaMemcpyAsync(&bad, dup, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-  SHCI_CUDA(cudaStreamSynchronize(s));
   c->launches += 1;
-  if (bad && !allow_dup) throw ArgError("the det list contains duplicates");
+  return dup;
+}
+
+void check_det_set(unsigned flag) {
+  if (flag) throw ArgError("the det list contains duplicates");
+}
+
+void rebuild_det_set(shci_ctx* c, bool allow_dup) {
+  const unsigned* dup = build_det_set(c);
+  unsigned flag = 0;
+  SHCI_CUDA(cudaMemcpyAsync(&flag, dup, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  SHCI_CUDA(cudaStreamSynchronize(c->stream));
+  if (!allow_dup) check_det_set(flag);
 }
 
 namespace {
@@ -539,7 +548,7 @@ size_t select_dets(shci_ctx* c, double eps_var, bool var_sd) {
   d_pairs.resize(pairs.empty() ? 1 : pairs.size());
   if (!pairs.empty())
     SHCI_CUDA(cudaMemcpyAsync(d_pairs.p, pairs.data(), pairs.size() * 4, cudaMemcpyHostToDevice, s));
-  rebuild_det_set(c);
+  const unsigned* dup = build_det_set(c);
 
   SelParams P{};
   P.I = c->dI;
@@ -617,7 +626,7 @@ size_t select_dets(shci_ctx* c, double eps_var, bool var_sd) {
       P, n_src, cnt.p, epsm.p);
   SHCI_LAUNCH_CHECK();
   PieceList L(c);
-  make_pieces(c, cnt, n_src, 1, 0.0, 0.0, nullptr, L);
+  check_det_set(make_pieces(c, cnt, n_src, 1, 0.0, 0.0, nullptr, L, dup));
   Candidates C(c);
   const uint64_t kCap = 1ull << 27;  // window entries per launch, and candidates held before a sort
   uint64_t base = 0;

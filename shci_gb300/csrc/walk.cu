@@ -7,9 +7,36 @@ namespace shci {
 
 namespace {
 
-__global__ void k_piece_count(const uint64_t* __restrict__ entries, uint32_t n_src, uint32_t* np) {
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src; k += gridDim.x * blockDim.x)
-    np[k] = static_cast<uint32_t>((entries[k] + kPieceLen - 1) / kPieceLen);
+// Region of a piece of l entries of a source that stands for `mult` of them.
+__device__ __forceinline__ uint64_t piece_region(uint64_t l, uint64_t mult, uint64_t n_batches,
+                                                 double slack, double pad) {
+  uint64_t r = l * mult;
+  if (n_batches > 1) {
+    const double est = ceil(static_cast<double>(r) / static_cast<double>(n_batches) * slack + pad);
+    if (est < static_cast<double>(r)) r = est > 0.0 ? static_cast<uint64_t>(est) : 0ull;
+  }
+  return r;
+}
+
+// Pieces of every source; back[0] = the regions of all, back[2] = *flag.
+__global__ void k_piece_count(const uint64_t* __restrict__ entries, uint32_t n_src,
+                              uint64_t n_batches, double slack, double pad,
+                              const uint32_t* __restrict__ ent_off, uint32_t* __restrict__ np,
+                              const unsigned* __restrict__ flag,
+                              unsigned long long* __restrict__ back) {
+  unsigned long long sum = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) back[2] = flag ? *flag : 0u;
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src;
+       k += gridDim.x * blockDim.x) {
+    const uint64_t m = entries[k], whole = m / kPieceLen, rest = m % kPieceLen;
+    const uint64_t mult = ent_off ? ent_off[k + 1] - ent_off[k] : 1u;
+    np[k] = static_cast<uint32_t>(whole + (rest != 0));
+    sum += whole * piece_region(kPieceLen, mult, n_batches, slack, pad);
+    if (rest) sum += piece_region(rest, mult, n_batches, slack, pad);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0 && sum) atomicAdd(back, sum);
 }
 
 // Region sizes go into off[p], to be scanned.
@@ -26,35 +53,42 @@ __global__ void k_piece_fill(const uint64_t* __restrict__ entries, const uint32_
     for (uint64_t b = 0; b < m; b += kPieceLen, p++) {
       const uint64_t l = min(static_cast<unsigned long long>(kPieceLen),
                              static_cast<unsigned long long>(m - b));
-      uint64_t r = l * mult;
-      if (n_batches > 1) {
-        const double est = ceil(static_cast<double>(r) / static_cast<double>(n_batches) * slack + pad);
-        if (est < static_cast<double>(r)) r = est > 0.0 ? static_cast<uint64_t>(est) : 0ull;
-      }
       src[p] = k;
       begin[p] = static_cast<uint32_t>(b);  // (a source's windows hold fewer than 2^32 entries)
       len[p] = static_cast<uint32_t>(l);
-      off[p] = r;
+      off[p] = piece_region(l, mult, n_batches, slack, pad);
     }
   }
 }
 
 }  // namespace
 
-void make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src, uint64_t n_batches,
-                 double slack, double pad, const uint32_t* ent_off, PieceList& L) {
+unsigned make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src,
+                     uint64_t n_batches, double slack, double pad, const uint32_t* ent_off,
+                     PieceList& L, const unsigned* flag) {
   cudaStream_t s = c->stream;
   L.n = 0;
   L.tot = 0;
-  if (n_src == 0) return;
+  if (n_src == 0) return 0;
   DevBuf<uint32_t> first;
   first.mt = &c->mem;
   first.resize(n_src);
-  k_piece_count<<<grid_for(n_src, 256), 256, 0, s>>>(entries.p, n_src, first.p);
+  DevBuf<unsigned long long> back;  // total of the regions, pieces, flag: one wait for all
+  back.mt = &c->mem;
+  back.resize(3);
+  SHCI_CUDA(cudaMemsetAsync(back.p, 0, 16, s));
+  k_piece_count<<<grid_for(n_src, 256), 256, 0, s>>>(
+      entries.p, n_src, n_batches, slack, pad, ent_off, first.p, flag, back.p);
   SHCI_LAUNCH_CHECK();
-  L.n = exclusive_scan_u32(first.p, first.p, n_src, s, c->sort);
+  exclusive_scan_u32_async(first.p, first.p, n_src, s, c->sort,
+                           reinterpret_cast<uint32_t*>(back.p + 1));
+  unsigned long long h[3];
+  SHCI_CUDA(cudaMemcpyAsync(h, back.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+  SHCI_CUDA(cudaStreamSynchronize(s));
+  L.tot = h[0];
+  L.n = static_cast<uint32_t>(h[1]);
   c->launches += 4;
-  if (L.n == 0) return;
+  if (L.n == 0) return static_cast<unsigned>(h[2]);
   L.src.resize(L.n);
   L.begin.resize(L.n);
   L.len.resize(L.n);
@@ -64,8 +98,7 @@ void make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src, u
                                                     L.off.p);
   SHCI_LAUNCH_CHECK();
   exclusive_scan_u64_async(L.off.p, L.off.p, L.n, s, c->sort, L.off.p + L.n);
-  SHCI_CUDA(cudaMemcpyAsync(&L.tot, L.off.p + L.n, 8, cudaMemcpyDeviceToHost, s));
-  SHCI_CUDA(cudaStreamSynchronize(s));
+  return static_cast<unsigned>(h[2]);
 }
 
 size_t piece_run(shci_ctx* c, const PieceList& L, size_t k0, uint64_t base, uint64_t cap,

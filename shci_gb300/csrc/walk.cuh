@@ -236,8 +236,10 @@ struct PieceList {
 // per entry of the source (ent_off: a det walked once for several entries), and len / n_batches *
 // slack + pad exceeds its mean by many standard deviations (pieces that overflow are emitted
 // again).
-void make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src, uint64_t n_batches,
-                 double slack, double pad, const uint32_t* ent_off, PieceList& L);
+// flag: a device word whose value is returned (read with the wait for the pieces' number).
+unsigned make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_src,
+                     uint64_t n_batches, double slack, double pad, const uint32_t* ent_off,
+                     PieceList& L, const unsigned* flag = nullptr);
 
 // walk.cu: the end of the run of pieces from k0 whose regions together hold at most `cap` (one piece
 // at least); base = off[k0], *end = off[result].
