@@ -24,20 +24,30 @@ namespace {
 constexpr int kDotBlocks = 304;
 constexpr int kDotThreads = 256;
 
-__device__ __forceinline__ double block_sum(double v) {
-  __shared__ double s[kDotThreads / 32];
+// dst[k * stride] = sum of acc[k] over the block, k < m <= M: the sums' shuffles side by side, then a
+// warp a sum.
+template <int M>
+__device__ __forceinline__ void block_sums(double (&acc)[M], int m, double* __restrict__ dst,
+                                           int stride) {
+  constexpr int kWarps = kDotThreads / 32;
+  static_assert(M <= kWarps, "a warp a sum");
+  __shared__ double s[M][kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  for (int o = 16; o; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < M; k++)
+      if (k < m) acc[k] += __shfl_xor_sync(kFull, acc[k], o);
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < M; k++) s[k][warp] = acc[k];
   __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x < 32) {
-    t = threadIdx.x < kDotThreads / 32 ? s[threadIdx.x] : 0.0;
+  if (warp < m) {
+    double t = lane < kWarps ? s[warp][lane] : 0.0;
 #pragma unroll
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+    for (int o = kWarps / 2; o; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+    if (lane == 0) dst[warp * stride] = t;
   }
-  __syncthreads();
-  return t;
 }
 
 struct Ptrs6 {
@@ -46,29 +56,28 @@ struct Ptrs6 {
 
 // Ends a reduction over the grid: every block leaves its m partial sums, and the block that arrives
 // last adds them up in block order into out[0, m) (so the result does not depend on timing) and
-// resets the counter.  A second launch for that sum cost as much as the sum itself.
-__device__ __forceinline__ void grid_sums(const double* acc, int m, double* __restrict__ partial,
+// resets the counter.  A second launch for that sum cost as much as the sum itself.  Bound by the
+// latency of its chains of shuffles and FP64 additions at the vector lengths of small systems: five
+// dots of 14,000 elements 11 us, 15 with one sum after the other.
+template <int M>
+__device__ __forceinline__ void grid_sums(double (&acc)[M], int m, double* __restrict__ partial,
                                           unsigned* __restrict__ counter,
                                           double* __restrict__ out) {
   __shared__ bool last;
-  for (int k = 0; k < m; k++) {
-    const double t = block_sum(acc[k]);
-    if (threadIdx.x == 0) partial[k * kDotBlocks + blockIdx.x] = t;
-  }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(counter, 1u) + 1u == gridDim.x;
-  }
+  block_sums(acc, m, partial + blockIdx.x, kDotBlocks);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) + 1u == gridDim.x;
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int k = 0; k < m; k++) {
-    double v = 0.0;
-    for (int b = threadIdx.x; b < static_cast<int>(gridDim.x); b += blockDim.x)
-      v += __ldcg(partial + k * kDotBlocks + b);
-    const double t = block_sum(v);
-    if (threadIdx.x == 0) out[k] = t;
-  }
+#pragma unroll
+  for (int k = 0; k < M; k++) acc[k] = 0.0;
+  for (int b = threadIdx.x; b < static_cast<int>(gridDim.x); b += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < M; k++)
+      if (k < m) acc[k] += __ldcg(partial + k * kDotBlocks + b);
+  block_sums(acc, m, out, 1);
   if (threadIdx.x == 0) *counter = 0u;
 }
 
@@ -80,7 +89,9 @@ __global__ void __launch_bounds__(kDotThreads)
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const double xi = x[i];
-    for (int k = 0; k < m; k++) acc[k] += ys.p[k] ? xi * ys.p[k][i] : xi;
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+      if (k < m) acc[k] += ys.p[k] ? xi * ys.p[k][i] : xi;
   }
   grid_sums(acc, m, partial, counter, out);
 }
@@ -173,7 +184,7 @@ __global__ void __launch_bounds__(kDotThreads)
                    unsigned* __restrict__ counter, double* __restrict__ out,
                    double* __restrict__ xmax) {
   if (xmax && blockIdx.x == 0 && threadIdx.x == 0) *xmax = 0.0;
-  double acc = 0.0;
+  double acc[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     double a, b;
@@ -192,9 +203,9 @@ __global__ void __launch_bounds__(kDotThreads)
     const double d = lambda - diag[i];
     const double x = fabs(d) < 1.0e-8 ? 0.0 : (b - lambda * a) / d;
     v[i] = x;
-    acc += x * (next ? next[i] : x);
+    acc[0] += x * (next ? next[i] : x);
   }
-  grid_sums(&acc, 1, partial, counter, out);
+  grid_sums(acc, 1, partial, counter, out);
 }
 
 // v -= (*coef) * u; out[0] = <v, next> (next null: <v, v>)
@@ -204,14 +215,14 @@ __global__ void __launch_bounds__(kDotThreads)
                double* __restrict__ partial, unsigned* __restrict__ counter,
                double* __restrict__ out) {
   const double a = *coef;
-  double acc = 0.0;
+  double acc[1] = {0.0};
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
     const double x = v[i] - a * u[i];
     v[i] = x;
-    acc += x * (next ? next[i] : x);
+    acc[0] += x * (next ? next[i] : x);
   }
-  grid_sums(&acc, 1, partial, counter, out);
+  grid_sums(acc, 1, partial, counter, out);
 }
 
 // The mixed product's end (spmv.cu, k_fix_out) and its dots: hv = yfix * 2^-s + diag * v, out[k] =
@@ -227,7 +238,9 @@ __global__ void __launch_bounds__(kDotThreads)
        i += (size_t)gridDim.x * blockDim.x) {
     const double x = static_cast<double>(static_cast<long long>(yfix[i])) * inv + diag[i] * v[i];
     hv[i] = x;
-    for (int k = 0; k < m; k++) acc[k] += x * ys.p[k][i];
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+      if (k < m) acc[k] += x * ys.p[k][i];
   }
   grid_sums(acc, m, partial, counter, out);
 }
