@@ -336,8 +336,15 @@ __global__ void __launch_bounds__(kJoinWarps * 32, kJoinCtas)
       base = row_ptr[i] + t_lo;
     } else {
       if (i >= n) break;
-      if (MODE) base = row_ptr[i];
-      if (PARTS && row_ptr[i + 1] - base > 2u * jv.part) continue;
+      if (MODE) {
+        base = row_ptr[i];
+        const uint64_t places = row_ptr[i + 1] - base;
+        if (PARTS && places > 2u * jv.part) continue;
+        if (places == 0) {  // most older rows of an incremental update
+          if (row_cnt && lane == 0) row_cnt[i] = 0;
+          continue;
+        }
+      }
     }
     const ulonglong2 det_i = __ldg(jv.dets + i);
     const uint64_t ui = det_i.x, di = det_i.y;
@@ -348,8 +355,6 @@ __global__ void __launch_bounds__(kJoinWarps * 32, kJoinCtas)
     for (uint32_t k0 = 0; k0 < K && (!PARTS || n_cand < t_hi); k0 += 32) {
       const uint32_t k = k0 + lane;
       uint32_t p = 0, len = 0;
-      uint64_t ru, rd;
-      el.masks(jv.pairs[min(k, K - 1u)], &ru, &rd);
       if (k < K) {
         const uint64_t sp = jv.span[(size_t)i * K + k];
         p = member_start(jv.jdet, sp, i, jv.n_prev);
@@ -357,6 +362,9 @@ __global__ void __launch_bounds__(kJoinWarps * 32, kJoinCtas)
       }
       const uint32_t inc = warp_inclusive_u32(len);
       const uint32_t total = __shfl_sync(kFull, inc, 31);
+      if (total == 0) continue;
+      uint64_t ru, rd;
+      el.masks(jv.pairs[min(k, K - 1u)], &ru, &rd);
       const uint32_t first = PARTS && t_lo > n_cand ? t_lo - n_cand : 0u;
       const uint32_t end = PARTS ? min(total, t_hi - n_cand) : total;
       n_cand += total;
@@ -427,7 +435,7 @@ __global__ void k_join_caps(const uint64_t* __restrict__ span, const uint32_t* _
     if (lane == 0) caps[i] = c;
     most = max(most, static_cast<uint32_t>(c));
   }
-  if (lane == 0) atomicMax(longest, most);
+  if (lane == 0 && most > __ldcg(longest)) atomicMax(longest, most);  // (rarely after the first)
 }
 
 void release_sort_pingpong(shci_ctx* c) {
@@ -596,15 +604,15 @@ void join_rows(shci_ctx* c, int mode, uint32_t* row_cnt, const uint64_t* row_ptr
     return;
   }
   // A warp takes about 75 ns a candidate however few others there are, so rows go to one warp each
-  // only while the longest is no longer than a resident warp's share of all candidates, else in
-  // parts of a quarter of that share.  30,000 dets of n = 40 (24 million candidates): 0.43 ms in
+  // only while the longest is no longer than half a resident warp's share of all candidates, else
+  // in parts of a quarter of that share.  30,000 dets of n = 40 (24 million candidates): 0.43 ms in
   // parts, 1.69 by rows; 120,000 (134 million): 1.96 and 4.95, most of it the longest row's warp
   // alone; 1.2 million (1.86 G): 26.1 in parts of 8,192, 25.5 by rows.  SHCI_JOIN_PART sets the
   // candidates of a part (0: whole rows).
   int dev_sms = 0;
   SHCI_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device));
   const uint64_t share = caps.total / (static_cast<uint64_t>(dev_sms) * kJoinWarps * kJoinCtas);
-  if (caps.longest > share)
+  if (2 * caps.longest > share)
     v.part = static_cast<uint32_t>(std::max<uint64_t>(kMinPart, std::min<uint64_t>(share / 4, 1u << 30)));
   if (const char* e = std::getenv("SHCI_JOIN_PART"))
     v.part = caps.longest ? static_cast<uint32_t>(std::max(0, std::atoi(e))) : 0u;
