@@ -227,6 +227,32 @@ __host__ __device__ __forceinline__ uint64_t rehash(uint64_t a) {
   h += (h << 15);
   return h;
 }
+// The low 7 bits of rehash(det_hash(up, dn)), with 32-bit words where the bits above cannot reach
+// them: a right shift by k takes k bits off those that are known, additions and left shifts none
+// (half_hash 32 bits, det_hash 30, then 24, 18 and 7 in rehash, whose last step starts at bit 15).
+constexpr uint64_t kLowBatches = 128;
+__host__ __device__ __forceinline__ uint32_t half_hash_low(uint64_t c0) {
+  uint64_t h = c0;
+  h += (h << 10);
+  h ^= (h >> 6);
+  h += (h << 10);
+  h ^= (h >> 6);
+  h += (h << 3);
+  const uint32_t l = static_cast<uint32_t>(h) ^ static_cast<uint32_t>(h >> 11);
+  return l + (l << 15);
+}
+__host__ __device__ __forceinline__ uint32_t batch_hash_low(uint64_t up, uint64_t dn) {
+  const uint32_t s = half_hash_low(up);
+  uint32_t h = s ^ (half_hash_low(dn) + 0x9e3779b9u + (s << 6) + (s >> 2));
+  h += (h << 10);
+  h ^= (h >> 6);
+  h += 982451653u;
+  h += (h << 10);
+  h ^= (h >> 6);
+  h += (h << 3);
+  h ^= (h >> 11);
+  return h & static_cast<uint32_t>(kLowBatches - 1);
+}
 
 // ---------------------------------------------------------------- compensated sums
 // Double-double accumulator: hi + lo carries the running sum with about 2^-106 relative

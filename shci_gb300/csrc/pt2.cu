@@ -50,6 +50,7 @@ struct PtParams {
   double eps_psto;   // sto: column split threshold
   uint64_t n_batches;
   uint64_t batch_magic;  // floor((2^64 - 1) / n_batches) for batch_of (set by set_batches)
+  uint32_t low_mask;     // n_batches - 1 where the low bits of the hash are enough, else 0
   uint64_t batch;    // dtm / psto: the batch being computed
   double factor;     // sto: 1 / (n_samples - n_dtm - 1)
   int iter_shift;    // sto: bit position of the iteration index in the emitted up key
@@ -96,6 +97,10 @@ __device__ __forceinline__ uint64_t batch_of(const PtParams& Q, uint64_t h) {
 void set_batches(PtParams& Q, uint64_t n_batches) {
   Q.n_batches = n_batches;
   Q.batch_magic = n_batches ? ~0ull / n_batches : 0;
+  // Powers of two up to kLowBatches need only the low bits of the hash (55 instructions for 85): a
+  // pseudo-stochastic batch of 16 at n = 40 5.3 -> 5.1 ms, six stochastic iterations 11.7 -> 11.4.
+  const bool low = n_batches > 1 && n_batches <= kLowBatches && (n_batches & (n_batches - 1)) == 0;
+  Q.low_mask = low ? static_cast<uint32_t>(n_batches - 1) : 0u;
 }
 
 // Window entries of each source: an upper bound of its candidates.
@@ -353,7 +358,9 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
         return;
       }
     }
-    const uint64_t b = act && Q.n_batches > 1 ? batch_of(Q, rehash(det_hash(cu, cd))) : 0ull;
+    uint64_t b = 0;
+    if (Q.low_mask) b = batch_hash_low(cu, cd) & Q.low_mask;
+    else if (Q.n_batches > 1) b = batch_of(Q, rehash(det_hash(cu, cd)));
     uint32_t e0 = 0, ne = act ? 1u : 0u;
     if (MODE == kSto && act) {
       e0 = ent_begin(S, kk);
