@@ -214,8 +214,8 @@ struct PtWarp {
 // against the source's strings and queues what passes; stage 2 builds 32 of those determinants and,
 // with several batches, hashes them and queues the members; the last stage evaluates 32 members.
 // Queues carry over from piece to piece.  Members keep their walk order within a piece.
-// At n = 40, 40,000 dets: 19.4 -> 4.6 ms deterministic (297M window entries), 11.3 -> 5.4 ms a
-// pseudo-stochastic batch of 16 (its hash is most of the work left), 21.4 -> 11.9 ms for six
+// At n = 40, 40,000 dets: 19.4 -> 4.6 ms deterministic (297M window entries), 11.3 -> 5.1 ms a
+// pseudo-stochastic batch of 16 (walk and hash are most of the work left), 21.4 -> 11.4 ms for six
 // stochastic iterations; n = 26, 30,000 dets: 5.3 -> 1.4 ms, of which the heaviest determinant's
 // window on one warp had been half.  (Before: build and hash at the walk, an output slot for
 // every window entry, a warp per source.)
