@@ -616,18 +616,23 @@ void join_rows(shci_ctx* c, int mode, uint32_t* row_cnt, const uint64_t* row_ptr
     v.part = static_cast<uint32_t>(std::max<uint64_t>(kMinPart, std::min<uint64_t>(share / 4, 1u << 30)));
   if (const char* e = std::getenv("SHCI_JOIN_PART"))
     v.part = caps.longest ? static_cast<uint32_t>(std::max(0, std::atoi(e))) : 0u;
-  if (v.part == 0 || caps.longest <= 2ull * v.part) {
+  // (a long row has more than two parts of the candidates, and at most one part that is not full)
+  if (v.part && caps.longest > 2ull * v.part) {
+    const size_t long_max = std::min<size_t>(n, caps.total / (2ull * v.part));
+    try {
+      J.long_rows.resize(long_max);
+      J.units.resize(caps.total / v.part + long_max);
+      J.unit_cnt.resize(J.units.n);
+      v.lists = J.lists.p;
+      v.units = J.units.p;
+      v.unit_cnt = J.unit_cnt.p;
+    } catch (const OomError&) {  // no room for the lists: whole rows
+    }
+  }
+  if (!v.lists) {
     launch_hjoin<false>(c, mode, n, v, row_cnt, row_ptr, col, v64, v32, r32, work, grid, absacc);
     return;
   }
-  // (a long row has more than two parts of the candidates, and at most one part that is not full)
-  const size_t long_max = std::min<size_t>(n, caps.total / (2ull * v.part));
-  J.long_rows.resize(long_max);
-  J.units.resize(caps.total / v.part + long_max);
-  J.unit_cnt.resize(J.units.n);
-  v.lists = J.lists.p;
-  v.units = J.units.p;
-  v.unit_cnt = J.unit_cnt.p;
   SHCI_CUDA(cudaMemsetAsync(J.lists.p, 0, 2 * sizeof(uint32_t), s));
   k_long_rows<<<grid_for(n, 256), 256, 0, s>>>(row_ptr, n, v.part, J.lists.p, J.units.p,
                                                J.long_rows.p);
