@@ -188,6 +188,7 @@ struct PtPieces {
   const uint32_t* len;
   const uint64_t* off;  // [n + 1]
   uint32_t* cnt;
+  uint32_t* work;  // pieces taken so far
   uint32_t n;
   uint64_t base;  // off of the output arrays' first entry
 };
@@ -214,9 +215,11 @@ struct PtWarp {
 // against the source's strings and queues what passes; stage 2 builds 32 of those determinants and,
 // with several batches, hashes them and queues the members; the last stage evaluates 32 members.
 // Queues carry over from piece to piece.  Members keep their walk order within a piece.
-// At n = 40, 40,000 dets: 19.4 -> 4.6 ms deterministic (297M window entries), 11.3 -> 5.1 ms a
-// pseudo-stochastic batch of 16 (walk and hash are most of the work left), 21.4 -> 11.4 ms for six
-// stochastic iterations; n = 26, 30,000 dets: 5.3 -> 1.4 ms, of which the heaviest determinant's
+// Warps take pieces from a counter, the next one while they walk (a fixed share left a tenth of the
+// chip idle: 26.3 -> 24.4 ms over the stages of an n = 40 run).
+// At n = 40, 40,000 dets: 19.4 -> 4.1 ms deterministic (297M window entries), 11.3 -> 4.8 ms a
+// pseudo-stochastic batch of 16 (walk and hash are most of the work left), 21.4 -> 10.6 ms for six
+// stochastic iterations; n = 26, 30,000 dets: 5.3 -> 1.3 ms, of which the heaviest determinant's
 // window on one warp had been half.  (Before: build and hash at the walk, an output slot for
 // every window entry, a warp per source.)
 template <int MODE>
@@ -227,7 +230,6 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
   PtWarp& W = reinterpret_cast<PtWarp*>(pt_smem)[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  const uint32_t wpg = gridDim.x * kPtWarps;
   uint32_t ah = 0, an = 0, bh = 0, bn = 0;           // warp-uniform ring states
   uint32_t run_piece = 0xffffffffu, run_cnt = 0;      // kept members of the last piece seen
 
@@ -393,7 +395,12 @@ __global__ void __launch_bounds__(kPtWarps * 32, 4)
     if (an >= 32u) drain_a(32u);
   };
 
-  for (uint32_t piece = blockIdx.x * kPtWarps + (threadIdx.x >> 5); piece < pc.n; piece += wpg) {
+  uint32_t next = 0;  // (lane 0) taken while the piece before is walked
+  if (lane == 0) next = atomicAdd(pc.work, 1u);
+  for (;;) {
+    const uint32_t piece = __shfl_sync(kFull, next, 0);
+    if (piece >= pc.n) break;
+    if (lane == 0) next = atomicAdd(pc.work, 1u);
     const uint32_t kk = pc.src[piece];
     const uint32_t skip = pc.begin[piece], left = pc.len[piece];
     const uint32_t i = src_det(S, kk, MODE);
@@ -831,14 +838,15 @@ void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSource
     const size_t k1 = piece_run(c, L, k0, base, kCap, &end);
     const uint64_t tot = end - base;
     const uint32_t n = static_cast<uint32_t>(k1 - k0);
-    d_cnt.resize((size_t)n + 1);  // (the overflow count after the pieces')
+    d_cnt.resize((size_t)n + 2);  // (the overflow count and the pieces taken after the pieces' counts)
     d_dst.resize((size_t)n + 1);
-    SHCI_CUDA(cudaMemsetAsync(d_cnt.p, 0, ((size_t)n + 1) * 4, s));
+    SHCI_CUDA(cudaMemsetAsync(d_cnt.p, 0, ((size_t)n + 2) * 4, s));
     out.resize(std::max<uint64_t>(tot, 1), 1.25);
-    const PtPieces pc{L.src.p + k0, L.begin.p + k0, L.len.p + k0, L.off.p + k0, d_cnt.p, n, base};
+    const PtPieces pc{L.src.p + k0, L.begin.p + k0, L.len.p + k0, L.off.p + k0, d_cnt.p,
+                      d_cnt.p + n + 1, n, base};
     {
       ProfScope ps(c->prof, s, "pt2_emit");
-      k_pt_emit<MODE><<<grid_for((size_t)n * 32, kPtWarps * 32, st.grid), kPtWarps * 32, smem, s>>>(
+      k_pt_emit<MODE><<<grid_for((size_t)n * 32, kPtWarps * 32, st.grid / 2), kPtWarps * 32, smem, s>>>(
           st.P, Q, S, F, pc, out.p);
       SHCI_LAUNCH_CHECK();
     }
