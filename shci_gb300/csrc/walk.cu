@@ -18,10 +18,10 @@ __device__ __forceinline__ uint64_t piece_region(uint64_t l, uint64_t mult, uint
   return r;
 }
 
-// Entries of a piece: two pieces a resident warp, within kPieceMin and kPieceLen.  (A piece costs a
+// Entries of a piece: eight pieces a resident warp, within kPieceMin and kPieceLen.  (A piece costs a
 // warp the search of its source's slots, about as long as a few hundred entries take.)
 __device__ __forceinline__ uint32_t piece_len(unsigned long long total, uint32_t warps) {
-  const unsigned long long len = total / (2ull * warps);
+  const unsigned long long len = total / (8ull * warps);
   return len <= kPieceMin ? kPieceMin : len >= kPieceLen ? kPieceLen : static_cast<uint32_t>(len);
 }
 

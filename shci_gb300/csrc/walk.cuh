@@ -12,10 +12,12 @@
 namespace shci {
 
 // Entries a warp walks at most before the next piece: the heaviest determinant's window holds
-// 100,000 entries, 3,000 rounds of one warp.  Where 4,096 entries a piece would leave warps without
-// one, pieces are shorter: the selections of an n = 16 variation took 0.43 ms in pieces of 4,096 and
-// take 0.20, those of an n = 26 variation 0.84 and 0.41.
-constexpr uint32_t kPieceLen = 4096, kPieceMin = 256;
+// 100,000 entries, 3,000 rounds of one warp, and a piece costs the search of its source's slots again.
+// Longer pieces where there are many entries: the PT2 emissions of an n = 40 run (297M entries and
+// more a stage) 24.3 ms with at most 4,096, 21.7 with 8,192, 20.8 with 16,384, 22.1 with 32,768 (30.3
+// with 2,048).  Shorter ones where warps would have none: the selections of an n = 16 variation took
+// 0.43 ms in pieces of 4,096 and take 0.20, those of an n = 26 variation 0.84 and 0.41.
+constexpr uint32_t kPieceLen = 16384, kPieceMin = 256;
 constexpr uint32_t kWalkWarps = 32;  // resident warps of a walk per SM
 constexpr uint32_t kWalkSlots = 256;  // slots listed at a time
 // Ranges of at least this many entries are walked slot by slot, the others flattened over the lanes:
