@@ -277,6 +277,7 @@ void sync_dets(shci_ctx* c) {
 void hamiltonian_elems(shci_ctx* c, const uint64_t* ui, const uint64_t* di, const uint64_t* uj,
                        const uint64_t* dj, size_t n, double* out) {
   if (n == 0) return;
+  if (!ui || !di || !uj || !dj || !out) throw ArgError("null pointer");
   cudaStream_t s = c->stream;
   DevBuf<double> o;
   o.mt = &c->mem;
