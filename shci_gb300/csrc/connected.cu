@@ -143,7 +143,14 @@ void find_connected(shci_ctx* c, const uint64_t* up, const uint64_t* dn, const d
   cudaStream_t s = c->stream;
   DevBuf<uint32_t> pairs;
   const SelParams P = conn_params(c, pairs);
-  const int n_slots = std::max(1, P.n_elecs + P.n_pairs);
+  const int n_slots = P.n_elecs + P.n_pairs;
+  if (n_slots == 0) {  // no electrons
+    for (size_t k = 0; k <= n; k++) {
+      if (emit && offsets[k] != 0) throw ArgError("offsets do not match the connected-det counts");
+      offsets[k] = 0;
+    }
+    return;
+  }
   // dets per pass: the units' windows and offsets (24 bytes each) stay within 100 MB, or what
   // there is room for
   size_t step = std::max<size_t>(1, (size_t{1} << 22) / n_slots);
