@@ -146,7 +146,7 @@ __device__ __forceinline__ uint32_t warp_run_end(const KT* __restrict__ keys, KT
 // After the sort every position p of a bucket of equal keys makes a span p | end << 32 and the det
 // id of its entry.  A warp per 32 positions: a bucket that ends among them ends at the next lane
 // whose successor differs; only the one that runs on is searched for.  ENTRY: the span goes to its
-// entry's place, else to position p (jdet and ents apart).
+// entry's place, else to position p, and the det ids are left for k_place_spans.
 // To entries, this is bound by the scattered 8-byte writes: 228 million entries 9.3 ms, and 11.4
 // with flags of the bucket starts, their scan and an array of starts (five launches and a wait
 // more: 0.05 against 0.25 ms over the six builds of an n = 16 variation).
@@ -168,7 +168,7 @@ __global__ void k_bucket_spans(const KT* __restrict__ keys, const uint32_t* ents
     if (p < m) {
       const uint32_t v = ents[p];
       span[ENTRY ? v : p] = p | (static_cast<uint64_t>(end) << 32);
-      jdet[p] = v / K;
+      if (ENTRY) jdet[p] = v / K;
     }
   }
 }
@@ -176,22 +176,27 @@ __global__ void k_bucket_spans(const KT* __restrict__ keys, const uint32_t* ents
 // out[ents[p]] = span[p], the entries split by their leading bits: the writes of a while fall in a
 // window that L2 holds, so that a sector goes to memory once and whole.  A block per stretch of
 // positions, in order (a grid that strides over the array writes to every window at once: 8.6 ms
-// against 1.7 at 228 million entries).
+// against 1.7 at 228 million entries).  Beside that, the entries of all positions in jdet become det ids.
 __global__ void __launch_bounds__(256)
     k_place_spans(const uint32_t* __restrict__ ents, const uint64_t* __restrict__ span, uint32_t m,
-                  uint64_t* __restrict__ out) {
+                  uint32_t K, uint64_t* __restrict__ out, uint32_t* __restrict__ jdet) {
   const uint64_t p0 = (uint64_t)blockIdx.x * kPlaceStretch + threadIdx.x;
   uint32_t e[kPlaceStretch / 256];
   uint64_t v[kPlaceStretch / 256];
+  uint32_t j[kPlaceStretch / 256];
 #pragma unroll
   for (int k = 0; k < kPlaceStretch / 256; k++) {
     const uint64_t p = p0 + k * 256;
     e[k] = p < m ? ents[p] : 0u;
     v[k] = p < m ? span[p] : 0u;
+    j[k] = p < m ? jdet[p] : 0u;
   }
 #pragma unroll
   for (int k = 0; k < kPlaceStretch / 256; k++)
-    if (p0 + k * 256 < m) out[e[k]] = v[k];
+    if (p0 + k * 256 < m) {
+      out[e[k]] = v[k];
+      jdet[p0 + k * 256] = j[k] / K;
+    }
 }
 
 }  // namespace
@@ -483,23 +488,24 @@ void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int
                                                                 J.span.p, J.jdet.p);
       SHCI_LAUNCH_CHECK();
     } else {
-      DevBuf<uint32_t> ents;
-      ents.mt = &c->mem;
-      ents.swap(J.jdet);
-      J.jdet.mt = &c->mem;
-      J.jdet.resize(m);
-      k_bucket_spans<KT, false><<<grid_for(m, 256), 256, 0, s>>>(keys.p, ents.p, m32, J.K,
-                                                                 J.span.p, J.jdet.p);
+      // Entries and spans and a sorted copy of both, 24 bytes an entry and no more: the sort is one
+      // digit long, so that the unsorted entries stay for the det ids and the unsorted spans' storage
+      // takes the placed ones.
+      k_bucket_spans<KT, false><<<grid_for(m, 256), 256, 0, s>>>(keys.p, J.jdet.p, m32, J.K,
+                                                                 J.span.p, nullptr);
       SHCI_LAUNCH_CHECK();
       keys.release();
       int top = 0;  // bits of an entry index
       while (top < 32 && (m32 - 1u) >> top) top++;
-      radix_sort_pairs32_64(ents, J.span, m, std::max(0, top - 8), top, s, c->sort, false);
+      c->sort.kalt32.resize(m);
       c->sort.valt64.resize(m);
+      radix_sort_pairs32_64(J.jdet, J.span, m, std::max(0, top - 8), top, s, c->sort, false);
       k_place_spans<<<static_cast<unsigned>((m + kPlaceStretch - 1) / kPlaceStretch), 256, 0, s>>>(
-          ents.p, J.span.p, m32, c->sort.valt64.p);
+          J.jdet.p, J.span.p, m32, J.K, c->sort.valt64.p, c->sort.kalt32.p);
       SHCI_LAUNCH_CHECK();
+      swap_storage(J.jdet, c->sort.kalt32);
       swap_storage(J.span, c->sort.valt64);
+      J.jdet.n = J.span.n = m;
       c->launches += 6;
       release_sort_pingpong(c);
     }
@@ -551,13 +557,12 @@ bool join_prepare(shci_ctx* c) {
     // SHCI_JOIN_BITS (4..40) narrows it, so tests can force colliding buckets.
     int bits = m <= (1ull << 30) ? 32 : 40;
     if (const char* e = std::getenv("SHCI_JOIN_BITS")) bits = std::min(40, std::max(4, std::atoi(e)));
-    // Spans by way of their entries' leading bits where they outgrow L2 and the storage of that
-    // (34 bytes an entry) is there.  Straight against by leading bits: 9.5 million entries 0.14
-    // against 0.21 ms, 17 million 0.43 against 0.35, 76 million 2.9 against 1.4, 228 million 9.3
-    // against 4.3.  SHCI_JOIN_SPLIT=0 or 1 takes the one or the other at any size.
-    const double want = static_cast<double>(m) * 34.0;
-    bool split = m > kSplitEntries && want < 0.85 * static_cast<double>(avail);
-    if (const char* e = std::getenv("SHCI_JOIN_SPLIT")) split = std::atoi(e) != 0;
+    // Spans by way of their entries' leading bits where they outgrow L2.  Straight against by
+    // leading bits: 9.5 million entries 0.14 against 0.21 ms, 17 million 0.43 against 0.35, 76
+    // million 2.9 against 1.4, 228 million 9.3 against 4.3.  SHCI_JOIN_SPLIT=0 or 1 takes the one or
+    // the other at any size (a single entry goes straight).
+    bool split = m > kSplitEntries;
+    if (const char* e = std::getenv("SHCI_JOIN_SPLIT")) split = std::atoi(e) != 0 && m > 1;
     if (bits <= 32) join_index(c, J.keys32, bits, n, n_up, n_dn, split);
     else join_index(c, J.keys, bits, n, n_up, n_dn, split);
   } catch (const OomError&) {
