@@ -38,8 +38,8 @@ struct OverflowError : std::runtime_error {
 // released blocks.  A build or a PT2 pass allocates and frees scratch of the same sizes again
 // and again (gigabytes at n = 40, where cudaMalloc / cudaFree of a large block costs about a
 // millisecond and the free synchronises the device); a released block is kept and handed to
-// the next request it fits (up to twice the size asked for).  All work of a context runs on
-// its one stream, so a block reused after a release is ordered after the work that used it.
+// the next request it fits (up to twice the size asked for, DevBuf::fit).  All work of a context
+// runs on its one stream, so a block reused after a release is ordered after the work that used it.
 // A request that does not fit the device or the budget first returns the cache to the driver.
 // The cache holds at most a quarter of the device's memory, so the driver always keeps room
 // for what it allocates by itself (local memory of launches, library workspaces).
@@ -57,10 +57,11 @@ struct MemTracker {
   MemTracker& operator=(const MemTracker&) = delete;
   ~MemTracker() { flush(); }
 
-  // A cached block of at least `bytes` (at most twice that); *got = its size.
-  void* take(size_t bytes, size_t* got) {
+  // A cached block of at least `bytes` (at most `fit` times that); *got = its size.
+  void* take(size_t bytes, size_t* got, double fit) {
     auto it = cache.lower_bound(bytes);
-    if (it == cache.end() || it->first > 2 * bytes) return nullptr;
+    if (it == cache.end() || static_cast<double>(it->first) > fit * static_cast<double>(bytes))
+      return nullptr;
     void* p = it->second;
     *got = it->first;
     cached -= it->first;
@@ -100,6 +101,7 @@ struct DevBuf {
   size_t n = 0;
   size_t cap = 0;
   MemTracker* mt = nullptr;
+  double fit = 2.0;  // largest cached block to take, in multiples of the size asked for
 
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
@@ -128,7 +130,7 @@ struct DevBuf {
     c = bytes / sizeof(T);
     if (mt) {
       size_t got = 0;
-      if (void* b = mt->take(bytes, &got)) {
+      if (void* b = mt->take(bytes, &got, fit)) {
         p = static_cast<T*>(b);
         cap = got / sizeof(T);
         mt->note_live();
