@@ -457,6 +457,20 @@ void sort_keys(DevBuf<uint64_t>& k, DevBuf<uint32_t>& v, size_t m, int bits, shc
   radix_sort_pairs(k, v, m, 0, bits, c->stream, c->sort, false);
 }
 
+// Room to sort entries and spans by their entries: the keys' storage, once the buckets are known,
+// and 8 or 4 bytes an entry more.
+void split_room(shci_ctx* c, const DevBuf<uint32_t>&, size_t m) { c->sort.valt64.resize(m); }
+void split_room(shci_ctx* c, const DevBuf<uint64_t>&, size_t m) { c->sort.kalt32.resize(m); }
+void split_take(shci_ctx* c, DevBuf<uint32_t>& keys) { swap_storage(keys, c->sort.kalt32); }
+void split_take(shci_ctx* c, DevBuf<uint64_t>& keys) { swap_storage(keys, c->sort.valt64); }
+
+// SHCI_JOIN_SPLIT: 0 places spans straight and 1 by their entries' leading bits, at any size; 2 is 1
+// with its storage refused.
+int split_env() {
+  const char* e = std::getenv("SHCI_JOIN_SPLIT");
+  return e ? std::atoi(e) : -1;
+}
+
 // Entries -> sorted buckets -> spans; keys of type KT hold `bits` hash bits.
 template <class KT>
 void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int n_dn,
@@ -483,22 +497,28 @@ void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int
   {
     ProfScope ps(c->prof, s, "join_buckets");
     const uint32_t m32 = static_cast<uint32_t>(m);
+    if (split) {
+      try {
+        if (split_env() == 2) throw OomError("refused");
+        split_room(c, keys, m);
+      } catch (const OomError&) {  // straight needs no more storage
+        split = false;
+      }
+    }
     if (!split) {
       k_bucket_spans<KT, true><<<grid_for(m, 256), 256, 0, s>>>(keys.p, J.jdet.p, m32, J.K,
                                                                 J.span.p, J.jdet.p);
       SHCI_LAUNCH_CHECK();
     } else {
-      // Entries and spans and a sorted copy of both, 24 bytes an entry and no more: the sort is one
+      // Entries and spans and a sorted copy of both, 24 bytes an entry with the keys': the sort is one
       // digit long, so that the unsorted entries stay for the det ids and the unsorted spans' storage
       // takes the placed ones.
       k_bucket_spans<KT, false><<<grid_for(m, 256), 256, 0, s>>>(keys.p, J.jdet.p, m32, J.K,
                                                                  J.span.p, nullptr);
       SHCI_LAUNCH_CHECK();
-      keys.release();
+      split_take(c, keys);
       int top = 0;  // bits of an entry index
       while (top < 32 && (m32 - 1u) >> top) top++;
-      c->sort.kalt32.resize(m);
-      c->sort.valt64.resize(m);
       radix_sort_pairs32_64(J.jdet, J.span, m, std::max(0, top - 8), top, s, c->sort, false);
       k_place_spans<<<static_cast<unsigned>((m + kPlaceStretch - 1) / kPlaceStretch), 256, 0, s>>>(
           J.jdet.p, J.span.p, m32, J.K, c->sort.valt64.p, c->sort.kalt32.p);
@@ -559,10 +579,9 @@ bool join_prepare(shci_ctx* c) {
     if (const char* e = std::getenv("SHCI_JOIN_BITS")) bits = std::min(40, std::max(4, std::atoi(e)));
     // Spans by way of their entries' leading bits where they outgrow L2.  Straight against by
     // leading bits: 9.5 million entries 0.14 against 0.21 ms, 17 million 0.43 against 0.35, 76
-    // million 2.9 against 1.4, 228 million 9.3 against 4.3.  SHCI_JOIN_SPLIT=0 or 1 takes the one or
-    // the other at any size (a single entry goes straight).
-    bool split = m > kSplitEntries;
-    if (const char* e = std::getenv("SHCI_JOIN_SPLIT")) split = std::atoi(e) != 0 && m > 1;
+    // million 2.9 against 1.4, 228 million 9.3 against 4.0.  (A single entry goes straight.)
+    const int env = split_env();
+    const bool split = env < 0 ? m > kSplitEntries : env != 0 && m > 1;
     if (bits <= 32) join_index(c, J.keys32, bits, n, n_up, n_dn, split);
     else join_index(c, J.keys, bits, n, n_up, n_dn, split);
   } catch (const OomError&) {

@@ -30,3 +30,31 @@ def test_index_within_its_estimate(monkeypatch, split, bits):
     c.close()
     entries = 16000 * 190
     assert peak - live < entries * (26 if bits == "32" else 28) + 16000 * 64
+
+
+@pytest.mark.parametrize("bits", ["9", "40"])
+def test_without_room_to_split(monkeypatch, bits):
+    """Without storage to place spans by their entries' leading bits they go straight: the join
+    still builds the matrix, with the same columns and bit-equal values."""
+    import shci_gb300
+    from conftest import C_ATOM
+    rng = np.random.default_rng(4)
+    occ = {(tuple(sorted(rng.choice(9, 4, replace=False))), tuple(sorted(rng.choice(9, 2, replace=False))))
+           for _ in range(900)}
+    up = np.array([sum(1 << int(o) for o in a) for a, _ in sorted(occ)], np.uint64)
+    dn = np.array([sum(1 << int(o) for o in b) for _, b in sorted(occ)], np.uint64)
+    monkeypatch.setenv("SHCI_JOIN_BITS", bits)
+    got = []
+    for split in ("0", "1", "2"):
+        monkeypatch.setenv("SHCI_JOIN_SPLIT", split)
+        c = shci_gb300.Context()
+        c.load_fcidump(C_ATOM, 4, 2, "d2h")
+        c.set_dets(up, dn)
+        nnz, _ = c.update_hamiltonian(shci_gb300.PREC_FP64)
+        assert c.hamiltonian_stats()["path"] == "core_join"
+        rp, cols, vals, diag = c.hamiltonian(nnz)
+        c.close()
+        o = np.lexsort((cols, np.repeat(np.arange(len(up)), np.diff(rp).astype(int))))
+        got.append((rp, cols[o], vals[o], diag))
+    for g in got[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(g, got[0]))
