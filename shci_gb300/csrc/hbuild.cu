@@ -485,6 +485,12 @@ __global__ void k_hb_row_bound(const uint64_t* __restrict__ up, const uint64_t* 
   }
 }
 
+// The join's index ends with the build, also with one that fails.
+struct JoinScope {
+  shci_ctx* c;
+  ~JoinScope() { join_release(c); }
+};
+
 }  // namespace
 
 size_t build_hamiltonian(shci_ctx* c, int precision) {
@@ -512,6 +518,7 @@ size_t build_hamiltonian(shci_ctx* c, int precision) {
   H.valid = false;
   H.build_id++;
   H.bound_valid = false;
+  JoinScope join_scope{c};
   H.join = !scan_only && join_prepare(c);
   if (!H.join) n_prev = 0;  // the group scan builds whole matrices only
   else if (two_pass) join_check(c);
