@@ -821,6 +821,7 @@ void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSource
   constexpr int NV = n_cols<MODE>();
   cudaStream_t s = c->stream;
   const uint64_t kCap = 1ull << 27;
+  uint64_t run = kCap;  // regions of a launch at most; fewer where these find no room
   DevBuf<PtRec<NV>> out;
   DevBuf<uint64_t> d_dst;
   DevBuf<uint32_t> d_cnt;
@@ -835,13 +836,19 @@ void pt_emit_append(shci_ctx* c, PtSetup& st, const PtParams& Q, const StoSource
   uint64_t base = 0;  // off[k0]
   while (k0 < L.n) {
     uint64_t end = 0;
-    const size_t k1 = piece_run(c, L, k0, base, kCap, &end);
+    const size_t k1 = piece_run(c, L, k0, base, run, &end);
     const uint64_t tot = end - base;
     const uint32_t n = static_cast<uint32_t>(k1 - k0);
+    try {
+      out.resize(std::max<uint64_t>(tot, 1), 1.25);
+    } catch (const OomError&) {
+      if (n == 1 || tot <= kCap >> 8) throw;
+      run = std::max(tot / 4, kCap >> 8);
+      continue;
+    }
     d_cnt.resize((size_t)n + 2);  // (the overflow count and the pieces taken after the pieces' counts)
     d_dst.resize((size_t)n + 1);
     SHCI_CUDA(cudaMemsetAsync(d_cnt.p, 0, ((size_t)n + 2) * 4, s));
-    out.resize(std::max<uint64_t>(tot, 1), 1.25);
     const PtPieces pc{L.src.p + k0, L.begin.p + k0, L.len.p + k0, L.off.p + k0, d_cnt.p,
                       d_cnt.p + n + 1, n, base};
     {
@@ -974,6 +981,27 @@ void pt_batch_sums(shci_ctx* c, const DevBuf<PtRec<n_cols<MODE>()>>& rec, size_t
   c->launches += 2;
 }
 
+// Runs one batch of n_batches in *parts parts: the batches b + n_batches j, j < *parts, of n_batches *
+// *parts, which together hold the dets of batch b (the remainder by the larger number fixes that by
+// the smaller).  Where their records find no room there are twice as many from then on.
+constexpr uint64_t kMaxParts = 1024;
+template <class F>
+void pt_in_parts(shci_ctx* c, uint64_t n_batches, uint64_t* parts, F&& run) {
+  for (;;) {
+    try {
+      run();
+      return;
+    } catch (const OomError&) {
+      if (*parts >= kMaxParts || n_batches * *parts >= 1ull << 31) throw;
+    }
+    *parts *= 2;
+    // scratch that the attempt has grown
+    c->u0.release();
+    c->sort.kalt32.release();
+    c->sort.valt32.release();
+  }
+}
+
 // Deterministic-style batched stage (dtm: MODE kDtm, psto: kPsto) with the batch accumulation,
 // uncertainty and (psto) early stopping of solver.h:691-764, 818-895.
 template <int MODE>
@@ -1014,11 +1042,31 @@ Pt2Out pt_batched(shci_ctx* c, double e_var, PtParams Q, size_t n_batches, doubl
   size_t n_sum = 0;
   DevBuf<PtRec<n_cols<MODE>()>> rec;
   rec.mt = &c->mem;
+  uint64_t parts = 1, listed = 1;  // listed: those that the pieces' regions are made for
   for (size_t batch = 0; batch < n_batches; batch++) {
-    Q.batch = batch;
-    const size_t bn = pt_emit_reduce<MODE>(c, st, Q, S, pieces, rec, 0);
-    double bs, bsq;
-    pt_batch_sums<MODE>(c, rec, bn, e_var, &bs, &bsq);
+    size_t bn = 0;
+    double bs = 0.0, bsq = 0.0;
+    pt_in_parts(c, n_batches, &parts, [&]() {
+      if (listed != parts) {
+        rec.release();
+        set_batches(Q, n_batches * parts);
+        DevBuf<uint64_t> again;
+        pt_counts<MODE>(c, st, Q, S, n_var, again);
+        make_pt_pieces(c, again, n_var, n_batches * parts, nullptr, pieces);
+        listed = parts;
+      }
+      bn = 0;
+      bs = bsq = 0.0;
+      for (uint64_t j = 0; j < parts; j++) {
+        Q.batch = batch + n_batches * j;
+        const size_t m = pt_emit_reduce<MODE>(c, st, Q, S, pieces, rec, 0);
+        double sum, sumsq;
+        pt_batch_sums<MODE>(c, rec, m, e_var, &sum, &sumsq);
+        bn += m;
+        bs += sum;
+        bsq += sumsq;
+      }
+    });
     n_sum += bn;
     esum += bs;
     esq += bsq;
@@ -1121,10 +1169,11 @@ size_t pilot_pt_dets(shci_ctx* c, PtSetup& st, const std::vector<size_t>& src, d
   std::vector<uint32_t> h_det(src.begin(), src.end()), h_zero(n_src, 0u);
   std::vector<double> h_one(n_src, 1.0);
   std::vector<uint8_t> h_dtm(n_src, 1);
-  DevBuf<uint32_t> d_det, d_zero;
+  DevBuf<uint32_t> d_det, d_zero, d_batch;
   DevBuf<double> d_one;
   DevBuf<uint8_t> d_dtm;
-  d_det.mt = d_zero.mt = d_one.mt = d_dtm.mt = &c->mem;
+  d_det.mt = d_zero.mt = d_batch.mt = d_one.mt = d_dtm.mt = &c->mem;
+  d_batch.resize(n_src);
   d_det.resize(n_src);
   d_zero.resize(n_src);
   d_one.resize(n_src);
@@ -1133,21 +1182,31 @@ size_t pilot_pt_dets(shci_ctx* c, PtSetup& st, const std::vector<size_t>& src, d
   SHCI_CUDA(cudaMemcpyAsync(d_zero.p, h_zero.data(), n_src * 4, cudaMemcpyHostToDevice, s));
   SHCI_CUDA(cudaMemcpyAsync(d_one.p, h_one.data(), n_src * 8, cudaMemcpyHostToDevice, s));
   SHCI_CUDA(cudaMemcpyAsync(d_dtm.p, h_dtm.data(), n_src, cudaMemcpyHostToDevice, s));
-  StoSources S{d_det.p, d_zero.p, d_one.p, d_one.p, d_zero.p, d_dtm.p};
+  StoSources S{d_det.p, d_zero.p, d_one.p, d_one.p, d_batch.p, d_dtm.p};
   PtParams Q{};
   Q.eps = eps_pt;
   Q.eps_psto = eps_pt;
   Q.factor = 0.0;
   Q.iter_shift = shift;
   Q.pilot = 1;
-  set_batches(Q, 128);
-  DevBuf<uint64_t> entries;
-  pt_counts<kSto>(c, st, Q, S, n_src, entries);
-  PieceList pieces(c);
-  make_pt_pieces(c, entries, n_src, 128, nullptr, pieces);
-  DevBuf<PtRec<5>> rec;
-  rec.mt = &c->mem;
-  return pt_emit_reduce<kSto>(c, st, Q, S, pieces, rec, 5);
+  size_t n = 0;
+  uint64_t parts = 1;
+  pt_in_parts(c, 128, &parts, [&]() {
+    set_batches(Q, 128 * parts);
+    DevBuf<uint64_t> entries;
+    pt_counts<kSto>(c, st, Q, S, n_src, entries);
+    PieceList pieces(c);
+    make_pt_pieces(c, entries, n_src, 128 * parts, nullptr, pieces);
+    DevBuf<PtRec<5>> rec;
+    rec.mt = &c->mem;
+    n = 0;
+    for (uint64_t j = 0; j < parts; j++) {
+      const std::vector<uint32_t> b(n_src, static_cast<uint32_t>(128 * j));
+      SHCI_CUDA(cudaMemcpyAsync(d_batch.p, b.data(), n_src * 4, cudaMemcpyHostToDevice, s));
+      n += pt_emit_reduce<kSto>(c, st, Q, S, pieces, rec, 5);
+    }
+  });
+  return n;
 }
 
 size_t psto_auto_batches(shci_ctx* c, double eps_pt_psto, double pt_mem_avail, double mem_usage,
@@ -1348,6 +1407,7 @@ Pt2Out pt2_sto(shci_ctx* c, double energy_var, double eps_pt_psto, double eps_pt
   std::vector<double> loop_vals;
   bool done = false;
   size_t iteration = 0;
+  uint64_t parts = 1;
   while (!done && iteration < max_iterations) {
     // draw the samples of the next chunk of iterations (solver.h:1048-1072)
     const uint32_t chunk = iteration == 0 ? kFirstChunk : kNextChunk;
@@ -1480,41 +1540,52 @@ Pt2Out pt2_sto(shci_ctx* c, double energy_var, double eps_pt_psto, double eps_pt
     PtParams Q{};
     Q.eps = eps_pt;
     Q.eps_psto = eps_pt_psto;
-    set_batches(Q, n_batches);
     Q.factor = factor;
     Q.iter_shift = shift;
-    DevBuf<uint64_t> entries;
-    pt_counts<kSto>(c, st, Q, S, n_src, entries);
-    PieceList pieces(c);
-    make_pt_pieces(c, entries, n_src, n_batches, d_off.p, pieces);
-    DevBuf<PtRec<5>> rec;
-    rec.mt = &c->mem;
-    const size_t bn = pt_emit_reduce<kSto>(c, st, Q, S, pieces, rec, 5);
-    // per-iteration sums of the contributions
-    std::vector<double> it_sum(n_it, 0.0);
-    if (bn) {
-      DevBuf<double> x, o;
-      DevBuf<uint64_t> starts;
-      x.mt = o.mt = starts.mt = &c->mem;
-      x.resize(bn);
-      o.resize(2 * n_it);
-      starts.resize(n_it + 1);
-      const uint64_t mask = shift == 64 ? ~0ull : ((1ull << shift) - 1ull);
-      {
-        ProfScope ps(c->prof, s, "pt2_contrib");
-        k_pt_x<kSto><<<grid_for(bn, 256), 256, 0, s>>>(diag_fix(c), rec.p, bn, energy_var,
-                                                       static_cast<double>(n_batches), mask, x.p);
-        SHCI_LAUNCH_CHECK();
-        k_iter_starts<<<1, 128, 0, s>>>(rec.p, bn, shift, n_it, starts.p);
-        SHCI_LAUNCH_CHECK();
-        seg_reduce2(c, x.p, starts.p, n_it, bn, o.p);
+    size_t bn = 0;
+    std::vector<double> it_sum;  // per-iteration sums of the contributions
+    pt_in_parts(c, n_batches, &parts, [&]() {
+      set_batches(Q, n_batches * parts);
+      DevBuf<uint64_t> entries;
+      pt_counts<kSto>(c, st, Q, S, n_src, entries);
+      PieceList pieces(c);
+      make_pt_pieces(c, entries, n_src, n_batches * parts, d_off.p, pieces);
+      DevBuf<PtRec<5>> rec;
+      rec.mt = &c->mem;
+      bn = 0;
+      it_sum.assign(n_it, 0.0);
+      for (uint64_t j = 0; j < parts; j++) {
+        std::vector<uint32_t> b;
+        if (parts > 1) {
+          for (uint32_t x : h_batch) b.push_back(static_cast<uint32_t>(x + n_batches * j));
+          SHCI_CUDA(cudaMemcpyAsync(d_batch.p, b.data(), n_ent * 4, cudaMemcpyHostToDevice, s));
+        }
+        const size_t m = pt_emit_reduce<kSto>(c, st, Q, S, pieces, rec, 5);
+        if (!m) continue;
+        DevBuf<double> x, o;
+        DevBuf<uint64_t> starts;
+        x.mt = o.mt = starts.mt = &c->mem;
+        x.resize(m);
+        o.resize(2 * n_it);
+        starts.resize(n_it + 1);
+        const uint64_t mask = shift == 64 ? ~0ull : ((1ull << shift) - 1ull);
+        {
+          ProfScope ps(c->prof, s, "pt2_contrib");
+          k_pt_x<kSto><<<grid_for(m, 256), 256, 0, s>>>(diag_fix(c), rec.p, m, energy_var,
+                                                        static_cast<double>(n_batches), mask, x.p);
+          SHCI_LAUNCH_CHECK();
+          k_iter_starts<<<1, 128, 0, s>>>(rec.p, m, shift, n_it, starts.p);
+          SHCI_LAUNCH_CHECK();
+          seg_reduce2(c, x.p, starts.p, n_it, m, o.p);
+        }
+        std::vector<double> h(2 * n_it);
+        SHCI_CUDA(cudaMemcpyAsync(h.data(), o.p, h.size() * 8, cudaMemcpyDeviceToHost, s));
+        SHCI_CUDA(cudaStreamSynchronize(s));
+        for (uint32_t it = 0; it < n_it; it++) it_sum[it] += h[2 * it];
+        bn += m;
+        c->launches += 3;
       }
-      std::vector<double> h(2 * n_it);
-      SHCI_CUDA(cudaMemcpyAsync(h.data(), o.p, h.size() * 8, cudaMemcpyDeviceToHost, s));
-      SHCI_CUDA(cudaStreamSynchronize(s));
-      for (uint32_t it = 0; it < n_it; it++) it_sum[it] = h[2 * it];
-      c->launches += 3;
-    }
+    });
     out.n_pt_dets += bn;
     // statistics and stopping rules, iteration by iteration (solver.h:1126-1147)
     for (uint32_t it = 0; it < n_it && !done; it++) {
