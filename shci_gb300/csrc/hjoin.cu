@@ -450,6 +450,14 @@ void release_sort_pingpong(shci_ctx* c) {
   c->sort.valt64.release();
 }
 
+// The sorts' storage goes back before the stored elements are allocated: their digit counts too, which
+// for m entries are more than the packed dets.
+void release_sort_scratch(shci_ctx* c) {
+  release_sort_pingpong(c);
+  c->sort.hist.release();
+  c->sort.part32.release();
+}
+
 void sort_keys(DevBuf<uint32_t>& k, DevBuf<uint32_t>& v, size_t m, int bits, shci_ctx* c) {
   radix_sort_pairs32(k, v, m, 0, bits, c->stream, c->sort, false);
 }
@@ -527,9 +535,9 @@ void join_index(shci_ctx* c, DevBuf<KT>& keys, int bits, size_t n, int n_up, int
       swap_storage(J.span, c->sort.valt64);
       J.jdet.n = J.span.n = m;
       c->launches += 6;
-      release_sort_pingpong(c);
     }
   }
+  release_sort_scratch(c);
   keys.release();
   J.key_bytes = sizeof(KT);
   J.bits = bits;
@@ -586,7 +594,7 @@ bool join_prepare(shci_ctx* c) {
     else join_index(c, J.keys, bits, n, n_up, n_dn, split);
   } catch (const OomError&) {
     join_release(c);
-    release_sort_pingpong(c);
+    release_sort_scratch(c);
     return false;
   }
   return true;

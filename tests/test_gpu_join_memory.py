@@ -58,3 +58,22 @@ def test_without_room_to_split(monkeypatch, bits):
         got.append((rp, cols[o], vals[o], diag))
     for g in got[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(g, got[0]))
+
+
+def test_scratch_is_given_back():
+    """After the build of next to no elements the context holds row arrays and items, 64 bytes a det,
+    and not the digit counts of the entries' sorts (0.3 bytes an entry, 60 a det)."""
+    import shci_gb300
+    from shci_gb300 import synthetic
+    h, g = synthetic.integrals(40, 9)
+    rng = np.random.default_rng(1)
+    n = 16000
+    up, dn = (np.array([sum(1 << int(o) for o in rng.choice(40, 10, replace=False)) for _ in range(n)],
+                       np.uint64) for _ in range(2))
+    c = shci_gb300.Context()
+    c.set_integrals(h, g, 10, 10, 0x3ff, 0x3ff)
+    c.set_dets(up, dn)
+    live = c.memory_stats()[0] - c.memory_cached()[0]
+    c.update_hamiltonian(shci_gb300.PREC_FP64)
+    assert c.memory_stats()[0] - c.memory_cached()[0] - live < 64 * n
+    c.close()
