@@ -39,7 +39,7 @@ __device__ __forceinline__ bool conn_window(const double* eps_max, const double*
   return !(*hi < *lo);
 }
 
-// Window of each (det, slot): {first entry, entries, electron orbitals (make_candidate_at), 0}.
+// Window of each (det, slot): {first entry, entries, slot code, 0}.
 __global__ void k_conn_windows(SelParams P, const uint64_t* __restrict__ up,
                                const uint64_t* __restrict__ dn,
                                const double* __restrict__ eps_max,
@@ -49,10 +49,10 @@ __global__ void k_conn_windows(SelParams P, const uint64_t* __restrict__ up,
        t += gridDim.x * blockDim.x) {
     const uint32_t k = t / n_slots;
     double lo, hi;
-    uint32_t first = 0, cnt = 0, orbs = 0;
+    uint32_t first = 0, cnt = 0, code = 0;
     if (conn_window(eps_max, eps_min, k, &lo, &hi))
-      slot_range(P, up[k], dn[k], static_cast<int>(t % n_slots), lo, hi, &first, &cnt, &orbs);
-    win[t] = make_uint4(first, cnt, orbs, 0u);
+      code = slot_range(P, up[k], dn[k], static_cast<int>(t % n_slots), lo, hi, &first, &cnt);
+    win[t] = make_uint4(first, cnt, code, 0u);
   }
 }
 
@@ -63,6 +63,15 @@ struct ConnOut {
   uint64_t* dn;
   uint8_t* nx;
 };
+
+// Entry x of det (u, d) to place q.
+__device__ __forceinline__ void conn_put(const ConnOut& out, uint64_t q, uint32_t x, uint64_t u,
+                                         uint64_t d) {
+  apply_entry(x, &u, &d);
+  out.up[q] = u;
+  out.dn[q] = d;
+  out.nx[q] = x & kOne ? 1 : 2;
+}
 
 // Units of one slot.  EMIT: writes the unit's valid entries at off[unit]; else counts them into
 // off[unit].
@@ -79,21 +88,15 @@ __global__ void __launch_bounds__(kConnWarps * 32)
        t < end; t += warps) {
     const uint4 w = win[t];
     const uint32_t k = t / n_slots;
-    const int slot = static_cast<int>(t % n_slots);
     uint64_t pos = EMIT ? off[t] - out.base : 0;
     if (w.y) {
       const uint64_t u = up[k], d = dn[k];
       for (uint32_t e0 = 0; e0 < w.y; e0 += 32) {
-        uint64_t cu = 0, cd = 0;
-        const bool ok = e0 + lane < w.y &&
-                        make_candidate_at(P, u, d, slot, w.z, w.x + e0 + lane, &cu, &cd);
+        uint32_t x = 0;
+        const bool ok = e0 + lane < w.y && entry_code(P, w.z, w.x + e0 + lane, u | P.inactive,
+                                                      d | P.inactive, &x);
         const unsigned bal = __ballot_sync(kFull, ok);
-        if (EMIT && ok) {
-          const uint64_t q = pos + __popc(bal & lt);
-          out.up[q] = cu;
-          out.dn[q] = cd;
-          out.nx[q] = slot < P.n_elecs ? 1 : 2;
-        }
+        if (EMIT && ok) conn_put(out, pos + __popc(bal & lt), x, u, d);
         pos += __popc(bal);
       }
     }
@@ -125,8 +128,8 @@ __global__ void __launch_bounds__(kConnWarps * 32)
         !(lo > P.max_singles && lo > P.max_hci)) {  // (narrow windows of light dets are empty)
       const uint64_t u = up[k], d = dn[k];
       for (int s0 = first; s0 < last; s0 += 32) {
-        uint32_t b = 0, c = 0, orbs = 0;
-        if (s0 + (int)lane < last) slot_range(P, u, d, s0 + lane, lo, hi, &b, &c, &orbs);
+        uint32_t b = 0, c = 0, code = 0;
+        if (s0 + (int)lane < last) code = slot_range(P, u, d, s0 + lane, lo, hi, &b, &c);
         uint32_t inc = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -143,17 +146,11 @@ __global__ void __launch_bounds__(kConnWarps * 32)
             if (v <= e) ol += step;
           }
           const uint32_t at = e - __shfl_sync(kFull, inc - c, ol) + __shfl_sync(kFull, b, ol);
-          const uint32_t o_orbs = __shfl_sync(kFull, orbs, ol);
-          const int slot = s0 + static_cast<int>(ol);
-          uint64_t cu = 0, cd = 0;
-          const bool ok = e < total && make_candidate_at(P, u, d, slot, o_orbs, at, &cu, &cd);
+          const uint32_t o_code = __shfl_sync(kFull, code, ol);
+          uint32_t x = 0;
+          const bool ok = e < total && entry_code(P, o_code, at, u | P.inactive, d | P.inactive, &x);
           const unsigned bal = __ballot_sync(kFull, ok);
-          if (EMIT && ok) {
-            const uint64_t q = pos + __popc(bal & lt);
-            out.up[q] = cu;
-            out.dn[q] = cd;
-            out.nx[q] = slot < P.n_elecs ? 1 : 2;
-          }
+          if (EMIT && ok) conn_put(out, pos + __popc(bal & lt), x, u, d);
           pos += __popc(bal);
         }
       }

@@ -70,11 +70,6 @@ __device__ __forceinline__ int nth_bit(uint64_t x, int k) {
   return pos;
 }
 
-// spin-orbital index of electron e (up electrons first, then dn + n)
-__device__ __forceinline__ int elec_orb(uint64_t up, uint64_t dn, int e, int n_up, int n) {
-  return e < n_up ? nth_bit(up, e) : nth_bit(dn, e - n_up) + n;
-}
-
 // First k in [lo, hi) with a[k] < x, for a descending array of non-negative values and
 // any x.  Non-negative doubles order like the integers of their bit patterns (a negative or
 // NaN x compares false against every entry, as in FP64), so the comparisons run on the
@@ -98,43 +93,101 @@ __device__ __forceinline__ size_t c2(size_t a, size_t b) {
   return a > b ? (a * (a + 1)) / 2 + b : (b * (b + 1)) / 2 + a;
 }
 
-// Entry range [lo, lo + cnt) of slot `slot` for the det (eps window [eps_min, eps_max)).
-// *orbs (optional) receives the slot's electron orbitals for make_candidate_at: the moved
-// orbital of a single, or the two spin-orbitals p | q << 8 of a pair.
-__device__ __forceinline__ void slot_range(const SelParams& P, uint64_t up, uint64_t dn, int slot,
-                                           double eps_min, double eps_max, uint32_t* lo,
-                                           uint32_t* cnt, uint32_t* orbs = nullptr) {
+// Slot code: the orbitals p and q that the electrons leave, and the strings that the targets r and s
+// of an entry must be free in; an entry's code adds its targets.  A queue entry's r | s << 16 holds
+// the targets of the stored pair; a beta-beta pair is stored as its alpha image and an alpha-beta
+// pair p > q as (q, p) (chem_system.cc:347-361), so the strings follow from the slot alone.
+constexpr int kPBit = 0, kQBit = 6, kRBit = 12, kSBit = 18;
+enum : uint32_t { kADn = 1u << 24, kBDn = 1u << 25, kOne = 1u << 26 };
+
+// Entry range [lo, lo + cnt) of slot `slot` of a det in the eps window [eps_min, eps_max), and the
+// slot's code; orb(e) is the spatial orbital of electron e, alpha electrons first.
+template <class Orb>
+__device__ __forceinline__ uint32_t slot_window(const SelParams& P, Orb&& orb, int slot,
+                                                double eps_min, double eps_max, uint32_t* lo,
+                                                uint32_t* cnt) {
   *lo = 0;
   *cnt = 0;
   const int n = P.n_orbs;
   if (slot < P.n_elecs) {
-    if (eps_min > P.max_singles) return;
-    const int p = slot < P.n_up ? nth_bit(up, slot) : nth_bit(dn, slot - P.n_up);
-    if (orbs) *orbs = static_cast<uint32_t>(p);
+    if (eps_min > P.max_singles) return 0;
+    const uint32_t p = orb(slot);
     const uint32_t a = P.s_off[p], b = P.s_off[p + 1];
     *lo = a;
     *cnt = first_below(P.s_S, a, b, eps_min) - a;
-    return;
+    return p << kPBit | kOne | (slot < P.n_up ? 0u : kADn);
   }
-  if (P.no_doubles || eps_min > P.max_hci) return;
+  if (P.no_doubles || eps_min > P.max_hci) return 0;
   const uint32_t pr = P.pair_tab[slot - P.n_elecs];
-  const int p = elec_orb(up, dn, pr & 0xffff, P.n_up, n);
-  const int q = elec_orb(up, dn, pr >> 16, P.n_up, n);
-  if (orbs) *orbs = static_cast<uint32_t>(p) | (static_cast<uint32_t>(q) << 8);
-  int p2 = p, q2 = q;
-  if (p >= n && q >= n) {
-    p2 -= n;
-    q2 -= n;
-  } else if (p < n && q >= n && p > q - n) {
-    p2 = q - n;
-    q2 = p + n;
+  const int e1 = pr & 0xffff, e2 = pr >> 16;
+  const uint32_t p = orb(e1), q = orb(e2);
+  const bool dn1 = e1 >= P.n_up, dn2 = e2 >= P.n_up;
+  uint32_t code;
+  size_t pq;
+  if (dn1 == dn2) {
+    pq = c2(p, q);
+    code = p << kPBit | q << kQBit | (dn1 ? kADn | kBDn : 0u);
+  } else if (p > q) {  // stored as (q, p + n): r goes to beta, s to alpha
+    pq = c2(q, p + n);
+    code = p << kPBit | q << kQBit | kADn;
+  } else {
+    pq = c2(p, q + n);
+    code = p << kPBit | q << kQBit | kBDn;
   }
-  const size_t pq = c2(p2, q2);
   const uint32_t a = static_cast<uint32_t>(P.d_off[pq]), b = static_cast<uint32_t>(P.d_off[pq + 1]);
   const uint32_t s = first_below(P.d_H, a, b, eps_max);
-  const uint32_t e = first_below(P.d_H, s, b, eps_min);
   *lo = s;
-  *cnt = e - s;
+  *cnt = first_below(P.d_H, s, b, eps_min) - s;
+  return code;
+}
+
+// The same with the orbitals from the det's strings.
+__device__ __forceinline__ uint32_t slot_range(const SelParams& P, uint64_t up, uint64_t dn,
+                                               int slot, double eps_min, double eps_max,
+                                               uint32_t* lo, uint32_t* cnt) {
+  return slot_window(
+      P, [&](int e) { return e < P.n_up ? nth_bit(up, e) : nth_bit(dn, e - P.n_up); }, slot, eps_min,
+      eps_max, lo, cnt);
+}
+
+__device__ __forceinline__ uint32_t bit_of(uint64_t x, uint32_t k) {
+  const uint32_t w = k & 32u ? static_cast<uint32_t>(x >> 32) : static_cast<uint32_t>(x);
+  return w >> (k & 31u) & 1u;
+}
+
+// Code of queue entry e of the slot with code `code`; false where a target is occupied or inactive
+// (active space): bu and bd hold those orbitals.
+__device__ __forceinline__ bool entry_code(const SelParams& P, uint32_t code, uint32_t e,
+                                           uint64_t bu, uint64_t bd, uint32_t* x) {
+  const uint32_t n = static_cast<uint32_t>(P.n_orbs);  // an alpha-beta pair's s is stored as s + n
+  const uint64_t A = code & kADn ? bd : bu;
+  const uint64_t B = code & kOne ? 0ull : code & kBDn ? bd : bu;
+  const uint32_t rs = code & kOne ? P.s_r[e] : P.d_rs[e];
+  const uint32_t r = rs & 0xffffu;
+  uint32_t s = rs >> 16;
+  if (s >= n) s -= n;
+  *x = code | r << kRBit | s << kSBit;
+  return !(bit_of(A, r) | bit_of(B, s));
+}
+
+// The determinant that entry `code` (with its targets) makes of (*u, *d).
+__device__ __forceinline__ void apply_entry(uint32_t code, uint64_t* u, uint64_t* d) {
+  const uint64_t out1 = 1ull << (code >> kPBit & 63u), out2 = 1ull << (code >> kQBit & 63u);
+  const uint64_t in1 = 1ull << (code >> kRBit & 63u), in2 = 1ull << (code >> kSBit & 63u);
+  // (targets are in the strings A and B; the electrons that leave: of the first electron's string
+  // and the second's, which for a swapped pair are B and A)
+  const bool a_dn = code & kADn, b_dn = code & kBDn;
+  if (code & kOne) {
+    if (a_dn) *d ^= out1 | in1;
+    else *u ^= out1 | in1;
+  } else if (a_dn == b_dn) {
+    const uint64_t x = out1 | out2 | in1 | in2;
+    if (a_dn) *d ^= x;
+    else *u ^= x;
+  } else {
+    *u ^= out1 | (a_dn ? in2 : in1);
+    *d ^= out2 | (a_dn ? in1 : in2);
+  }
 }
 
 // Slot hash of a det for the variational hash set (this set is internal: no other hash has
@@ -178,55 +231,6 @@ __device__ __forceinline__ double src_eps_min(const SelParams& P, uint32_t i) {
   if (i == 0 && P.var_sd) e = 0.0;
   if (P.time_sym && P.up[i] != P.dn[i]) e *= kSqrt2;  // solver.h:447
   return e;
-}
-
-
-// Candidate det for entry e of slot `slot` of det (up, dn), with the slot's electron orbitals from
-// slot_range.  Returns false when the target orbitals are occupied (the reference's occupancy checks).
-__device__ __forceinline__ bool make_candidate_at(const SelParams& P, uint64_t up, uint64_t dn,
-                                                  int slot, uint32_t orbs, uint32_t e,
-                                                  uint64_t* cu, uint64_t* cd) {
-  const int n = P.n_orbs;
-  *cu = up;
-  *cd = dn;
-  if (slot < P.n_elecs) {
-    const int p = static_cast<int>(orbs);
-    const int r = static_cast<int>(P.s_r[e]);
-    // an inactive target (active space) fails like an occupied one
-    if (slot < P.n_up) {
-      if ((up | P.inactive) >> r & 1) return false;
-      *cu = (up & ~(1ull << p)) | (1ull << r);
-    } else {
-      if ((dn | P.inactive) >> r & 1) return false;
-      *cd = (dn & ~(1ull << p)) | (1ull << r);
-    }
-    return true;
-  }
-  const int p = static_cast<int>(orbs & 0xffu), q = static_cast<int>(orbs >> 8);
-  const uint32_t rs = P.d_rs[e];
-  int r = rs & 0xffff, s = rs >> 16;
-  if (p >= n && q >= n) {
-    r += n;
-    s += n;
-  } else if (p < n && q >= n && p > q - n) {
-    const int tmp = s - n;
-    s = r + n;
-    r = tmp;
-  }
-  // an inactive target (active space) fails like an occupied one
-  const uint64_t bu = up | P.inactive, bd = dn | P.inactive;
-  const bool occ_r = r < n ? (bu >> r & 1) : (bd >> (r - n) & 1);
-  if (occ_r) return false;
-  const bool occ_s = s < n ? (bu >> s & 1) : (bd >> (s - n) & 1);
-  if (occ_s) return false;
-  uint64_t u = up, d = dn;
-  if (p < n) u &= ~(1ull << p); else d &= ~(1ull << (p - n));
-  if (q < n) u &= ~(1ull << q); else d &= ~(1ull << (q - n));
-  if (r < n) u |= 1ull << r; else d |= 1ull << (r - n);
-  if (s < n) u |= 1ull << s; else d |= 1ull << (s - n);
-  *cu = u;
-  *cd = d;
-  return true;
 }
 
 }  // namespace shci

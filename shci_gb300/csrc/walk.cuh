@@ -34,77 +34,6 @@ struct WalkWarp {
   uint8_t occ[128];  // electron -> spatial orbital, alpha electrons first
 };
 
-// Slot code: the orbitals p and q that the electrons leave, and the strings that the targets r and s
-// of an entry must be free in; a queued entry adds its targets.  A queue entry's r | s << 16 holds
-// the targets of the stored pair; a beta-beta pair is stored as its alpha image and an alpha-beta
-// pair p > q as (q, p) (chem_system.cc:347-361), so the strings follow from the slot alone.
-constexpr int kPBit = 0, kQBit = 6, kRBit = 12, kSBit = 18;
-enum : uint32_t { kADn = 1u << 24, kBDn = 1u << 25, kOne = 1u << 26 };
-
-// Entry range and code of slot `slot`; as slot_range (heatbath.cuh), the orbitals from `occ`.
-__device__ __forceinline__ uint32_t walk_slot(const SelParams& P, const uint8_t* occ, int slot,
-                                            double eps_min, double eps_max, uint32_t* lo,
-                                            uint32_t* cnt) {
-  *lo = 0;
-  *cnt = 0;
-  const int n = P.n_orbs;
-  if (slot < P.n_elecs) {
-    if (eps_min > P.max_singles) return 0;
-    const uint32_t p = occ[slot];
-    const uint32_t a = P.s_off[p], b = P.s_off[p + 1];
-    *lo = a;
-    *cnt = first_below(P.s_S, a, b, eps_min) - a;
-    return p << kPBit | kOne | (slot < P.n_up ? 0u : kADn);
-  }
-  if (P.no_doubles || eps_min > P.max_hci) return 0;
-  const uint32_t pr = P.pair_tab[slot - P.n_elecs];
-  const int e1 = pr & 0xffff, e2 = pr >> 16;
-  const uint32_t p = occ[e1], q = occ[e2];
-  const bool dn1 = e1 >= P.n_up, dn2 = e2 >= P.n_up;
-  uint32_t code;
-  size_t pq;
-  if (dn1 == dn2) {
-    pq = c2(p, q);
-    code = p << kPBit | q << kQBit | (dn1 ? kADn | kBDn : 0u);
-  } else if (p > q) {  // stored as (q, p + n): r goes to beta, s to alpha
-    pq = c2(q, p + n);
-    code = p << kPBit | q << kQBit | kADn;
-  } else {
-    pq = c2(p, q + n);
-    code = p << kPBit | q << kQBit | kBDn;
-  }
-  const uint32_t a = static_cast<uint32_t>(P.d_off[pq]), b = static_cast<uint32_t>(P.d_off[pq + 1]);
-  const uint32_t s = first_below(P.d_H, a, b, eps_max);
-  *lo = s;
-  *cnt = first_below(P.d_H, s, b, eps_min) - s;
-  return code;
-}
-
-__device__ __forceinline__ uint32_t bit_of(uint64_t x, uint32_t k) {
-  const uint32_t w = k & 32u ? static_cast<uint32_t>(x >> 32) : static_cast<uint32_t>(x);
-  return w >> (k & 31u) & 1u;
-}
-
-// The determinant that entry `code` (with its targets) makes of (*u, *d).
-__device__ __forceinline__ void apply_entry(uint32_t code, uint64_t* u, uint64_t* d) {
-  const uint64_t out1 = 1ull << (code >> kPBit & 63u), out2 = 1ull << (code >> kQBit & 63u);
-  const uint64_t in1 = 1ull << (code >> kRBit & 63u), in2 = 1ull << (code >> kSBit & 63u);
-  // (targets are in the strings A and B; the electrons that leave: of the first electron's string
-  // and the second's, which for a swapped pair are B and A)
-  const bool a_dn = code & kADn, b_dn = code & kBDn;
-  if (code & kOne) {
-    if (a_dn) *d ^= out1 | in1;
-    else *u ^= out1 | in1;
-  } else if (a_dn == b_dn) {
-    const uint64_t x = out1 | out2 | in1 | in2;
-    if (a_dn) *d ^= x;
-    else *u ^= x;
-  } else {
-    *u ^= out1 | (a_dn ? in2 : in1);
-    *d ^= out2 | (a_dn ? in1 : in2);
-  }
-}
-
 // Entries [skip, skip + left) of det (up, dn)'s windows [eps_min, eps_max), 32 at a time: all lanes
 // call push(valid, free, x, e) with x = slot code and targets, e = queue entry, free = both
 // targets are free (valid lanes only).
@@ -132,7 +61,7 @@ __device__ __forceinline__ void walk_window(const SelParams& P, WalkWarp& W, uin
     for (int s0 = f0; s0 < f1; s0 += 32) {
       uint32_t lo = 0, c = 0, code = 0;
       if (s0 + (int)lane < f1)
-        code = walk_slot(P, W.occ, s0 + lane, eps_min, eps_max, &lo, &c);
+        code = slot_window(P, [&](int e) { return W.occ[e]; }, s0 + lane, eps_min, eps_max, &lo, &c);
       const unsigned bl = __ballot_sync(kFull, c >= kWalkLong);
       const unsigned bs = __ballot_sync(kFull, c && c < kWalkLong);
       if (c) {
@@ -204,15 +133,8 @@ __device__ __forceinline__ void walk_window(const SelParams& P, WalkWarp& W, uin
         uint32_t x = 0, e = 0;
         if (t < end) {
           const uint32_t ok = kWalkSlots - 1u - (g + ol);
-          const uint32_t code = W.s_code[ok];
           e = W.s_lo[ok] + (t - o_first);
-          const uint64_t A = code & kADn ? bd : bu;
-          const uint64_t B = code & kOne ? 0ull : code & kBDn ? bd : bu;
-          const uint32_t rs = code & kOne ? P.s_r[e] : P.d_rs[e];
-          uint32_t r = rs & 0xffffu, s = rs >> 16;
-          if (s >= n_off) s -= n_off;
-          free = !(bit_of(A, r) | bit_of(B, s));
-          x = code | r << kRBit | s << kSBit;
+          free = entry_code(P, W.s_code[ok], e, bu, bd, &x);
         }
         push(t < end, free, x, e);
       }
