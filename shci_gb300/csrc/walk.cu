@@ -1,6 +1,9 @@
 // Pieces of the heat-bath windows (walk.cuh).
 #include "walk.cuh"
 
+#include <algorithm>
+#include <cstdlib>
+
 #include "kernels.h"
 
 namespace shci {
@@ -20,7 +23,9 @@ __device__ __forceinline__ uint64_t piece_region(uint64_t l, uint64_t mult, uint
 
 // Entries of a piece: eight pieces a resident warp, within kPieceMin and kPieceLen.  (A piece costs a
 // warp the search of its source's slots, about as long as a few hundred entries take.)
-__device__ __forceinline__ uint32_t piece_len(unsigned long long total, uint32_t warps) {
+__device__ __forceinline__ uint32_t piece_len(unsigned long long total, uint32_t warps,
+                                              uint32_t fixed) {
+  if (fixed) return fixed;
   const unsigned long long len = total / (8ull * warps);
   return len <= kPieceMin ? kPieceMin : len >= kPieceLen ? kPieceLen : static_cast<uint32_t>(len);
 }
@@ -39,11 +44,11 @@ __global__ void k_window_total(const uint64_t* __restrict__ entries, uint32_t n_
 __global__ void k_piece_count(const uint64_t* __restrict__ entries, uint32_t n_src,
                               uint64_t n_batches, double slack, double pad,
                               const uint32_t* __restrict__ ent_off, uint32_t warps,
-                              uint32_t* __restrict__ np, const unsigned* __restrict__ flag,
+                              uint32_t fixed, uint32_t* __restrict__ np, const unsigned* __restrict__ flag,
                               unsigned long long* __restrict__ back) {
   unsigned long long sum = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) back[2] = flag ? *flag : 0u;
-  const uint32_t plen = piece_len(back[3], warps);
+  const uint32_t plen = piece_len(back[3], warps, fixed);
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src;
        k += gridDim.x * blockDim.x) {
     const uint64_t m = entries[k], whole = m / plen, rest = m % plen;
@@ -60,11 +65,11 @@ __global__ void k_piece_count(const uint64_t* __restrict__ entries, uint32_t n_s
 // Region sizes go into off[p], to be scanned.
 __global__ void k_piece_fill(const uint64_t* __restrict__ entries, const uint32_t* __restrict__ first,
                              uint32_t n_src, uint64_t n_batches, double slack, double pad,
-                             const uint32_t* __restrict__ ent_off, uint32_t warps,
+                             const uint32_t* __restrict__ ent_off, uint32_t warps, uint32_t fixed,
                              const unsigned long long* __restrict__ total, uint32_t* __restrict__ src,
                              uint32_t* __restrict__ begin, uint32_t* __restrict__ len,
                              uint64_t* __restrict__ off) {
-  const uint32_t plen = piece_len(*total, warps);
+  const uint32_t plen = piece_len(*total, warps, fixed);
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_src;
        k += gridDim.x * blockDim.x) {
     const uint64_t m = entries[k];
@@ -96,6 +101,9 @@ unsigned make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_sr
   int sms = 0;
   SHCI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
   const uint32_t warps = static_cast<uint32_t>(sms) * kWalkWarps;
+  // SHCI_WALK_PIECE sets the entries of a piece.
+  const char* env = std::getenv("SHCI_WALK_PIECE");
+  const uint32_t fixed = env ? static_cast<uint32_t>(std::max(1, std::atoi(env))) : 0u;
   // total of the regions, pieces, flag (one wait for these); total of the windows
   DevBuf<unsigned long long> back;
   back.mt = &c->mem;
@@ -104,7 +112,7 @@ unsigned make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_sr
   k_window_total<<<grid_for(n_src, 256, 152), 256, 0, s>>>(entries.p, n_src, back.p + 3);
   SHCI_LAUNCH_CHECK();
   k_piece_count<<<grid_for(n_src, 256), 256, 0, s>>>(
-      entries.p, n_src, n_batches, slack, pad, ent_off, warps, first.p, flag, back.p);
+      entries.p, n_src, n_batches, slack, pad, ent_off, warps, fixed, first.p, flag, back.p);
   SHCI_LAUNCH_CHECK();
   exclusive_scan_u32_async(first.p, first.p, n_src, s, c->sort,
                            reinterpret_cast<uint32_t*>(back.p + 1));
@@ -120,7 +128,7 @@ unsigned make_pieces(shci_ctx* c, const DevBuf<uint64_t>& entries, uint32_t n_sr
   L.len.resize(L.n);
   L.off.resize(L.n + 1);
   k_piece_fill<<<grid_for(n_src, 256), 256, 0, s>>>(
-      entries.p, first.p, n_src, n_batches, slack, pad, ent_off, warps, back.p + 3, L.src.p,
+      entries.p, first.p, n_src, n_batches, slack, pad, ent_off, warps, fixed, back.p + 3, L.src.p,
       L.begin.p, L.len.p, L.off.p);
   SHCI_LAUNCH_CHECK();
   exclusive_scan_u64_async(L.off.p, L.off.p, L.n, s, c->sort, L.off.p + L.n);
