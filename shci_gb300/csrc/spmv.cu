@@ -24,6 +24,7 @@
 // The row abs-sum bound is computed once per matrix (float atomics; inflated by 5% against
 // their rounding).
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 
 #include "ctx.h"
@@ -334,6 +335,9 @@ void build_items(shci_ctx* c) {
   if (n == 0) return;
   R.cap = H.nnz_current / kItemLen + n;  // sum of ceil(len / kItemLen) over n rows
   if (R.cap >= 0xffffffffull) return;
+  // SHCI_ROW_ITEMS=0: whole rows, as without room for the list.
+  const char* env = std::getenv("SHCI_ROW_ITEMS");
+  if (env && std::strcmp(env, "0") == 0) return;
   try {
     R.off.resize((size_t)n + 1, 1.1);
     R.it.resize(R.cap, 1.1);
