@@ -108,7 +108,7 @@ void jacobi_eig(int k, const double* lower, int ld, double* evals, double* evecs
 
 // select.cu
 size_t select_dets(shci_ctx* c, double eps_var, bool var_sd);
-void rebuild_det_set(shci_ctx* c, bool allow_dup = false);
+bool rebuild_det_set(shci_ctx* c, bool allow_dup = false);
 // The same in two halves: the set, and its check with a wait that the caller has anyway.  The first
 // half returns a device word that is not 0 when the list contains duplicates.
 const unsigned* build_det_set(shci_ctx* c);

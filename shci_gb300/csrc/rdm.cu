@@ -29,7 +29,7 @@ constexpr int kRdmWarps = 8;
 // per det and one hash probe per excitation.
 __global__ void __launch_bounds__(kRdmWarps * 32)
     k_rdm1(SelParams P, const double* __restrict__ coef, uint32_t n_dets,
-           const unsigned* __restrict__ orb_sym, int n, double* __restrict__ out) {
+           const unsigned* __restrict__ orb_sym, int n, bool dup, double* __restrict__ out) {
   extern __shared__ double tile[];
   __shared__ uint8_t occ[kRdmWarps][64], virt[kRdmWarps][64];
   __shared__ unsigned sym[64];
@@ -42,6 +42,8 @@ __global__ void __launch_bounds__(kRdmWarps * 32)
   for (uint32_t i = blockIdx.x * kRdmWarps + w; i < n_dets; i += warps) {
     const uint64_t u = P.up[i], d = P.dn[i];
     const double ci = coef[i];
+    // (of equal dets the set holds the first: a det's own partner too)
+    const double cc = ci * (dup ? coef[set_index(P, u, d)] : ci);
     for (int spin = 0; spin < 2; spin++) {
       const uint64_t h = spin ? d : u;
       __syncwarp();
@@ -51,8 +53,8 @@ __global__ void __launch_bounds__(kRdmWarps * 32)
         else virt[w][o - k] = static_cast<uint8_t>(o);
       }
       __syncwarp();
-      if (h >> lane & 1) dg0 += ci * ci;
-      if (h >> (lane + 32) & 1) dg1 += ci * ci;
+      if (h >> lane & 1) dg0 += cc;
+      if (h >> (lane + 32) & 1) dg1 += cc;
       const uint32_t ne = static_cast<uint32_t>(popc64(h)), nv = static_cast<uint32_t>(n) - ne;
       for (uint32_t t = lane; t < ne * nv; t += 32) {
         const int p = occ[w][t / nv], r = virt[w][t % nv];
@@ -235,7 +237,7 @@ void rdm1_dev(shci_ctx* c, double* res_dev) {
   const uint32_t n_dets = static_cast<uint32_t>(c->up.size());
   const int n = c->I.n;
   cudaStream_t s = c->stream;
-  rebuild_det_set(c, true);
+  const bool dup = rebuild_det_set(c, true);
   SelParams P{};
   P.up = c->d_up.p;
   P.dn = c->d_dn.p;
@@ -251,7 +253,7 @@ void rdm1_dev(shci_ctx* c, double* res_dev) {
   {
     ProfScope ps(c->prof, s, "rdm1");
     k_rdm1<<<grid_for((size_t)n_dets * 32, kRdmWarps * 32, (unsigned)sms * 6u), kRdmWarps * 32,
-             (size_t)n * n * sizeof(double), s>>>(P, c->d_coef.p, n_dets, sym.p, n, res_dev);
+             (size_t)n * n * sizeof(double), s>>>(P, c->d_coef.p, n_dets, sym.p, n, dup, res_dev);
     SHCI_LAUNCH_CHECK();
   }
   SHCI_CUDA(cudaStreamSynchronize(s));

@@ -405,6 +405,7 @@ __global__ void k_hash_insert(const uint64_t* __restrict__ up, const uint64_t* _
         const uint32_t id = static_cast<uint32_t>(old) - 1u;
         if (up[id] == u && dn[id] == d) {
           atomicOr(dup, 1u);
+          atomicMin(&table[p], v);  // (the same fingerprint: the lower id stays)
           break;
         }
       }
@@ -414,9 +415,9 @@ __global__ void k_hash_insert(const uint64_t* __restrict__ up, const uint64_t* _
 }
 
 // The membership set used by selection, PT2, S^2 and the 1-RDM: a hash set of the det list, a power
-// of two >= 2n slots.  allow_dup: the set holds one of each group of equal dets instead of refusing
-// the list.  (The set used to come with a sorted copy of the list that only the duplicate check
-// read: two radix sorts per call.)
+// of two >= 2n slots.  allow_dup: the set holds the first of each group of equal dets instead of
+// refusing the list; returns whether there are such.  (The set used to come with a sorted copy of the
+// list that only the duplicate check read: two radix sorts per call.)
 const unsigned* build_det_set(shci_ctx* c) {
   const size_t n = c->up.size();
   cudaStream_t s = c->stream;
@@ -440,12 +441,13 @@ void check_det_set(unsigned flag) {
   if (flag) throw ArgError("the det list contains duplicates");
 }
 
-void rebuild_det_set(shci_ctx* c, bool allow_dup) {
+bool rebuild_det_set(shci_ctx* c, bool allow_dup) {
   const unsigned* dup = build_det_set(c);
   unsigned flag = 0;
   SHCI_CUDA(cudaMemcpyAsync(&flag, dup, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   SHCI_CUDA(cudaStreamSynchronize(c->stream));
   if (!allow_dup) check_det_set(flag);
+  return flag != 0;
 }
 
 namespace {
