@@ -3,7 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <cstdlib>
 #include <map>
 #include <stdexcept>
 #include <string>
@@ -42,7 +44,8 @@ struct OverflowError : std::runtime_error {
 // runs on its one stream, so a block reused after a release is ordered after the work that used it.
 // A request that does not fit the device or the budget first returns the cache to the driver.
 // The cache holds at most a quarter of the device's memory, so the driver always keeps room
-// for what it allocates by itself (local memory of launches, library workspaces).
+// for what it allocates by itself (local memory of launches, library workspaces), and when it is full
+// the blocks released longest ago go.
 struct MemTracker {
   size_t budget = 0;  // 0 = unlimited
   size_t used = 0;    // held: live blocks and cached ones
@@ -50,7 +53,12 @@ struct MemTracker {
   size_t peak_live = 0;  // the most held by live blocks
   size_t cached = 0;     // held in the cache
   size_t cache_cap = 0;  // 0: not set yet (a quarter of the device's memory)
-  std::multimap<size_t, void*> cache;  // released blocks by size in bytes
+  struct Block {
+    void* p;
+    uint64_t when;  // order of the releases
+  };
+  std::multimap<size_t, Block> cache;  // released blocks by size in bytes
+  uint64_t releases = 0;
 
   MemTracker() = default;
   MemTracker(const MemTracker&) = delete;
@@ -62,7 +70,7 @@ struct MemTracker {
     auto it = cache.lower_bound(bytes);
     if (it == cache.end() || static_cast<double>(it->first) > fit * static_cast<double>(bytes))
       return nullptr;
-    void* p = it->second;
+    void* p = it->second.p;
     *got = it->first;
     cached -= it->first;
     cache.erase(it);
@@ -72,13 +80,27 @@ struct MemTracker {
     if (cache_cap == 0) {
       size_t f = 0, t = 0;
       cache_cap = cudaMemGetInfo(&f, &t) == cudaSuccess ? t / 4 : 1;
+      // (SHCI_CACHE_MB sets it)
+      if (const char* e = std::getenv("SHCI_CACHE_MB"))
+        cache_cap = static_cast<size_t>(std::max(1, std::atoi(e))) << 20;
     }
-    if (cached + bytes > cache_cap) {
+    if (bytes > cache_cap) {
       cudaFree(p);
       used -= bytes;
       return;
     }
-    cache.emplace(bytes, p);
+    // The blocks released longest ago make room: a full cache of sizes that no call asks for any more
+    // would cost every call its allocations (n = 40: the three PT2 stages 0.507 -> 0.517 s).
+    while (cached + bytes > cache_cap) {
+      auto old = cache.begin();
+      for (auto it = cache.begin(); it != cache.end(); ++it)
+        if (it->second.when < old->second.when) old = it;
+      cudaFree(old->second.p);
+      used -= old->first;
+      cached -= old->first;
+      cache.erase(old);
+    }
+    cache.emplace(bytes, Block{p, releases++});
     cached += bytes;
   }
   void note_live() {
@@ -86,7 +108,7 @@ struct MemTracker {
   }
   // Returns every cached block to the driver.
   void flush() {
-    for (auto& kv : cache) cudaFree(kv.second);
+    for (auto& kv : cache) cudaFree(kv.second.p);
     used -= cached;
     cached = 0;
     cache.clear();
