@@ -10,7 +10,7 @@
 //
 // Few dets: the unit is one slot, its window found by a kernel before (with a warp per det, 16 dets
 // of an n = 26 system kept 16 warps of the chip busy for 785 rounds per walk: 2.06 -> 0.39 ms for the
-// two calls, 98 us of kernels).  Many dets: most slots' windows are empty, and a warp for each costs
+// two calls, 85 us of kernels).  Many dets: most slots' windows are empty, and a warp for each costs
 // more than the walk, so the unit is 32 slots of a det or more, whose windows the lanes find and
 // whose entries are flattened over them.
 #include <algorithm>

@@ -557,7 +557,8 @@ bool join_prepare(shci_ctx* c) {
   const uint64_t K = static_cast<uint64_t>(ne) * (ne - 1) / 2;
   const uint64_t m = n * K;
   if (m >= 0xffffffffull) return false;
-  // memory: keys + sort ping-pong (16 B), entry values + ping-pong (8 B), then span (8 B)
+  // memory of an entry: key and id with their sorted copies and a quarter to spare (18 B, 27 with
+  // 64-bit keys), then id, span and, placed by leading bits, their sorted copies (24 B)
   size_t free_b = 0, total_b = 0;
   SHCI_CUDA(cudaMemGetInfo(&free_b, &total_b));
   size_t avail = free_b + c->mem.cached;  // cached blocks return to the driver on demand

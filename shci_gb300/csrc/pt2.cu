@@ -217,8 +217,8 @@ struct PtWarp {
 // Queues carry over from piece to piece.  Members keep their walk order within a piece.
 // Warps take pieces from a counter, the next one while they walk (a fixed share left a tenth of the
 // chip idle: 26.3 -> 24.4 ms over the stages of an n = 40 run).
-// At n = 40, 40,000 dets: 19.4 -> 4.1 ms deterministic (297M window entries), 11.3 -> 4.8 ms a
-// pseudo-stochastic batch of 16 (walk and hash are most of the work left), 21.4 -> 10.6 ms for six
+// At n = 40, 40,000 dets: 19.4 -> 4.1 ms deterministic (297M window entries), 11.3 -> 4.0 ms a
+// pseudo-stochastic batch of 16 (walk and hash are most of the work left), 21.4 -> 8.6 ms for six
 // stochastic iterations; n = 26, 30,000 dets: 5.3 -> 1.3 ms, of which the heaviest determinant's
 // window on one warp had been half.  (Before: build and hash at the walk, an output slot for
 // every window entry, a warp per source.)
@@ -1016,9 +1016,11 @@ Pt2Out pt_batched(shci_ctx* c, double e_var, PtParams Q, size_t n_batches, doubl
   DevBuf<uint64_t> entries;
   pt_counts<MODE>(c, st, Q, S, n_var, entries);
   if (n_batches == 0) {
-    // Automatic batch count: every candidate pair costs ~48 device bytes while a batch is
-    // processed (keys, value columns, compaction, sort ping-pong); keep a batch within 40% of
-    // the free HBM.  (The dtm energy does not depend on the batch count.)
+    // Automatic batch count: 48 device bytes a window entry within 40 % of the free HBM.  A record
+    // costs about 100 while it is grouped (32 and half as much for growth, 32 gathered, 19 for keys,
+    // indexes and their sorted copies), but one window entry in two or fewer makes one (four of five
+    // targets are occupied at n = 40), and a batch that still finds no room is taken in parts.  (The
+    // dtm energy does not depend on the batch count.)
     uint64_t tot = 0;
     {
       DevBuf<uint64_t> sum;

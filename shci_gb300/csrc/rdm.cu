@@ -128,7 +128,7 @@ __device__ __forceinline__ void rdm2_double(double* __restrict__ half, int n, ui
 
 // Off-diagonal pairs.  A single excitation adds about 4 n_e terms and a double 2 or 4, so a warp
 // that finished its lanes' elements in place would run the singles' loop for one or two lanes:
-// singles wait in a per-warp queue and are finished 32 at a time.  5.6 -> 1.14 ms at n = 26, 80,000
+// singles wait in a per-warp queue and are finished 32 at a time.  5.6 -> 1.24 ms at n = 26, 80,000
 // dets, 36M elements (a warp per row and the diagonal on one lane of it before); bound by the
 // FP64 atomics' L1 and L2 traffic (about 60 % busy each).
 __global__ void __launch_bounds__(kRdmWarps * 32)
