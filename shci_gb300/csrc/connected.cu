@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(kConnWarps * 32)
 //   60,000: 0.88, 1.81 by 32 (420,000 units), 0.77, 1.85 by 64, 0.77, 2.07 by 128.
 int slots_per_unit(uint64_t n, uint64_t n_slots) {
   // SHCI_CONNECTED_SLOTS sets them.
-  if (const char* env = std::getenv("SHCI_CONNECTED_SLOTS")) return std::max(1, std::atoi(env));
+  if (const char* env = std::getenv("SHCI_CONNECTED_SLOTS"))
+    return std::min(1 << 20, std::max(1, std::atoi(env)));
   if (n * n_slots <= kSlotUnits) return 1;
   const uint64_t units = n * ((n_slots + 31) / 32);
   return units <= kGroup32Units ? 32 : units <= kGroup64Units ? 64 : 128;
